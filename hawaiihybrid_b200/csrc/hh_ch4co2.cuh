@@ -154,6 +154,15 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct Ch4
     f[17] = STG(-(uh[2] * g.Gu[0] - uh[0] * g.Gu[2]));
     f[18] = STG(-(uh[0] * g.Gu[1] - uh[1] * g.Gu[0]));
   }
+  // component c of f (solo kernel): the full stage point gathered from the lanes, the
+  // right-hand side on every lane
+  __device__ __forceinline__ STG rhs_c(STG ysc, int c) const {
+    STG ys[N], f[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
+    rhs(ys, f);
+    return pick_component<N>(f, c);
+  }
   // samples are written as records; no dipole on this path
   __device__ void dipole(const double *, PHYS d[3]) const { d[0] = d[1] = d[2] = PHYS(0); }
 };

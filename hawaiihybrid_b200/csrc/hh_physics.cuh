@@ -31,6 +31,15 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
 
+// component c of v, all indices compile-time (v stays in registers)
+template <int N, typename T> __device__ __forceinline__ T pick_component(const T (&v)[N], int c) {
+  T r = v[0];
+#pragma unroll
+  for (int i = 1; i < N; ++i)
+    if (c == i) r = v[i];
+  return r;
+}
+
 // ----------------------------------------------------------------------------
 // He-Ar (PES-IDS/HeAr.h:33-107): exponential repulsion + damped dispersion
 // V = A exp(-g1 R - g2 R^2) - sum_{n=3..8} C_2n f_2n(bR) / R^2n,
@@ -68,6 +77,52 @@ __device__ __forceinline__ void hear_V_dV(T R, T iR, T &V, T &dV) {
     V -= C[n - 3] * f * iRp;
     dV -= C[n - 3] * (fp * iRp - T(2 * n) * f * iRp * iR);
   }
+}
+
+// dV/dR of hear_V_dV with the 32 lanes of a warp on one R, bit for bit: the exponential
+// of the damping on even lanes and that of the repulsion on odd ones, dispersion term
+// n = 3 + lane % 6 per lane, the terms subtracted in order from shuffles.
+template <typename T>
+__device__ __forceinline__ T hear_dV_coop(T R, T iR, int lane) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const T A = T(0.2303058634e2), G1 = T(0.163051044e1), G2 = T(0.4680016e-1);
+  const T B = T(0.16274792500000e1);
+  const T C[6] = {T(0.940835513e1), T(0.165523018e3), T(0.379715796e4),
+                  T(0.1165179999e6), T(0.466258000e7), T(0.236861000e9)};
+  T x = B * R;
+  const int nn = 3 + lane % 6;
+  T term = T(1), S = T(1);
+#pragma unroll
+  for (int m = 1; m <= 4; ++m) {
+    term *= x * T(1.0 / double(m));
+    S += term;
+  }
+  T iR2 = iR * iR;
+  T iRp = iR2 * iR2;
+  T my_term = T(0), my_S = T(0), my_iRp = T(0);
+#pragma unroll
+  for (int n = 3; n <= 8; ++n) {
+    term *= x * T(1.0 / double(2 * n - 1));
+    S += term;
+    term *= x * T(1.0 / double(2 * n));
+    S += term;
+    iRp *= iR2;
+    if (nn == n) {
+      my_term = term;
+      my_S = S;
+      my_iRp = iRp;
+    }
+  }
+  const T em = exp((lane & 1) ? -G1 * R - G2 * R * R : -x);
+  const T ex = __shfl_sync(FULL, em, 0);
+  T rep = A * __shfl_sync(FULL, em, 1);
+  T dV = rep * (-G1 - T(2) * G2 * R);
+  T f = T(1) - ex * my_S;
+  T fp = B * ex * my_term;
+  const T w = fp * my_iRp - T(2 * nn) * f * my_iRp * iR;
+#pragma unroll
+  for (int n = 3; n <= 8; ++n) dV -= C[n - 3] * __shfl_sync(FULL, w, n - 3);
+  return dV;
 }
 
 template <typename T>

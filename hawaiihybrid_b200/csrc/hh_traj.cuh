@@ -224,6 +224,20 @@ __device__ void load_tables(Co2arTables<T> *s, const Co2arTablesGlobal *g) {
   }
 }
 
+// Component c of the He-Ar right-hand side with the 32 lanes of a warp on one stage point,
+// bit for bit as HeArSys::rhs; out of line, one copy for the stages of the solo kernel.
+template <typename T> __device__ __noinline__ T hear_rhs_lane(T ysc, T im, int c) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const T r0 = __shfl_sync(FULL, ysc, 0), r1 = __shfl_sync(FULL, ysc, 1), r2 = __shfl_sync(FULL, ysc, 2);
+  const T pc = __shfl_sync(FULL, ysc, c < 3 ? c + 3 : c - 3);  // p_c, or r_c on the momentum lanes
+  T R2 = r0 * r0 + r1 * r1 + r2 * r2;
+  T iR = inv_sqrt(R2);
+  T R = R2 * iR;
+  const T dV = hear_dV_coop<T>(R, iR, threadIdx.x & 31);
+  T g = dV * iR;
+  return (c < 3 ? im : -g) * pc;
+}
+
 // ---- systems ----
 // SOLO_ (every system): the solo kernel's instance, one trajectory per warp
 template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct HeArSys {
@@ -254,6 +268,9 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct HeA
     f[4] = STG(-g * r1);
     f[5] = STG(-g * r2);
   }
+  // component c of f at the stage point whose component c is ysc (solo kernel: lane c
+  // holds component c, lanes >= N mirror the last one); the values are those of rhs
+  __device__ __forceinline__ STG rhs_c(STG ysc, int c) const { return hear_rhs_lane<PHYS>(ysc, STG(inv_mu), c); }
   __device__ void dipole(const double *y, PHYS d[3]) const {
     PHYS r0 = PHYS(y[0]), r1 = PHYS(y[1]), r2 = PHYS(y[2]);
     PHYS R2 = r0 * r0 + r1 * r1 + r2 * r2;
@@ -328,6 +345,136 @@ __device__ __noinline__ PesGrad<T> co2ar_pes_grad(const Co2arTables<T> *tb, T R,
   }
 }
 
+// legendre10 with the rounding of every operation fixed, as the out-of-line per-lane
+// gradient rounds it (the last P_l, which feeds one sum only, fuses the other product)
+template <typename T> __device__ __forceinline__ void legendre10_rn(T x, T (&P)[11], T (&dP)[11]) {
+  P[0] = T(1);
+  P[1] = x;
+  dP[0] = T(0);
+  dP[1] = T(1);
+#pragma unroll
+  for (int l = 1; l < 10; ++l) {
+    const T ax = n2_mul(T(2 * l + 1), x);
+    const T d = l < 9 ? n2_fma(ax, P[l], -n2_mul(T(l), P[l - 1])) : n2_fma(-T(l), P[l - 1], n2_mul(ax, P[l]));
+    P[l + 1] = n2_mul(d, T(1.0 / double(l + 1)));
+    dP[l + 1] = n2_fma(T(2 * l + 1), P[l], dP[l - 1]);
+  }
+}
+
+template <typename T, bool EXP>
+__device__ __forceinline__ PesGrad<T> co2ar_pes_grad_lanes(const Co2arTables<T> *tb, T R, T iR, T x, int i, int li) {
+  constexpr unsigned FULL = 0xffffffffu;
+  T P[11], dP[11], c, dc;
+  const T t = R - tb->rlo[i];
+  if constexpr (sizeof(T) == 4) {
+    const float4 *rw = tb->pes2 + (i * CO2AR_NL + li) * (CO2AR_PAIR_WORDS / 4);
+    const float4 a = rw[0], b = rw[1], p = rw[2], q = rw[3];
+    const float iR2 = iR * iR, iR4 = iR2 * iR2;
+    const float2 q4 = make_float2(iR4, iR4 * iR), q5 = mul2(q4, splat2(iR)), q6 = mul2(q5, splat2(iR)),
+                 q7 = mul2(q6, splat2(iR));
+    float2 v = fma2(make_float2(a.x, a.y), splat2(t), make_float2(a.z, a.w));
+    v = fma2(v, splat2(t), make_float2(b.x, b.y));
+    v = fma2(v, splat2(t), make_float2(b.z, b.w));
+    v = fma2(make_float2(p.x, p.y), q4, v);
+    v = fma2(make_float2(p.z, p.w), q5, v);
+    v = fma2(make_float2(q.x, q.y), q6, v);
+    v = fma2(make_float2(q.z, q.w), q7, v);
+    if constexpr (EXP) {
+      const float4 e = rw[4];
+      v = fma2(make_float2(e.x, e.y), splat2(expf(e.z * R)), v);
+    }
+    c = v.x;
+    dc = v.y;
+  } else {
+    // the row in 16-byte loads
+    const double2 *rw = reinterpret_cast<const double2 *>(tb->pes + (i * CO2AR_NL + li) * CO2AR_ROW);
+    double row[CO2AR_ROW];
+#pragma unroll
+    for (int e = 0; e < (EXP ? 5 : 4); ++e) {
+      const double2 v = rw[e];
+      row[2 * e] = v.x;
+      row[2 * e + 1] = v.y;
+    }
+    radial<T>(row, R, t, iR, EXP ? 3 : 1, c, dc);
+  }
+  legendre10_rn(x, P, dP);
+  T aR = T(0), ax = T(0);
+#pragma unroll
+  for (int l = 0; l < CO2AR_NL; ++l) {
+    const T cl = __shfl_sync(FULL, c, l), dcl = __shfl_sync(FULL, dc, l);
+    aR = n2_fma(P[2 * l], dcl, aR);
+    ax = n2_fma(dP[2 * l], cl, ax);
+  }
+  // (rounded here: the caller's expressions must not fuse with these products)
+  const T sc = T(1.0 / HH_HTOCM);
+  return {n2_mul(aR, sc), n2_mul(ax, sc)};
+}
+
+// Where lane c = 3 g + k of the solo kernel finds its operands: the source lanes of the
+// four values that its component reads besides r and u.
+//   g = 0 (dr/dt)  s1: p_k
+//   g = 1 (dp/dt)  s1: r_k   s2: u_k
+//   g = 2 (du/dt)  s1: j_k1  s2: u_k2  s3: u_k1  s4: j_k2
+//   g = 3 (dj/dt)  s1: r_k2  s2: u_k1  s3: u_k2  s4: r_k1       (k1 = k + 1, k2 = k + 2 mod 3)
+struct LinearLane {
+  int g, s1, s2, s3, s4, li;
+  __device__ __forceinline__ explicit LinearLane(int lane) {
+    const int c = lane < 12 ? lane : 11, k = c % 3, k1 = (k + 1) % 3, k2 = (k + 2) % 3;
+    g = c / 3;
+    s1 = g == 0 ? c + 3 : g == 1 ? k : g == 2 ? 9 + k1 : k2;
+    s2 = 6 + (g == 1 ? k : g == 2 ? k2 : k1);
+    s3 = 6 + (g == 2 ? k1 : k2);
+    s4 = g == 2 ? 9 + k2 : k1;
+    li = lane % CO2AR_NL;
+  }
+};
+
+// Component c of the CO2-Ar right-hand side with the 32 lanes of a warp on one stage point,
+// bit for bit as Co2ArSys::rhs; out of line, one copy for the stages of the solo kernel.
+// Every lane forms R, x and the Legendre recurrence; lane li % 6 the radial function of
+// l = 2 li, summed in order from shuffles; lane c its own component.  The interval is the
+// number of bounds at or below R, one bound per lane and a ballot: the reference's
+// `R < bound` search without its loops.  The inverse powers are evaluated in every
+// interval (zero coefficients add exact zeros), so that outside the innermost interval,
+// the one with exponentials, the radial functions share a basic block with the recurrence.
+template <typename T>
+__device__ __noinline__ T co2ar_rhs_lane(const Co2arTables<T> *tb, T ysc, T im, T iI, LinearLane L) {
+  static_assert(CO2AR_NINT <= 32, "one interval bound per lane");
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const T rb = tb->rbound[lane < CO2AR_NINT - 1 ? lane : CO2AR_NINT - 2];
+  T r[3], u[3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r[i] = __shfl_sync(FULL, ysc, i);
+    u[i] = __shfl_sync(FULL, ysc, 6 + i);
+  }
+  const T v1 = __shfl_sync(FULL, ysc, L.s1), v2 = __shfl_sync(FULL, ysc, L.s2);
+  const T v3 = __shfl_sync(FULL, ysc, L.s3), v4 = __shfl_sync(FULL, ysc, L.s4);
+  T R2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
+  T iR = inv_sqrt(R2);
+  T R = R2 * iR;
+  T iu = inv_sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
+  T rh[3] = {r[0] * iR, r[1] * iR, r[2] * iR};
+  T uh[3] = {u[0] * iu, u[1] * iu, u[2] * iu};
+  T x = rh[0] * uh[0] + rh[1] * uh[1] + rh[2] * uh[2];
+  const int i = __popc(__ballot_sync(FULL, lane < CO2AR_NINT - 1 && R >= rb));
+  const PesGrad<T> G = tb->fpes[i] & 2 ? co2ar_pes_grad_lanes<T, true>(tb, R, iR, x, i, L.li)
+                                       : co2ar_pes_grad_lanes<T, false>(tb, R, iR, x, i, L.li);
+  const T VR = G.VR, Vx = G.Vx;
+  T a = VR - Vx * x * iR;  // dV/dr = a r^ + (Vx/R) u^
+  T b = Vx * iR;
+  // force: b u^_k + a r^_k; axis: j_k1 u_k2 - j_k2 u_k1; torque: u^_k1 r^_k2 - u^_k2 r^_k1
+  // (the first product is the one that is fused with the sum in rhs)
+  const T s = L.g == 2 ? T(1) : iu;
+  const T A = n2_mul(v1, iR), B = n2_mul(v2, s), C = n2_mul(v3, s), D = n2_mul(v4, iR);
+  const T X = L.g == 1 ? b : L.g == 2 ? v1 : A;
+  const T Y = L.g == 1 ? a : L.g == 2 ? -v4 : -C;
+  const T Z = L.g == 1 ? A : L.g == 2 ? C : D;
+  const T q = L.g == 0 ? v1 : n2_fma(X, B, n2_mul(Y, Z));
+  return (L.g == 0 ? im : L.g == 1 ? T(-1) : L.g == 2 ? iI : -Vx) * q;
+}
+
 // Body-frame dipole sums (d_z, a_x) of CO2-Ar, out of line for the same reason:
 // the sample loop evaluates two pooled samples per lane and the item set-up one
 // more, and each inlined copy repeats the whole dipole surface.
@@ -386,6 +533,11 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct Co2
     f[9] = STG(-Vx * (uh[1] * rh[2] - uh[2] * rh[1]));
     f[10] = STG(-Vx * (uh[2] * rh[0] - uh[0] * rh[2]));
     f[11] = STG(-Vx * (uh[0] * rh[1] - uh[1] * rh[0]));
+  }
+  // component c of f at the stage point whose component c is ysc (solo kernel, as
+  // HeArSys::rhs_c); the values are those of rhs
+  __device__ __forceinline__ STG rhs_c(STG ysc, int) const {
+    return co2ar_rhs_lane<PHYS>(tb, ysc, STG(inv_mu), STG(inv_II), LinearLane(threadIdx.x & 31));
   }
   // q = (r[3], u[3])
   __device__ void dipole(const double *q, PHYS d[3]) const {
@@ -468,6 +620,15 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     f[9] = STG(-(uh[1] * Gu[2] - uh[2] * Gu[1]));
     f[10] = STG(-(uh[2] * Gu[0] - uh[0] * Gu[2]));
     f[11] = STG(-(uh[0] * Gu[1] - uh[1] * Gu[0]));
+  }
+  // component c of f (solo kernel): the full stage point gathered from the lanes, the
+  // right-hand side on every lane
+  __device__ __forceinline__ STG rhs_c(STG ysc, int c) const {
+    STG ys[N], f[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
+    rhs(ys, f);
+    return pick_component<N>(f, c);
   }
   // q = (r[3], u[3]); the body-frame dipole is the FP64 network on the FP64 path and
   // the FP32 table of hh_n2ar.cuh (the network outside its R range) on the mixed path
@@ -694,68 +855,84 @@ __device__ __forceinline__ void dense_stages(const Sys &sys, STG (&K)[16][Sys::N
 // ---- solo kernel: one trajectory per warp, component `lane` of the state per lane ----
 // The stage sums, the 8th-order solution, the error terms and the dense-output
 // coefficients of component i are formed by lane i with the same operations in
-// the same order as the per-lane functions above; the stage points are gathered
-// by shuffles and every lane evaluates the right-hand side on the full point.  The
-// error norm is summed over the components in order.  A trajectory therefore takes
-// the same steps in either kernel.
-template <int N, typename T> __device__ __forceinline__ T pick_component(const T (&v)[N], int c) {
-  T r = v[0];
-#pragma unroll
-  for (int i = 1; i < N; ++i)
-    if (c == i) r = v[i];
-  return r;
-}
+// the same order as the per-lane functions above; the lanes share the right-hand side
+// (Sys::rhs_c).  The error norm is summed over the components in order.  A trajectory
+// therefore takes the same steps in either kernel.
 
-// K[S] of this lane's component from the stage point built from K[0..S-1]
+// One warp per scheduler runs this, so a step costs its instructions and their latencies
+// (FP64: 8.6 cycles dependent, 3.4 issued).  The right-hand side is out of line, one copy
+// for all stages (15 inlined copies stalled on instruction fetches for 46 % of their
+// time), and its independent parts are spread over the lanes.  The sums are formed
+// right-looking: once K_j is known, a_{S,j} K_j goes into the sums of the later stages, of
+// the solution, the error estimates and the dense output.  Each sum takes its terms in the
+// order j = 0, 1, .. of the per-lane code, but only its last term waits for K_{S-1}.
+// Measured, solo launch: He-Ar 10,240 x 65,536 FP64 80 -> 58 ms (12.0 -> 9.0 us per step),
+// CO2-Ar 102,400 x 32,768 FP64 229 -> 134 ms, PR_MU 4,096 x 4,096 FP64 26.3 -> 16.8 ms.  A
+// rolled stage loop with the right-hand side inlined took 28 % (CO2-Ar) more per step.
+// rows: A[i] the sum of stage i + 1 (A[11]: the solution), X the stages 13..15, D the
+// dense-output rows
+template <typename STG, typename ET> struct SoloSums {
+  STG A[12], X[3], D[4];
+  ET a5, a3, m5;
+};
+template <class Sys, typename STG>
+using SysSums = SoloSums<STG, typename std::conditional<Sys::EST64, double, STG>::type>;
+
+// K_j into the sums of all rows that come later
+template <int J, typename STG, typename ET> __device__ __forceinline__ void solo_add(SoloSums<STG, ET> &s, STG K) {
+#pragma unroll
+  for (int i = J; i < 12; ++i)
+    if (hh_dop853_a[i + 1][J] != 0.0) s.A[i] += STG(hh_dop853_a[i + 1][J]) * K;
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+    if (J < 13 + i && hh_dop853_a[13 + i][J] != 0.0) s.X[i] += STG(hh_dop853_a[13 + i][J]) * K;
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    if (hh_dop853_d[r][J] != 0.0) s.D[r] += STG(hh_dop853_d[r][J]) * K;
+  if constexpr (J < 13) {
+    if (hh_dop853_e5[J] != 0.0) {
+      const ET t = ET(hh_dop853_e5[J]) * ET(K);
+      s.a5 += t;
+      if (sizeof(STG) == 4) s.m5 += fabs(t);
+    }
+    if (hh_dop853_e3[J] != 0.0) s.a3 += ET(hh_dop853_e3[J]) * ET(K);
+  }
+}
+// stage S of this lane's component, then K_S into the sums
 template <class Sys, typename STG, int S>
-__device__ __forceinline__ void cp_stage(const Sys &sys, STG (&K)[16][1], STG ys0, STG hs, int c) {
-  constexpr int N = Sys::N;
-  STG acc = STG(0);
-#pragma unroll
-  for (int j = 0; j < S; ++j)
-    if (hh_dop853_a[S][j] != 0.0) acc += STG(hh_dop853_a[S][j]) * K[j][0];
-  const STG ysc = ys0 + hs * acc;
-  STG ys[N], f[N];
-#pragma unroll
-  for (int i = 0; i < N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
-  sys.rhs(ys, f);
-  K[S][0] = pick_component<N>(f, c);
+__device__ __forceinline__ void cp_stage(const Sys &sys, SysSums<Sys, STG> &s, STG ys0, STG hs, int c) {
+  const STG K = sys.rhs_c(ys0 + hs * (S < 13 ? s.A[S < 13 ? S - 1 : 0] : s.X[S < 13 ? 0 : S - 13]), c);
+  solo_add<S>(s, K);
 }
 
 template <class Sys, typename STG>
-__device__ __forceinline__ double step_attempt_cp(const Sys &sys, const TrajParams &P, STG (&K)[16][1],
-                                                  double y, double h, double &y_new) {
+__device__ __forceinline__ double step_attempt_cp(const Sys &sys, const TrajParams &P, STG k0, double y, double h,
+                                                  double &y_new, STG &k12, SysSums<Sys, STG> &s) {
   constexpr int N = Sys::N;
   const int lane = threadIdx.x & 31;
   const int c = lane < N ? lane : N - 1;
   const STG ys0 = STG(y);
   const STG hs = STG(h);
-  cp_stage<Sys, STG, 1>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 2>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 3>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 4>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 5>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 6>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 7>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 8>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 9>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 10>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 11>(sys, K, ys0, hs, c);
-  {
-    STG acc = STG(0);
-#pragma unroll
-    for (int j = 0; j < 12; ++j)
-      if (hh_dop853_a[12][j] != 0.0) acc += STG(hh_dop853_a[12][j]) * K[j][0];
-    y_new = y + h * double(acc);
-    double yn[N];
-    STG f[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) yn[i] = __shfl_sync(0xffffffffu, y_new, i);
-    sys.rhs(yn, f);
-    K[12][0] = pick_component<N>(f, c);
-  }
-  double q5, q3;
-  err_terms<STG, Sys::EST64>(K, 0, y, y_new, h, P, q5, q3);
+  s = SysSums<Sys, STG>{};
+  solo_add<0>(s, k0);
+  cp_stage<Sys, STG, 1>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 2>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 3>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 4>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 5>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 6>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 7>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 8>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 9>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 10>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 11>(sys, s, ys0, hs, c);
+  y_new = y + h * double(s.A[11]);
+  k12 = sys.rhs_c(STG(y_new), c);
+  solo_add<12>(s, k12);
+  double sc = P.atol + fmax(fabs(y), fabs(y_new)) * P.rtol;
+  if (sizeof(STG) == 4) sc += fabs(h) * P.noise_floor * double(s.m5);
+  const double isc = 1.0 / sc;
+  const double q5 = double(s.a5) * isc, q3 = double(s.a3) * isc;
   double e5 = 0.0, e3 = 0.0;
 #pragma unroll
   for (int i = 0; i < N; ++i) {
@@ -769,28 +946,22 @@ __device__ __forceinline__ double step_attempt_cp(const Sys &sys, const TrajPara
 
 // stages 13..15 and this lane's dense-output coefficients F[0..6]
 template <class Sys, typename STG>
-__device__ __forceinline__ void dense_stages_cp(const Sys &sys, STG (&K)[16][1], double y_old, double y_new,
-                                                double h, STG (&F)[7]) {
+__device__ __forceinline__ void dense_stages_cp(const Sys &sys, STG k0, STG k12, SysSums<Sys, STG> &s, double y_old,
+                                                double y_new, double h, STG (&F)[7]) {
   constexpr int N = Sys::N;
   const int lane = threadIdx.x & 31;
   const int c = lane < N ? lane : N - 1;
   const STG ys0 = STG(y_old);
   const STG hs = STG(h);
-  cp_stage<Sys, STG, 13>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 14>(sys, K, ys0, hs, c);
-  cp_stage<Sys, STG, 15>(sys, K, ys0, hs, c);
+  cp_stage<Sys, STG, 13>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 14>(sys, s, ys0, hs, c);
+  cp_stage<Sys, STG, 15>(sys, s, ys0, hs, c);
   double dy = y_new - y_old;
   F[0] = STG(dy);
-  F[1] = STG(h * double(K[0][0]) - dy);
-  F[2] = STG(2.0 * dy - h * (double(K[12][0]) + double(K[0][0])));
+  F[1] = STG(h * double(k0) - dy);
+  F[2] = STG(2.0 * dy - h * (double(k12) + double(k0)));
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    STG acc = STG(0);
-#pragma unroll
-    for (int j = 0; j < 16; ++j)
-      if (hh_dop853_d[r][j] != 0.0) acc += STG(hh_dop853_d[r][j]) * K[j][0];
-    F[3 + r] = STG(h * double(acc));
-  }
+  for (int r = 0; r < 4; ++r) F[3 + r] = STG(h * double(s.D[r]));
 }
 
 // dense output y(t_old + x h) = y_old + x(F0 + (1-x)(F1 + x(F2 + ... ))); the
@@ -810,6 +981,30 @@ __device__ __forceinline__ void dense_eval(const double *y_old, const STG (&F)[7
     v = (v + F[0][i]) * xs;
     q[i] = y_old[Sys::qidx(i)] + double(v);
   }
+}
+
+// Whether |r(x)| of the dense-output polynomial y = y_old + F0 x + F1 x(1-x) + F2 x^2(1-x)
+// + ... + F6 x^4(1-x)^3 stays below Rcut on [0, 1], with a margin for the evaluation in
+// the stage precision: |r(x)| <= max(|r_old|, |r_old + F0|) + sum_i c_i |F_i|, c_i the
+// maxima of its basis (|r_old + F0 x| is convex in x).  f(r, c): component c of F_r.
+template <typename FF>
+__device__ __forceinline__ bool dense_stays_inside(const FF &f, const double *q, double Rcut) {
+  constexpr double cb[7] = {0.0, 0.25, 4.0 / 27.0, 1.0 / 16.0, 108.0 / 3125.0, 1.0 / 64.0, 6912.0 / 823543.0};
+  double ro2 = 0.0, rn2 = 0.0, f02 = 0.0, tail = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double qo = q[c], f0 = f(0, c);
+    ro2 += qo * qo;
+    rn2 += (qo + f0) * (qo + f0);
+    f02 += f0 * f0;
+  }
+#pragma unroll
+  for (int r = 1; r < 7; ++r) {
+    const double a0 = f(r, 0), a1 = f(r, 1), a2 = f(r, 2);
+    tail += cb[r] * sqrt(a0 * a0 + a1 * a1 + a2 * a2);
+  }
+  const double bound = fmax(sqrt(ro2), sqrt(rn2)) + tail;
+  return bound + 1e-5 * (sqrt(f02) + tail) + 1e-12 * bound < Rcut;
 }
 
 // Per-item set-up, out of line (once per half-trajectory): Cartesian initial
@@ -936,7 +1131,9 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
   // bulk: the whole state per lane; solo: component `lane` (clamped to N - 1) per lane
   constexpr int NL = Sys::SOLO ? 1 : N;
   const int comp = lane < N ? lane : N - 1;
-  STG K[16][NL];
+  // bulk: the stage derivatives; solo: K[0] and K[12] of this lane's component
+  STG K[Sys::SOLO ? 13 : 16][NL];
+  SysSums<Sys, STG> dsum;
   double y[NL], y_new[NL];
   double t = 0.0, h = 0.0;
   PHYS mu0[3] = {PHYS(0), PHYS(0), PHYS(0)};
@@ -1034,6 +1231,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
   auto item_of = [&](unsigned idx) {
     return io.items ? io.items[idx] : (io.fwd_only ? 2 * (int)idx : (int)idx);
   };
+  unsigned long long ctx_slot = ~0ull;  // solo mode, deferred samples: lane 0's reserved context
   bool handing = false;  // bulk mode: this warp hands its open items to the solo kernel
   unsigned round = 0;
   int sync_round = 0;    // bulk mode: rounds since the last block barrier
@@ -1160,7 +1358,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
       } else {
         double err;
         if constexpr (Sys::SOLO)
-          err = step_attempt_cp<Sys, STG>(sys, P, K, y[0], h_att, y_new[0]);
+          err = step_attempt_cp<Sys, STG>(sys, P, K[0][0], y[0], h_att, y_new[0], K[12][0], dsum);
         else
           err = step_attempt<Sys, STG>(sys, P, K, y, h_att, y_new);
         nrhs += 12;
@@ -1191,100 +1389,221 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
     // failure) is cut off per owner with an atomicMin on (end, reason).
     bool pending = accepted && (landed || double(k) * dt <= t + h_taken);
     const double t_land = double(k) * dt;  // REQ: the sample time a landed step ends at
+    // the last sample time the step passed
+    auto last_k = [&]() {
+      const double t_new = t + h_taken;
+      int kl = (int)fmin(floor(t_new / dt), double(P.N - 1));
+      while (kl + 1 <= P.N - 1 && double(kl + 1) * dt <= t_new) ++kl;
+      while (kl > k && double(kl) * dt > t_new) --kl;
+      return REQ && landed ? k : kl;
+    };
+    // the item's status when a sample ended its branch, by the reason of the cut
+    auto end_at_cut = [&](unsigned reason) {
+      switch (reason) {
+        case 0: status = HH_ST_OK; exited = true; break;  // R > Rcut
+        case 1: status = HH_ST_NAN_DIPOLE; hard = 1; break;
+        case 2: status = HH_ST_OVERFLOW; hard = 1; break;
+        case 3: status = HH_ST_JUMP; hard = 1; break;
+        default:
+          status = P.inject_status;
+          hard = (P.inject_status >= HH_ST_NAN_DIPOLE);
+          break;
+      }
+    };
+    // Solo mode: the warp's one item, lane i taking its i-th sample of a chunk of 32.  No
+    // pool: the context is the same for every lane (shared memory, linear), the previous
+    // sample is the lane before, and the first cut is a warp minimum.
+    if constexpr (Sys::SOLO) {
+      if (pending) {
+        STG Fc[7];
+        if constexpr (REQ) {
+          // the sample is the step's end point: y_old + dy at x = 1
+          Fc[0] = STG(y_new[0] - y[0]);
+#pragma unroll
+          for (int r = 1; r < 7; ++r) Fc[r] = STG(0);
+        } else {
+          dense_stages_cp<Sys, STG>(sys, K[0][0], K[12][0], dsum, y[0], y_new[0], h_taken, Fc);
+          nrhs += 3;
+        }
+        ++ndense;
+        constexpr int NQ = Sys::NQ;
+        STG *sF = &ws->F[0][0][0];       // [7][NQ]
+        double *sq = &ws->qold[0][0];    // [NQ]
+#pragma unroll
+        for (int cq = 0; cq < NQ; ++cq)
+          if (Sys::qidx(cq) == lane) {
+#pragma unroll
+            for (int r = 0; r < 7; ++r) sF[r * NQ + cq] = Fc[r];
+            sq[cq] = y[0];
+          }
+        const int cnt = last_k() - k + 1;
+        const double inv_h = 1.0 / h_taken;
+        __syncwarp();
+        bool safe = false;  // deferred samples: no sample of the step passes R > Rcut
+        if constexpr (!Sys::RECORDS)
+          if (defer && cnt > 0)
+            safe = dense_stays_inside([&](int r, int c) { return double(sF[r * NQ + c]); }, sq, P.Rcut);
+        unsigned cut = 0xffffffffu;
+        PHYS tail = curr;
+        if (safe) {
+          if (lane == 0) nsamp += cnt;  // evaluated by the sample kernels
+        } else {
+          for (int base = 0; base < cnt; base += 32) {
+            const int m = min(32, cnt - base);
+            const int j = base + lane, kk = k + j;
+            unsigned code = 0xffffffffu;
+            PHYS val = PHYS(1);
+            bool nan = false, out = false;
+            if (lane < m) {
+              const double x = (double(kk) * dt - t) * inv_h;
+              const STG xs = STG(x), x1 = STG(1) - STG(x);
+              double q[NQ];
+#pragma unroll
+              for (int c = 0; c < NQ; ++c) {
+                if (c >= 3 && defer) {  // deferred: only r, for the R > Rcut test
+                  q[c] = 0.0;
+                  continue;
+                }
+                STG v = sF[6 * NQ + c] * xs;
+                v = (v + sF[5 * NQ + c]) * x1;
+                v = (v + sF[4 * NQ + c]) * xs;
+                v = (v + sF[3 * NQ + c]) * x1;
+                v = (v + sF[2 * NQ + c]) * xs;
+                v = (v + sF[1 * NQ + c]) * x1;
+                v = (v + sF[0 * NQ + c]) * xs;
+                q[c] = sq[c] + double(v);
+              }
+              ++nsamp;
+              out = q[0] * q[0] + q[1] * q[1] + q[2] * q[2] > P.Rcut * P.Rcut;
+              const size_t slot = (size_t)(item >> 1) * io.rec_stride + ((item & 1) ? P.N - 1 + kk : kk);
+              if constexpr (Sys::RECORDS) {
+                PHYS *rec = static_cast<PHYS *>(io.records) + slot * HH_REC_WORDS;
+#pragma unroll
+                for (int c = 0; c < NQ; ++c) rec[c] = PHYS(q[c]);
+              } else if (!defer) {
+                PHYS d[3];
+                sys.dipole(q, d);
+                nan = isnan(d[0]) || isnan(d[1]) || isnan(d[2]);
+                val = mu0[0] * d[0] + mu0[1] * d[1] + mu0[2] * d[2];
+                if (io.series) {
+                  PHYS *sv = static_cast<PHYS *>(io.series) + slot * 4;
+                  const bool zero = P.prmu && nan;
+#pragma unroll
+                  for (int c = 0; c < 3; ++c) sv[c] = zero ? PHYS(0) : d[c];
+                }
+                if (P.prmu && nan) out = false;
+              }
+            }
+            // the reference's per-sample tests (src/hawaii.c:2183-2243), in its order
+            PHYS pv = __shfl_up_sync(FULL, val, 1);
+            if (lane == 0) pv = tail;
+            if (lane < m) {
+              if (Sys::RECORDS || P.prmu || defer) {
+                if (out) code = (unsigned(j + 1) << 3);
+              } else if (nan) code = (unsigned(j) << 3) | 1u;
+              else if (item == P.inject_item && kk == P.inject_k) code = (unsigned(j) << 3) | 4u;
+              else if (fabs(double(val)) > 1e100) code = (unsigned(j) << 3) | 2u;
+              else if (kk > 1 && fabs(double(val) / double(pv)) > 1e10) code = (unsigned(j) << 3) | 3u;
+              else if (out) code = (unsigned(j + 1) << 3);  // stored, then the branch ends
+            }
+            cut = __reduce_min_sync(FULL, code);
+            const int stop = cut == 0xffffffffu ? base + m : min(base + m, int(cut >> 3));
+            if (lane < m && j < stop && !(Sys::RECORDS || io.series || defer)) {
+              if (io.n_sat == 0) {
+                atomicAdd(&crln[kk], P.weight * double(val));
+              } else {
+                for (int s = 0; s < io.n_sat; ++s)
+                  atomicAdd(&crln[(size_t)s * P.N + kk], P.weight * satw[s] * double(val));
+              }
+            }
+            // the item's last stored sample so far, and the last sample of this chunk
+            if (stop > base) curr = __shfl_sync(FULL, val, stop - 1 - base);
+            tail = __shfl_sync(FULL, val, m - 1);
+            if (cut != 0xffffffffu) {
+              if (lane == 0) nsamp += cnt - base - m;  // counted as the pooled path counts them
+              break;
+            }
+          }
+        }
+        const int nc = cut == 0xffffffffu ? cnt : min(cnt, int(cut >> 3));
+        if constexpr (!Sys::RECORDS) {
+          if (defer && nc > 0) {
+            // the context's slot was reserved a step ago, so the atomic's latency is hidden
+            if (lane == 0 && ctx_slot == ~0ull) ctx_slot = atomicAdd(io.ctx_count, 1ull);
+            const unsigned long long idx = __shfl_sync(FULL, ctx_slot, 0);
+            if (idx < io.ctx_cap) {
+              auto *cx = static_cast<SampleCtx<STG, NQ> *>(io.ctx) + idx;
+              for (int e = lane; e < 7 * NQ; e += 32) (&cx->F[0][0])[e] = sF[e];
+              if (lane < NQ) cx->qold[lane] = sq[lane];
+              if (lane == 0) {
+                cx->t0 = t;
+                cx->inv_h = inv_h;
+                cx->item = item;
+                cx->k0 = k;
+                cx->n = nc;
+                cx->prev = last_ctx;
+              }
+            }
+            // past the capacity the host repeats the call with a larger buffer
+            last_ctx = (int)idx;
+            if (lane == 0) ctx_slot = atomicAdd(io.ctx_count, 1ull);
+          }
+        }
+        if (nc > 0) {
+          k += nc;
+          since = 0;
+        }
+        if (cut != 0xffffffffu) end_at_cut(cut & 7u);
+        __syncwarp();
+      }
+    } else
     if (__any_sync(FULL, pending)) {
       int cnt = 0;
       int nsafe = 0;  // deferred samples: stored without per-sample R > Rcut tests
       if (pending) {
         STG F[7][Sys::NQ];
-        if constexpr (Sys::SOLO) {
-          // this lane's component; published below by the lane that holds it
-          STG Fc[7];
-          if constexpr (REQ) {
-            // the sample is the step's end point: y_old + dy at x = 1
-            Fc[0] = STG(y_new[0] - y[0]);
+        if constexpr (REQ) {
+          // the sample is the step's end point: y_old + dy at x = 1
 #pragma unroll
-            for (int r = 1; r < 7; ++r) Fc[r] = STG(0);
-          } else {
-            dense_stages_cp<Sys, STG>(sys, K, y[0], y_new[0], h_taken, Fc);
+          for (int c = 0; c < Sys::NQ; ++c) {
+            F[0][c] = STG(y_new[Sys::qidx(c)] - y[Sys::qidx(c)]);
+#pragma unroll
+            for (int r = 1; r < 7; ++r) F[r][c] = STG(0);
           }
-#pragma unroll
-          for (int cq = 0; cq < Sys::NQ; ++cq)
-            if (Sys::qidx(cq) == lane) {
-#pragma unroll
-              for (int r = 0; r < 7; ++r) ws->F[r][cq][0] = Fc[r];
-              ws->qold[cq][0] = y[0];
-            }
         } else {
-          if constexpr (REQ) {
-#pragma unroll
-            for (int c = 0; c < Sys::NQ; ++c) {
-              F[0][c] = STG(y_new[Sys::qidx(c)] - y[Sys::qidx(c)]);
-#pragma unroll
-              for (int r = 1; r < 7; ++r) F[r][c] = STG(0);
-            }
-          } else {
-            dense_stages<Sys, STG>(sys, K, y, y_new, h_taken, F);
-          }
+          dense_stages<Sys, STG>(sys, K, y, y_new, h_taken, F);
         }
         if (!REQ) nrhs += 3;
         ++ndense;
-        const double t_new = t + h_taken;
-        int kl = (int)fmin(floor(t_new / dt), double(P.N - 1));
-        while (kl + 1 <= P.N - 1 && double(kl + 1) * dt <= t_new) ++kl;
-        while (kl > k && double(kl) * dt > t_new) --kl;
-        if (REQ && landed) kl = k;
-        cnt = owner ? kl - k + 1 : 0;  // solo mode: the owner's samples, evaluated by all lanes
-        if constexpr (!Sys::SOLO && !Sys::RECORDS) {
-          // deferred samples: no sample of the step can pass R > Rcut when the bound
-          // |r(x)| <= max(|r_old|, |r_old + F0|) + sum_i c_i |F_i| of the dense-output
-          // polynomial y = y_old + F0 x + F1 x(1-x) + F2 x^2(1-x) + ... + F6 x^4(1-x)^3
-          // (c_i the maxima of its basis on [0, 1]; |r_old + F0 x| is convex in x) stays
-          // below Rcut with a margin for the FP32 evaluation; such steps store all
-          // their samples without pooled tests
+        cnt = last_k() - k + 1;
+        if constexpr (!Sys::RECORDS) {
+          // deferred samples: a step that stays inside Rcut stores all its samples without
+          // pooled tests
           if (defer && cnt > 0) {
-            constexpr double cb[7] = {0.0, 0.25, 4.0 / 27.0, 1.0 / 16.0, 108.0 / 3125.0, 1.0 / 64.0,
-                                      6912.0 / 823543.0};
-            double ro2 = 0.0, rn2 = 0.0, f02 = 0.0, tail = 0.0;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-              const double qo = y[Sys::qidx(c)], f0 = double(F[0][c]);
-              ro2 += qo * qo;
-              rn2 += (qo + f0) * (qo + f0);
-              f02 += f0 * f0;
-            }
-#pragma unroll
-            for (int r = 1; r < 7; ++r) {
-              const double a0 = F[r][0], a1 = F[r][1], a2 = F[r][2];
-              tail += cb[r] * sqrt(a0 * a0 + a1 * a1 + a2 * a2);
-            }
-            const double bound = fmax(sqrt(ro2), sqrt(rn2)) + tail;
-            if (bound + 1e-5 * (sqrt(f02) + tail) + 1e-12 * bound < P.Rcut) {
+            const double q3[3] = {y[0], y[1], y[2]};
+            if (dense_stays_inside([&](int r, int c) { return double(F[r][c]); }, q3, P.Rcut)) {
               nsafe = cnt;
               nsamp += cnt;  // evaluated by the sample kernels
               cnt = 0;
             }
           }
         }
-        if (owner) {
-          if constexpr (!Sys::SOLO) {
 #pragma unroll
-            for (int r = 0; r < 7; ++r)
+        for (int r = 0; r < 7; ++r)
 #pragma unroll
-              for (int c = 0; c < Sys::NQ; ++c) ws->F[r][c][lane] = F[r][c];
+          for (int c = 0; c < Sys::NQ; ++c) ws->F[r][c][lane] = F[r][c];
 #pragma unroll
-            for (int c = 0; c < Sys::NQ; ++c) ws->qold[c][lane] = y[Sys::qidx(c)];
-          }
+        for (int c = 0; c < Sys::NQ; ++c) ws->qold[c][lane] = y[Sys::qidx(c)];
 #pragma unroll
-          for (int c = 0; c < 3; ++c) ws->mu0[c][lane] = mu0[c];
-          ws->t0[lane] = t;
-          ws->inv_h[lane] = 1.0 / h_taken;
-          ws->prev[lane] = curr;
-          ws->crln[lane] = crln;
-          ws->satw[lane] = satw;
-          ws->kst[lane] = k;
-          ws->item[lane] = item;
-          ws->cut[lane] = 0xffffffffu;
-        }
+        for (int c = 0; c < 3; ++c) ws->mu0[c][lane] = mu0[c];
+        ws->t0[lane] = t;
+        ws->inv_h[lane] = 1.0 / h_taken;
+        ws->prev[lane] = curr;
+        ws->crln[lane] = crln;
+        ws->satw[lane] = satw;
+        ws->kst[lane] = k;
+        ws->item[lane] = item;
+        ws->cut[lane] = 0xffffffffu;
       }
       int incl = cnt;
 #pragma unroll
@@ -1424,7 +1743,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
         if (defer) {
           // one context per owner with stored samples (one atomic per warp)
           int nc = 0;
-          if (pending && owner) {
+          if (pending) {
             const unsigned cut = ws->cut[lane];
             nc = nsafe + ((cut == 0xffffffffu) ? my_off + cnt : min(my_off + cnt, int(cut >> 3))) - my_off;
           }
@@ -1437,14 +1756,13 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
             if (nc > 0) {
               const unsigned long long idx = cbase + __popc(wm & ((1u << lane) - 1u));
               if (idx < io.ctx_cap) {
-                const int col = Sys::SOLO ? 0 : lane;
                 auto *cx = static_cast<SampleCtx<STG, Sys::NQ> *>(io.ctx) + idx;
 #pragma unroll
                 for (int r = 0; r < 7; ++r)
 #pragma unroll
-                  for (int c = 0; c < Sys::NQ; ++c) cx->F[r][c] = ws->F[r][c][col];
+                  for (int c = 0; c < Sys::NQ; ++c) cx->F[r][c] = ws->F[r][c][lane];
 #pragma unroll
-                for (int c = 0; c < Sys::NQ; ++c) cx->qold[c] = ws->qold[c][col];
+                for (int c = 0; c < Sys::NQ; ++c) cx->qold[c] = ws->qold[c][lane];
                 cx->t0 = ws->t0[lane];
                 cx->inv_h = ws->inv_h[lane];
                 cx->item = item;
@@ -1458,7 +1776,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
           }
         }
       }
-      if (pending && owner) {
+      if (pending) {
         const unsigned cut = ws->cut[lane];
         const int stop = (cut == 0xffffffffu) ? my_off + cnt : min(my_off + cnt, int(cut >> 3));
         const int committed = nsafe + stop - my_off;
@@ -1467,27 +1785,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
           curr = ws->last[lane];
           since = 0;
         }
-        if (cut != 0xffffffffu) {
-          switch (cut & 7u) {
-            case 0: status = HH_ST_OK; exited = true; break;  // R > Rcut
-            case 1: status = HH_ST_NAN_DIPOLE; hard = 1; break;
-            case 2: status = HH_ST_OVERFLOW; hard = 1; break;
-            case 3: status = HH_ST_JUMP; hard = 1; break;
-            default:
-              status = P.inject_status;
-              hard = (P.inject_status >= HH_ST_NAN_DIPOLE);
-              break;
-          }
-        }
-      }
-      if constexpr (Sys::SOLO) {
-        // the other lanes follow the owner's progress
-        k = __shfl_sync(FULL, k, 0);
-        curr = __shfl_sync(FULL, curr, 0);
-        since = __shfl_sync(FULL, since, 0);
-        status = __shfl_sync(FULL, status, 0);
-        hard = __shfl_sync(FULL, hard, 0);
-        exited = __shfl_sync(FULL, exited ? 1 : 0, 0) != 0;
+        if (cut != 0xffffffffu) end_at_cut(cut & 7u);
       }
       __syncwarp();
     }
@@ -1604,6 +1902,16 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
         }
       }
       item = -1;
+    }
+  }
+  if constexpr (Sys::SOLO && !Sys::RECORDS) {
+    // a reserved context that was not used holds no samples
+    if (defer && ctx_slot < io.ctx_cap) {
+      auto *cx = static_cast<SampleCtx<STG, Sys::NQ> *>(io.ctx) + ctx_slot;
+      cx->item = 0;
+      cx->k0 = 0;
+      cx->n = 0;
+      cx->prev = -1;
     }
   }
   if (!owner) nsteps = nrej = nrhs = ndense = nitems = 0;  // solo mode: counted once per item
