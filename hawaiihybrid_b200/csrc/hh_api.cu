@@ -154,7 +154,8 @@ struct Ctx {
   DevBuf<int> item_status;
   DevBuf<unsigned> item_fail;
   DevBuf<unsigned char> istart;  // precomputed item starts (ItemStart per item)
-  double defer_est = 32.0;  // contexts per item, from the previous calls
+  // contexts per item per [system][FP64, mixed], from the previous calls (0: none yet)
+  double defer_est[5][2] = {};
   // CORRELATION_ARRAY weights [n][n_sat]: with ratios (C(t)) and without (nstar)
   DevBuf<double> sat_w, sat_wraw;
   // CH4-CO2 record path: sample records, their dipoles, the piece sort
@@ -619,26 +620,35 @@ int run_traj_dispatch(int precision, const TrajParams &P, const TrajIO &io) {
 // ---------------------------------------------------------------------------
 // deferred samples (hh_defer.cuh)
 // ---------------------------------------------------------------------------
-// the mixed path's plain C(t) of the systems with a surface dipole; records, series,
-// satellite temperatures, PR_MU and a failure injection with a soft status keep
-// in-kernel samples.  g_defer (hh_cuda_debug_set_defer; environment HH_DEFER_SAMPLES,
-// default 1): 0 in-kernel samples for every call, 1 deferred for CO2-Ar, 2 also N2-Ar.
-using DeferCtx = SampleCtx<float, 6>;
-constexpr size_t DEFER_CTX_BYTES = sizeof(DeferCtx) + 2 * sizeof(float);  // + first/last value
+// plain C(t) of the systems with a surface dipole; records, series, satellite
+// temperatures, PR_MU and a failure injection with a soft status keep in-kernel samples.
+// g_defer (hh_cuda_debug_set_defer; environment HH_DEFER_SAMPLES, default 1): 0 in-kernel
+// samples for every call; 1 deferred for CO2-Ar on both paths and for N2-Ar in FP64, whose
+// samples are the FP64 network (the mixed N2-Ar dipole is a table lookup, which gains
+// nothing: 365 against 368 ms per iteration); 2 also mixed N2-Ar.  In FP64 (ms per call,
+// samples in the kernel / deferred): CO2-Ar 102,400 x 32,768 222 / 172, its bulk launch
+// 88 / 41; N2-Ar 20,011 x 5,000 205 / 142, its bulk launch 145 / 82.
 int g_defer = [] {
   const char *e = getenv("HH_DEFER_SAMPLES");
   return e ? atoi(e) : 1;
 }();
 bool defer_eligible(int precision, const TrajParams &P, const TrajIO &io) {
-  // the CO2-Ar sample kernel evaluates dipole intervals without exponential terms
-  const bool sys_ok = g.sys == SYS_CO2AR ? g_defer >= 1 && !g_co2ar_dip_exp : (g.sys == SYS_N2AR && g_defer >= 2);
-  return sys_ok && precision == HH_PRECISION_MIXED && io.n_sat == 0 && !io.series && !io.records && !P.prmu &&
+  // the CO2-Ar sample kernels evaluate dipole intervals without exponential terms
+  const bool sys_ok = g.sys == SYS_CO2AR
+                          ? g_defer >= 1 && !g_co2ar_dip_exp
+                          : (g.sys == SYS_N2AR && g_defer >= (precision == HH_PRECISION_MIXED ? 2 : 1));
+  return sys_ok && io.n_sat == 0 && !io.series && !io.records && !P.prmu &&
          (P.inject_item < 0 || P.inject_status >= HH_ST_NAN_DIPOLE);
+}
+
+template <int SYS, typename T> auto defer_eval_fn() {
+  if constexpr (SYS == SYS_CO2AR && sizeof(T) == 4) return defer_eval_co2ar_kernel<float, float>;
+  else return defer_eval_kernel<SYS, T, T>;
 }
 
 // the sample kernels for the contexts of the launch just made with io; n_items and
 // items as io's; traj_base: io.ic's first trajectory in the call (for the fail list)
-template <int SYS>
+template <int SYS, typename T>
 int run_deferred_sys(const TrajParams &P, const TrajIO &io, long long traj_base) {
   DeferArgs a;
   memset(&a, 0, sizeof a);
@@ -651,7 +661,7 @@ int run_deferred_sys(const TrajParams &P, const TrajIO &io, long long traj_base)
   a.item_mu0 = io.item_mu0;
   a.item_fail = g.item_fail.p + 2 * traj_base;
   a.first_v = g.dvals.p;
-  a.last_v = g.dvals.p + io.ctx_cap * sizeof(float);
+  a.last_v = g.dvals.p + io.ctx_cap * sizeof(T);
   a.crln = io.crln;
   a.traj_per_iter = io.traj_per_iter;
   a.inv_traj_per_iter = 1.0 / double(io.traj_per_iter);
@@ -661,10 +671,10 @@ int run_deferred_sys(const TrajParams &P, const TrajIO &io, long long traj_base)
   a.fail_count = io.fail_count;
   a.traj_base = traj_base;
   a.peak = g.dcount.p + DEFER_PEAK;
-  auto eval = SYS == SYS_CO2AR ? defer_eval_co2ar_kernel<float, float> : defer_eval_kernel<SYS_N2AR, float, float>;
-  const size_t smem = DeferSys<SYS, float, float>::smem();
+  auto eval = defer_eval_fn<SYS, T>();
+  const size_t smem = DeferSys<SYS, T, T>::smem();
   if (smem > 48 * 1024) CK(cudaFuncSetAttribute(eval, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  constexpr int threads = defer_eval_threads<SYS>();
+  constexpr int threads = defer_eval_threads<SYS, T>();
   int per_sm = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, eval, threads, smem));
   const int grid = std::max(1, per_sm) * g.num_sms;
@@ -690,9 +700,9 @@ int run_deferred_sys(const TrajParams &P, const TrajIO &io, long long traj_base)
     eval<<<grid, threads, smem, g.st>>>(a, P, io, g.d_tab);
     CK(cudaGetLastError());
   }
-  defer_jump_kernel<float, float, 6><<<8 * g.num_sms, DEFER_THREADS, 0, g.st>>>(a, P);
+  defer_jump_kernel<T, T, 6><<<8 * g.num_sms, DEFER_THREADS, 0, g.st>>>(a, P);
   CK(cudaGetLastError());
-  defer_items_kernel<float><<<(unsigned)std::max(1, (io.n_items + DEFER_THREADS - 1) / DEFER_THREADS),
+  defer_items_kernel<T><<<(unsigned)std::max(1, (io.n_items + DEFER_THREADS - 1) / DEFER_THREADS),
                               DEFER_THREADS, 0, g.st>>>(a, P);
   CK(cudaGetLastError());
   kt_end(HH_KT_SAMPLES);
@@ -700,25 +710,26 @@ int run_deferred_sys(const TrajParams &P, const TrajIO &io, long long traj_base)
   return HH_OK;
 }
 
-// the launch's item starts (mixed path: CO2-Ar, CH4-CO2) into buf, which then backs
-// io.setup
-using DeferStart = ItemStart<12, float, float>;
-using Ch4Start = ItemStart<19, float, float>;
-int run_item_starts(const TrajParams &P, TrajIO &io, unsigned char *buf) {
+// the launch's item starts (CO2-Ar, N2-Ar, CH4-CO2) into buf, which then backs io.setup
+template <typename T> constexpr size_t item_start_bytes(int sys) {
+  return sys == SYS_CH4CO2 ? sizeof(ItemStart<19, T, T>) : sizeof(ItemStart<12, T, T>);
+}
+template <typename T> int run_item_starts_t(const TrajParams &P, TrajIO &io, unsigned char *buf) {
   if (g.sys != SYS_CO2AR && g.sys != SYS_N2AR && g.sys != SYS_CH4CO2) return HH_OK;
+  constexpr bool mixed = sizeof(T) == 4;
   TrajIO is = io;
-  auto k = item_start_kernel<SYS_CH4CO2, float, float>;
+  auto k = item_start_kernel<SYS_CH4CO2, T, T>;
   size_t smem = 0;
   if (g.sys == SYS_CO2AR) {
-    k = item_start_kernel<SYS_CO2AR, float, float>;
-    smem = smem_tables_bytes<float>();
+    k = item_start_kernel<SYS_CO2AR, T, T>;
+    smem = smem_tables_bytes<T>();
   } else if (g.sys == SYS_N2AR) {
-    // the mixed path's networks, as run_traj_dispatch gives them
-    k = item_start_kernel<SYS_N2AR, float, float>;
-    smem = sizeof(N2arDipFold) + sizeof(N2arPesNet<float>);
+    // the networks as run_traj_dispatch gives them
+    k = item_start_kernel<SYS_N2AR, T, T>;
+    smem = sizeof(N2arDipFold) + sizeof(N2arPesNet<T>);
     is.dipnet = g.d_n2ar_fold;
-    is.pesnet = g.d_n2ar_pes_f;
-    is.diptab = g.d_n2ar_tab;
+    is.pesnet = mixed ? (const void *)g.d_n2ar_pes_f : (const void *)g.d_n2ar_pes_d;
+    is.diptab = mixed ? g.d_n2ar_tab : nullptr;
   }
   if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   int per_sm = 0;
@@ -732,15 +743,21 @@ int run_item_starts(const TrajParams &P, TrajIO &io, unsigned char *buf) {
   io.setup = buf;
   return HH_OK;
 }
+int run_item_starts(int precision, const TrajParams &P, TrajIO &io, unsigned char *buf) {
+  return precision == HH_PRECISION_MIXED ? run_item_starts_t<float>(P, io, buf) : run_item_starts_t<double>(P, io, buf);
+}
 
-int run_deferred(const TrajParams &P, const TrajIO &io, long long traj_base) {
+int run_deferred(int precision, const TrajParams &P, const TrajIO &io, long long traj_base) {
+  const bool mixed = precision == HH_PRECISION_MIXED;
   if (g.sys == SYS_N2AR) {
     TrajIO io2 = io;
     io2.dipnet = g.d_n2ar_fold;
-    io2.diptab = g.d_n2ar_tab;
-    return run_deferred_sys<SYS_N2AR>(P, io2, traj_base);
+    io2.diptab = mixed ? g.d_n2ar_tab : nullptr;
+    return mixed ? run_deferred_sys<SYS_N2AR, float>(P, io2, traj_base)
+                 : run_deferred_sys<SYS_N2AR, double>(P, io2, traj_base);
   }
-  return run_deferred_sys<SYS_CO2AR>(P, io, traj_base);
+  return mixed ? run_deferred_sys<SYS_CO2AR, float>(P, io, traj_base)
+               : run_deferred_sys<SYS_CO2AR, double>(P, io, traj_base);
 }
 
 // device memory the CH4-CO2 record path may hold for one chunk of trajectories
@@ -902,8 +919,8 @@ int run_records_t(const TrajParams &P, const double *d_ic, uint64_t n, uint64_t 
     io.item_trace = trace ? trace + 2 * base : nullptr;
     if (precision == HH_PRECISION_MIXED) {
       // item starts precomputed, one thread per item (the refills then load them)
-      CK(g.istart.ensure(2 * chunk * sizeof(Ch4Start)));
-      int rc1 = run_item_starts(P, io, g.istart.p);
+      CK(g.istart.ensure(2 * chunk * item_start_bytes<float>(SYS_CH4CO2)));
+      int rc1 = run_item_starts_t<float>(P, io, g.istart.p);
       if (rc1) return rc1;
     }
     int rc = (precision == HH_PRECISION_MIXED) ? launch_traj<SYS_CH4CO2, float, float, false>(P, io, nullptr)
@@ -1094,7 +1111,8 @@ int traj_block_sync() {
 // (the reference drops a trajectory whose correlation_eval returns 1 while still
 // counting it: both branches are replayed with the opposite weight).  With deferred
 // samples the iterations go in launches whose sample contexts fit the buffer (at most
-// 32 GiB and 40 % of the free memory, or HH_DEFER_BUDGET_MB); a launch that wrote
+// 32 GiB and 40 % of the free memory, or HH_DEFER_BUDGET_MB; in FP64, whose contexts are
+// larger, an iteration that does not fit goes in several launches); a launch that wrote
 // more contexts than the buffer holds repeats the call with a larger estimate of
 // contexts per item (HH_DEFER_EST sets the first one), and a second overflow with
 // in-kernel samples.
@@ -1102,6 +1120,13 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
               uint64_t n_iter, int *nfail_out) {
   const size_t N = (size_t)P.N;
   const bool eligible = defer_eligible(precision, P, io0);
+  const bool mixed = precision == HH_PRECISION_MIXED;
+  const size_t vb = mixed ? sizeof(float) : sizeof(double);
+  const size_t ctx_b = mixed ? sizeof(SampleCtx<float, 6>) : sizeof(SampleCtx<double, 6>);
+  const size_t start_b = mixed ? item_start_bytes<float>(g.sys) : item_start_bytes<double>(g.sys);
+  double &est = g.defer_est[g.sys][mixed ? 1 : 0];
+  // contexts per item: about 21 (mixed), 70 (CO2-Ar FP64) and 100 (N2-Ar FP64)
+  if (est == 0.0) est = mixed ? 32.0 : 128.0;
   for (int attempt = 0;; ++attempt) {
     const bool defer = eligible && attempt < 2;
     if (attempt > 0) {
@@ -1114,35 +1139,37 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     CK(cudaMemsetAsync(g.queue.p, 0, sizeof(unsigned int), g.st));
     TrajIO io = io0;
     unsigned long long cap = 0;
-    uint64_t it_launch = n_iter, items_launch = 2 * n;
+    uint64_t it_launch = n_iter, tr_launch = n, items_launch = 2 * n;
     if (defer) {
       size_t free_b = 0, total_b = 0;
       CK(cudaMemGetInfo(&free_b, &total_b));
       double budget = std::min(32.0 * double(1ull << 30), 0.4 * double(free_b + g.dctx.cap + g.dvals.cap));
       if (const char *eb = getenv("HH_DEFER_BUDGET_MB")) budget = std::max(1.0, atof(eb)) * double(1 << 20);
       if (attempt == 0)
-        if (const char *ee = getenv("HH_DEFER_EST")) g.defer_est = std::max(0.01, atof(ee));
-      const double per_item = g.defer_est * double(DEFER_CTX_BYTES);
+        if (const char *ee = getenv("HH_DEFER_EST")) est = std::max(0.01, atof(ee));
+      const double per_item = est * double(ctx_b + 2 * vb);
       const uint64_t max_items = (uint64_t)std::max(1.0, budget / per_item);
       it_launch = std::min<uint64_t>(n_iter, std::max<uint64_t>(1, max_items / (2 * per_iter)));
-      items_launch = 2 * std::min<uint64_t>(n, it_launch * per_iter);
-      cap = (unsigned long long)(g.defer_est * double(items_launch)) + 4096ull;
+      tr_launch = std::min<uint64_t>(n, it_launch * per_iter);
+      if (!mixed) tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
+      items_launch = 2 * tr_launch;
+      cap = (unsigned long long)(est * double(items_launch)) + 4096ull;
       if (getenv("HH_DEFER_TRACE"))
-        fprintf(stderr, "[defer] attempt %d est %.3f items %llu cap %llu (buffer %llu) launches of %llu iterations, "
-                "budget %.2f GB, free %.2f GB\n", attempt, g.defer_est, (unsigned long long)items_launch, cap,
-                (unsigned long long)(g.dctx.cap / sizeof(DeferCtx)), (unsigned long long)it_launch, budget / 1e9,
+        fprintf(stderr, "[defer] attempt %d est %.3f items %llu cap %llu (buffer %llu) launches of %llu trajectories, "
+                "budget %.2f GB, free %.2f GB\n", attempt, est, (unsigned long long)items_launch, cap,
+                (unsigned long long)(g.dctx.cap / ctx_b), (unsigned long long)tr_launch, budget / 1e9,
                 free_b / 1e9);
       // 10 % headroom: the estimate moves a little from call to call, and a larger
       // buffer would otherwise be reallocated (cudaFree and cudaMalloc of gigabytes)
       // inside a call
       const size_t alloc = (size_t)(1.1 * double(cap));
-      if (g.dctx.cap < cap * sizeof(DeferCtx)) CK(g.dctx.ensure(alloc * sizeof(DeferCtx)));
-      if (g.dvals.cap < cap * 2 * sizeof(float)) CK(g.dvals.ensure(alloc * 2 * sizeof(float)));
+      if (g.dctx.cap < cap * ctx_b) CK(g.dctx.ensure(alloc * ctx_b));
+      if (g.dvals.cap < cap * 2 * vb) CK(g.dvals.ensure(alloc * 2 * vb));
       CK(g.dcount.ensure(DEFER_WORDS));
       CK(g.item_status.ensure(2 * n));
-      CK(g.item_mu0.ensure(2 * n * 4 * sizeof(float)));
+      CK(g.item_mu0.ensure(2 * n * 4 * vb));
       CK(g.item_fail.ensure(2 * n));
-      if (g.sys == SYS_CO2AR) CK(g.istart.ensure(2 * n * sizeof(DeferStart)));
+      CK(g.istart.ensure(2 * n * start_b));
       CK(cudaMemsetAsync(g.item_fail.p, 0xff, 2 * n * sizeof(unsigned), g.st));
       CK(cudaMemsetAsync(g.dcount.p, 0, 2 * sizeof(unsigned long long), g.st));
       io.ctx = g.dctx.p;
@@ -1153,36 +1180,40 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     }
     // item starts precomputed for the mixed N2-Ar path (its refill set-up evaluates the
     // PIP-NN surface twice and the dipole once on one lane)
-    const bool starts = !defer && precision == HH_PRECISION_MIXED && g.sys == SYS_N2AR && io.n_sat == 0 &&
-                        !io.series && !io.records;
+    const bool starts = !defer && mixed && g.sys == SYS_N2AR && io.n_sat == 0 && !io.series && !io.records;
     if (!defer) {
       if (starts) {
-        CK(g.istart.ensure(2 * n * sizeof(DeferStart)));
-        int rc = run_item_starts(P, io, g.istart.p);
+        CK(g.istart.ensure(2 * n * start_b));
+        int rc = run_item_starts(precision, P, io, g.istart.p);
         if (rc) return rc;
       }
       int rc = run_traj_dispatch(precision, P, io);
       if (rc) return rc;
     } else {
-      for (uint64_t i0 = 0; i0 < n_iter; i0 += it_launch) {
-        const uint64_t t0 = i0 * per_iter, t1 = std::min(n, (i0 + it_launch) * per_iter);
+      uint64_t t1 = 0;
+      for (uint64_t t0 = 0; t0 < n; t0 = t1) {
+        // whole iterations, or (FP64) a part of one
+        const uint64_t i0 = t0 / per_iter;
+        const bool part = tr_launch < per_iter;
+        t1 = part ? std::min({n, (i0 + 1) * per_iter, t0 + tr_launch}) : std::min(n, (i0 + it_launch) * per_iter);
         TrajIO il = io;
         il.ic = io.ic + t0 * (uint64_t)g.QP;
         il.n_items = (int)(2 * (t1 - t0));
         il.crln = io.crln + i0 * N;
+        if (part) il.traj_per_iter = LLONG_MAX / 4;
         il.fail_flag = io.fail_flag + t0;
         il.item_status = g.item_status.p + 2 * t0;
-        il.item_mu0 = g.item_mu0.p + 2 * t0 * 4 * sizeof(float);
+        il.item_mu0 = g.item_mu0.p + 2 * t0 * 4 * vb;
         il.item_trace = io.item_trace ? io.item_trace + 2 * t0 : nullptr;
-        if (i0 > 0) {
+        if (t0 > 0) {
           CK(cudaMemsetAsync(g.queue.p, 0, sizeof(unsigned int), g.st));
           CK(cudaMemsetAsync(g.dcount.p, 0, sizeof(unsigned long long), g.st));
         }
-        int rc = run_item_starts(P, il, g.istart.p + 2 * t0 * sizeof(DeferStart));
+        int rc = run_item_starts(precision, P, il, g.istart.p + 2 * t0 * start_b);
         if (rc) return rc;
         rc = run_traj_dispatch(precision, P, il);
         if (rc) return rc;
-        rc = run_deferred(P, il, (long long)t0);
+        rc = run_deferred(precision, P, il, (long long)t0);
         if (rc) return rc;
       }
     }
@@ -1194,10 +1225,10 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     if (defer) {
       const double per = double(peak) / double(std::max<uint64_t>(1, items_launch));
       if (peak > cap) {
-        g.defer_est = std::max(2.0 * g.defer_est, 1.25 * per);
+        est = std::max(2.0 * est, 1.25 * per);
         continue;
       }
-      g.defer_est = std::max(8.0, 1.25 * per);
+      est = std::max(8.0, 1.25 * per);
     }
     if (nfail > 0) {
       std::vector<int> fl(nfail), it(2 * (size_t)nfail);
@@ -1219,23 +1250,22 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       io2.status_hist = g.status_hist.p + HH_ST_COUNT;
       io2.item_trace = nullptr;
       if (defer) {
-        io2.ctx_cap = g.dctx.cap / sizeof(DeferCtx);
-        if (io2.ctx_cap > g.dvals.cap / (2 * sizeof(float))) io2.ctx_cap = g.dvals.cap / (2 * sizeof(float));
+        io2.ctx_cap = std::min(g.dctx.cap / ctx_b, g.dvals.cap / (2 * vb));
         CK(cudaMemsetAsync(g.dcount.p, 0, 2 * sizeof(unsigned long long), g.st));
       }
       if (defer || starts) {
-        int rc = run_item_starts(P2, io2, g.istart.p);
+        int rc = run_item_starts(precision, P2, io2, g.istart.p);
         if (rc) return rc;
       }
       int rc = run_traj_dispatch(precision, P2, io2);
       if (rc) return rc;
       if (defer) {
-        rc = run_deferred(P2, io2, 0);
+        rc = run_deferred(precision, P2, io2, 0);
         if (rc) return rc;
         CK(cudaMemcpyAsync(&peak, g.dcount.p + DEFER_PEAK, sizeof peak, cudaMemcpyDeviceToHost, g.st));
         CK(cudaStreamSynchronize(g.st));
         if (peak > io2.ctx_cap) {
-          g.defer_est *= 2.0;
+          est *= 2.0;
           continue;
         }
       }
@@ -2538,6 +2568,13 @@ void hh_cuda_shutdown(void) {
   g.zf_a.release();
   g.zf_b.release();
   g.hcount.release();
+  g.dctx.release();
+  g.dvals.release();
+  g.item_mu0.release();
+  g.dcount.release();
+  g.item_status.release();
+  g.item_fail.release();
+  g.istart.release();
   g.trace.release();
   g.sat_w.release();
   g.sat_wraw.release();

@@ -7,9 +7,9 @@
 // With io.ctx set the kernel interpolates only r (for the reference's R > Rcut exit,
 // src/hawaii.c:2244) and writes one SampleCtx per dense-output step; the kernels here
 // then run the per-sample work at full occupancy:
-//   defer_eval_co2ar_kernel (CO2-Ar) and defer_eval_kernel (N2-Ar)
+//   defer_eval_co2ar_kernel (CO2-Ar, mixed) and defer_eval_kernel (N2-Ar, CO2-Ar in FP64)
 //                       pooled (context, sample) pairs, 32 lanes per warp round (two
-//                       samples per lane for CO2-Ar): y(t_k) from the context, the
+//                       samples per lane for mixed CO2-Ar): y(t_k) from the context, the
 //                       dipole, mu0 . mu(t_k) into C(t_k), and the reference's
 //                       per-sample tests (src/hawaii.c:2183-2243: NaN dipole, |value| >
 //                       1e100, |value / previous| > 1e10 for k > 1) within the context,
@@ -37,9 +37,18 @@
 namespace hh {
 
 constexpr int DEFER_THREADS = 256;
-// block size of the sample kernels: CO2-Ar in blocks of two warps, which fit into the
-// registers that finished solo-kernel warps release while the solo kernel still runs
-template <int SYS> constexpr int defer_eval_threads() { return SYS == SYS_CO2AR ? 64 : DEFER_THREADS; }
+// block size of the sample kernels: mixed CO2-Ar in blocks of two warps, which fit into the
+// registers that finished solo-kernel warps release while the solo kernel still runs;
+// FP64 N2-Ar in blocks of four, three of which share an SM's registers and shared memory
+// (12 warps against 8 in one block of eight)
+template <int SYS, typename T> constexpr int defer_eval_threads() {
+  return SYS == SYS_CO2AR && sizeof(T) == 4 ? 64 : SYS == SYS_N2AR && sizeof(T) == 8 ? 128 : DEFER_THREADS;
+}
+// blocks per SM the one-sample-per-lane kernel's register allocation must allow: two for
+// CO2-Ar (128 registers a thread), three of the smaller FP64 N2-Ar ones (170)
+template <int SYS, typename T> constexpr int defer_eval_min_blocks() {
+  return SYS == SYS_CO2AR ? 2 : sizeof(T) == 8 ? 3 : 1;
+}
 // words of the context counter block: the count the trajectory kernels advance, the
 // largest count of a call, and the snapshot of the count after the bulk kernel
 constexpr int DEFER_COUNT = 0, DEFER_PEAK = 1, DEFER_SNAP = 2, DEFER_WORDS = 3;
@@ -101,7 +110,7 @@ struct DeferCo2arDip {
   int fdip[CO2AR_NINT];
   unsigned char ivl[164];               // interval of R in [j / 4, (j + 1) / 4), j <= 160
 };
-template <typename PHYS, typename STG> struct DeferSys<SYS_CO2AR, PHYS, STG> {
+template <> struct DeferSys<SYS_CO2AR, float, float> {
   static constexpr int NQ = 6;
   static constexpr size_t smem() { return (sizeof(DeferCo2arDip) + 15) / 16 * 16; }
   const DeferCo2arDip *t;
@@ -199,8 +208,79 @@ template <typename PHYS, typename STG> struct DeferSys<SYS_CO2AR, PHYS, STG> {
     for (int c = 0; c < 3; ++c) d[c] = fma2(nax, fma2(nx, rh[c], uh[c]), mul2(dz, rh[c]));
   }
 };
+// (319e6 samples, 102,400 trajectories x 32,768: 13.7 ms.)
+// The FP64 path's CO2-Ar dipole: the same interleaved (z, x) rows and interval lookup in
+// FP64, one sample per lane.  Consecutive samples lie in the same interval or the next,
+// so a warp's 16-byte row loads are broadcasts of one or two rows.
+struct DeferCo2arDipD {
+  double2 row[CO2AR_NINT][CO2AR_NL][8];  // coefficient k of the (z, x) rows: a0..a3, b4..b7
+  double rlo[CO2AR_NINT];
+  int fdip[CO2AR_NINT];
+  unsigned char ivl[164];                // interval of R in [j / 4, (j + 1) / 4), j <= 160
+};
+template <> struct DeferSys<SYS_CO2AR, double, double> {
+  static constexpr int NQ = 6;
+  static constexpr bool WARP = false;
+  static constexpr size_t smem() { return (sizeof(DeferCo2arDipD) + 15) / 16 * 16; }
+  const DeferCo2arDipD *t;
+  __device__ void init(unsigned char *sm, const Co2arTablesGlobal *g, const TrajIO &) {
+    auto *d = reinterpret_cast<DeferCo2arDipD *>(sm);
+    double2 *w = &d->row[0][0][0];
+    for (int e = threadIdx.x; e < CO2AR_NINT * CO2AR_NL * 8; e += blockDim.x) {
+      const int r = (e / 8) * CO2AR_ROW + e % 8;
+      w[e] = make_double2(g->dipz[r], g->dipx[r]);
+    }
+    for (int i = threadIdx.x; i < CO2AR_NINT; i += blockDim.x) {
+      d->rlo[i] = g->rlo[i];
+      d->fdip[i] = g->fdip[i];
+    }
+    for (int j = threadIdx.x; j < 164; j += blockDim.x) {
+      const double r = 0.25 * j;
+      int i = 0;
+      while (i < CO2AR_NINT - 1 && !(r < g->rbound[i])) ++i;
+      d->ivl[j] = (unsigned char)i;
+    }
+    t = d;
+  }
+  // q = (r[3], u[3]): mu = dz r^ - ax (u^ - x r^), dz = sum_l z_l P_l(x), ax = sum_l x_l P_l'(x)
+  __device__ __forceinline__ void dipole(const double *q, double d[3]) const {
+    const double R2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
+    const double iR = rsqrt(R2), iu = rsqrt(q[3] * q[3] + q[4] * q[4] + q[5] * q[5]);
+    const double rh[3] = {q[0] * iR, q[1] * iR, q[2] * iR};
+    const double uh[3] = {q[3] * iu, q[4] * iu, q[5] * iu};
+    const double x = rh[0] * uh[0] + rh[1] * uh[1] + rh[2] * uh[2];
+    const double R = R2 * iR;
+    const int i = t->ivl[min(int(R * 4.0), 163)];
+    const double tt = R - t->rlo[i];
+    const bool inv = t->fdip[i] & 1;
+    const double iR2 = iR * iR, iR4 = iR2 * iR2, iR5 = iR4 * iR, iR6 = iR4 * iR2, iR7 = iR5 * iR2;
+    double P0 = 1.0, P1 = x, dP = 0.0, dz = 0.0, ax = 0.0;  // P_l and P_{l+1}, P_l' at l = 2 li
+#pragma unroll
+    for (int li = 0; li < CO2AR_NL; ++li) {
+      const double2 *w = t->row[i][li];
+      double cz = ((w[3].x * tt + w[2].x) * tt + w[1].x) * tt + w[0].x;
+      double cx = ((w[3].y * tt + w[2].y) * tt + w[1].y) * tt + w[0].y;
+      if (inv) {
+        cz += w[4].x * iR4 + w[5].x * iR5 + w[6].x * iR6 + w[7].x * iR7;
+        cx += w[4].y * iR4 + w[5].y * iR5 + w[6].y * iR6 + w[7].y * iR7;
+      }
+      dz += P0 * cz;
+      ax += dP * cx;
+      if (li + 1 < CO2AR_NL) {
+        const int l = 2 * li + 1;  // P_l = P1: to P_{l+1} and P_{l+2}
+        dP += double(2 * l + 1) * P1;
+        const double a = (double(2 * l + 1) * x * P1 - double(l) * P0) * (1.0 / double(l + 1));
+        P1 = (double(2 * l + 3) * x * a - double(l + 1) * P1) * (1.0 / double(l + 2));
+        P0 = a;
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) d[c] = dz * rh[c] - ax * (uh[c] - x * rh[c]);
+  }
+};
 template <typename PHYS, typename STG> struct DeferSys<SYS_N2AR, PHYS, STG> {
   static constexpr int NQ = 6;
+  static constexpr bool WARP = false;  // the dipole is per lane
   static constexpr size_t smem() { return sizeof(N2arDipFold); }
   N2ArSys<PHYS, STG, false, false> sys;
   __device__ void init(unsigned char *sm, const Co2arTablesGlobal *, const TrajIO &io) {
@@ -210,8 +290,175 @@ template <typename PHYS, typename STG> struct DeferSys<SYS_N2AR, PHYS, STG> {
     sys.pes = nullptr;
     sys.dtab = static_cast<const float4 *>(io.diptab);
   }
-  static constexpr bool FLOAT_Q = false;
   __device__ __forceinline__ void dipole(const double *q, PHYS d[3]) const { sys.dipole(q, d); }
+};
+
+// The FP64 path's N2-Ar dipole: the network of n2ar_dip_body for the 32 samples of a warp at
+// once.  Its first layer is a dense contraction, dh (32 x 40) = z (32 x 34) w (34 x 40) per
+// charge model, and runs on the FP64 tensor cores (mma.sync m8n8k4: the fifth-generation
+// tcgen05 has no FP64 form); per lane it was bound by the shared-memory reads of the
+// weights (17.9 TFLOP/s at best with one sample per lane in a loop of 16-byte broadcasts,
+// against 36.9 TFLOP/s of the FP64 mma).  The monomials go through shared memory into the
+// A fragments, the weights lie there in B-fragment order, and each lane applies the SiLU
+// differences to the 40 (sample, unit) sums of its C fragments.  62.8e6 samples (20,011
+// trajectories x 5,000): 47.0 -> 19.6 ms.
+constexpr int N2D_KS = (N2AR_NZ + 3) / 4;  // k steps of 4 monomials (two zero rows at the end)
+constexpr int N2D_NT = N2AR_NH / 8;        // tiles of 8 hidden units
+constexpr int N2D_ZROW = 36;               // doubles per monomial row of a warp's z buffer (conflict-free)
+static_assert(N2AR_NH % 8 == 0, "whole unit tiles");
+struct N2arDipFrag {
+  double w[2][N2D_KS][N2D_NT][32];  // B fragments: lane l holds w[k = 4 ks + l % 4][n = 8 nt + l / 4]
+  double e0[2][N2AR_NH], c1[2][N2AR_NH], wo[2][N2AR_NH];
+};
+__device__ __forceinline__ void dmma_8x8x4(double (&c)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(c[0]), "+d"(c[1])
+      : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void n2ar_frag_init(N2arDipFrag *f, const N2arDipFold *g) {
+  for (int i = threadIdx.x; i < 2 * N2D_KS * N2D_NT * 32; i += blockDim.x) {
+    const int l = i % 32, nt = i / 32 % N2D_NT, ks = i / (32 * N2D_NT) % N2D_KS, m = i / (32 * N2D_NT * N2D_KS);
+    const int k = 4 * ks + l % 4, n = 8 * nt + l / 4;
+    (&f->w[0][0][0][0])[i] = k < N2AR_NZ ? g->w[m][k][n] : 0.0;
+  }
+  for (int i = threadIdx.x; i < 2 * N2AR_NH; i += blockDim.x) {
+    (&f->e0[0][0])[i] = (&g->e0[0][0])[i];
+    (&f->c1[0][0])[i] = (&g->c1[0][0])[i];
+    (&f->wo[0][0])[i] = (&g->wo[0][0])[i];
+  }
+}
+// body-frame dipoles of the warp's 32 samples (lane i: sample i at R, c = cos T; all lanes
+// call).  zb: this warp's [4 N2D_KS][N2D_ZROW] buffer, its last rows zero.
+__device__ __forceinline__ N2arDipBody<double> n2ar_dip_warp(const N2arDipFrag *F, double *zb, double R, double c) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, quad = lane & 3, row = lane >> 2;
+  const double h = N2AR_L / 2.0;
+  const double s = sqrt(fmax(0.0, (1.0 - c) * (1.0 + c)));
+  const double base = h * h + R * R, hc = 2.0 * h * c * R, hs = 2.0 * h * s * R;
+  // the varying distances N1-Ar, N2-Ar, N1'-Ar, N2'-Ar
+  const double dv[4] = {sqrt(base - hc), sqrt(base + hc), sqrt(base + hs), sqrt(base - hs)};
+  const double sw = n2ar_switch(R, 9.5, 12.5);
+  N2arDipBody<double> out = {0.0, 0.0};
+#pragma unroll 1
+  for (int m = 0; m < 2; ++m) {
+    const double wm = (m == 0) ? 1.0 - sw : sw;
+    if (!__any_sync(FULL, wm != 0.0)) continue;
+    const double ia0 = (m == 0) ? 0.5 : 1.0 / 6.0;
+    double v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = exp(-dv[i] * ia0);
+    double *z = zb + lane;
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) z[N2D_ZROW * k++] = v[i];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j) z[N2D_ZROW * k++] = v[i] * v[j];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = i; j < 4; ++j)
+#pragma unroll
+        for (int l = j; l < 4; ++l) z[N2D_ZROW * k++] = v[i] * v[j] * v[l];
+    __syncwarp();
+    // dh: four tiles of 8 samples x five of 8 units; this lane's C entries are the samples
+    // 8 mt + row and the units 8 nt + 2 quad, 8 nt + 2 quad + 1
+    double dh[4][N2D_NT][2];
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt)
+#pragma unroll
+      for (int nt = 0; nt < N2D_NT; ++nt) dh[mt][nt][0] = dh[mt][nt][1] = 0.0;
+#pragma unroll 3
+    for (int ks = 0; ks < N2D_KS; ++ks) {
+      double a[4];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) a[mt] = zb[(4 * ks + quad) * N2D_ZROW + 8 * mt + row];
+#pragma unroll
+      for (int nt = 0; nt < N2D_NT; ++nt) {
+        const double b = F->w[m][ks][nt][lane];
+#pragma unroll
+        for (int mt = 0; mt < 4; ++mt) dmma_8x8x4(dh[mt][nt], a[mt], b);
+      }
+    }
+    __syncwarp();
+    // partial sums over this lane's units: A (units 0..15), B (16..31), Q (32..39)
+    double A[4] = {0.0, 0.0, 0.0, 0.0}, B[4] = {0.0, 0.0, 0.0, 0.0}, Q[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int nt = 0; nt < N2D_NT; ++nt) {
+      // this lane's two units of the tile: t = sd (d - c1 u) wo with sd = 1 / (1 + e0 + e0 u),
+      // both quotients over one denominator (one division for two units)
+      const int j = 8 * nt + 2 * quad;
+      const double e0 = F->e0[m][j], f0 = F->c1[m][j], g0 = F->wo[m][j];
+      const double e1 = F->e0[m][j + 1], f1 = F->c1[m][j + 1], g1 = F->wo[m][j + 1];
+#pragma unroll
+      for (int mt = 0; mt < 4; ++mt) {
+        const double d0 = dh[mt][nt][0], d1 = dh[mt][nt][1], u0 = expm1(-d0), u1 = expm1(-d1);
+        const double q0 = 1.0 + (e0 + e0 * u0), q1 = 1.0 + (e1 + e1 * u1);
+        const double n0 = (d0 - f0 * u0) * g0, n1 = (d1 - f1 * u1) * g1;
+        const double t = (n0 * q1 + n1 * q0) / (q0 * q1);
+        if (nt < 2) A[mt] += t;
+        else if (nt < 4) B[mt] += t;
+        else Q[mt] += t;
+      }
+    }
+    // over the four lanes of a row, then from the row's lanes to the sample's lane
+    double a = 0.0, b = 0.0, q = 0.0;
+#pragma unroll
+    for (int mt = 0; mt < 4; ++mt) {
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        A[mt] += __shfl_xor_sync(FULL, A[mt], o);
+        B[mt] += __shfl_xor_sync(FULL, B[mt], o);
+        Q[mt] += __shfl_xor_sync(FULL, Q[mt], o);
+      }
+      const int src = 4 * (lane & 7);
+      const double as = __shfl_sync(FULL, A[mt], src), bs = __shfl_sync(FULL, B[mt], src),
+                   qs = __shfl_sync(FULL, Q[mt], src);
+      if ((lane >> 3) == mt) {
+        a = as;
+        b = bs;
+        q = qs;
+      }
+    }
+    if (wm != 0.0) {
+      out.dx += wm * (h * s * a + h * c * b);
+      out.dz += wm * (h * c * a - h * s * b + R * q);
+    }
+  }
+  return out;
+}
+// body-frame (d_x, d_z) to the lab: N2ArSys::dipole around n2ar_dip_warp (all lanes call)
+__device__ __forceinline__ void n2ar_dipole_warp(const N2arDipFrag *F, double *zb, const double *q, double d[3]) {
+  const double R2 = q[0] * q[0] + q[1] * q[1] + q[2] * q[2];
+  const double iR = rsqrt(R2);
+  const double iu = rsqrt(q[3] * q[3] + q[4] * q[4] + q[5] * q[5]);
+  const double rh[3] = {q[0] * iR, q[1] * iR, q[2] * iR};
+  const double uh[3] = {q[3] * iu, q[4] * iu, q[5] * iu};
+  const double x = rh[0] * uh[0] + rh[1] * uh[1] + rh[2] * uh[2];
+  const double e[3] = {uh[0] - x * rh[0], uh[1] - x * rh[1], uh[2] - x * rh[2]};
+  const double en2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
+  const double ie = en2 > 0.0 ? rsqrt(en2) : 0.0;
+  const N2arDipBody<double> b = n2ar_dip_warp(F, zb, R2 * iR, x);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) d[c] = b.dz * rh[c] + b.dx * e[c] * ie;
+}
+
+template <> struct DeferSys<SYS_N2AR, double, double> {
+  static constexpr int NQ = 6;
+  static constexpr bool WARP = true;  // the warp's dipoles together, all lanes calling
+  static constexpr int ZB = 4 * N2D_KS * N2D_ZROW;
+  static constexpr size_t smem() { return sizeof(N2arDipFrag) + defer_eval_threads<SYS_N2AR, double>() / 32 * ZB * sizeof(double); }
+  const N2arDipFrag *f;
+  double *zb;
+  __device__ void init(unsigned char *sm, const Co2arTablesGlobal *, const TrajIO &io) {
+    auto *fr = reinterpret_cast<N2arDipFrag *>(sm);
+    n2ar_frag_init(fr, static_cast<const N2arDipFold *>(io.dipnet));
+    f = fr;
+    zb = reinterpret_cast<double *>(sm + sizeof(N2arDipFrag)) + (threadIdx.x >> 5) * ZB;
+    for (int i = N2AR_NZ * N2D_ZROW + (threadIdx.x & 31); i < ZB; i += 32) zb[i] = 0.0;
+  }
+  __device__ __forceinline__ void dipole(const double *q, double d[3]) const { n2ar_dipole_warp(f, zb, q, d); }
 };
 
 // The C(t) slice of an item: its trajectory's iteration, (item / 2) / traj_per_iter,
@@ -238,6 +485,26 @@ __device__ __forceinline__ unsigned sample_code(float v, bool nan, int kk, bool 
   return 0xffffffffu;
 }
 
+// The same on an FP64 value: the overflow test is |v| > 1e100.
+__device__ __forceinline__ unsigned sample_code(double v, bool nan, int kk, bool inject, bool jump, double pv) {
+  if (nan) return (unsigned(kk) << 3) | 1u;
+  if (inject) return (unsigned(kk) << 3) | 4u;
+  if (fabs(v) > 1e100) return (unsigned(kk) << 3) | 2u;
+  if (jump && fabs(v) > 1e10 * fabs(pv)) return (unsigned(kk) << 3) | 3u;
+  return 0xffffffffu;
+}
+// whether a sample value goes into C(t) (in the first pass and in a replay alike)
+__device__ __forceinline__ bool sample_finite(float v) { return !isnan(v) && !isinf(v); }
+__device__ __forceinline__ bool sample_finite(double v) { return fabs(v) <= 1e100; }
+__device__ __forceinline__ float load_mu0v(const float *m, const float *d) {
+  const float4 v = *reinterpret_cast<const float4 *>(m);
+  return v.x * d[0] + v.y * d[1] + v.z * d[2];
+}
+__device__ __forceinline__ double load_mu0v(const double *m, const double *d) {
+  const double2 a = reinterpret_cast<const double2 *>(m)[0];
+  return a.x * d[0] + a.y * d[1] + m[2] * d[2];
+}
+
 // the context in 16-byte loads: qold, (t0, inv_h), (item, k0, n, prev), F
 template <int NQ>
 __device__ __forceinline__ void load_ctx(const SampleCtx<float, NQ> *cp, double (&qo)[NQ], double2 &th, int4 &hd,
@@ -260,6 +527,25 @@ __device__ __forceinline__ void load_ctx(const SampleCtx<float, NQ> *cp, double 
   }
 #pragma unroll
   for (int i = 4 * (7 * NQ / 4); i < 7 * NQ; ++i) F[i] = (&cp->F[0][0])[i];
+}
+
+template <int NQ>
+__device__ __forceinline__ void load_ctx(const SampleCtx<double, NQ> *cp, double (&qo)[NQ], double2 &th, int4 &hd,
+                                         double (&F)[7 * NQ]) {
+#pragma unroll
+  for (int i = 0; i < NQ / 2; ++i) {
+    const double2 v2 = reinterpret_cast<const double2 *>(cp->qold)[i];
+    qo[2 * i] = v2.x;
+    qo[2 * i + 1] = v2.y;
+  }
+  th = *reinterpret_cast<const double2 *>(&cp->t0);
+  hd = *reinterpret_cast<const int4 *>(&cp->item);
+#pragma unroll
+  for (int i = 0; i < 7 * NQ / 2; ++i) {
+    const double2 v2 = reinterpret_cast<const double2 *>(&cp->F[0][0])[i];
+    F[2 * i] = v2.x;
+    F[2 * i + 1] = v2.y;
+  }
 }
 
 // The warp's 32 contexts (base + lane) and the exclusive prefix sum of `units`
@@ -286,15 +572,16 @@ __device__ __forceinline__ int warp_owner(int off, int j) {
   return o;
 }
 
-// N2-Ar: one sample per lane, the position in FP64 as the trajectory kernel forms it.
+// One sample per lane, the position in FP64 as the trajectory kernel forms it: N2-Ar on
+// both paths and CO2-Ar on the FP64 path.
 template <int SYS, typename PHYS, typename STG>
-__global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs a, TrajParams P, TrajIO io,
-                                                                      const Co2arTablesGlobal *gtab) {
+__global__ void __launch_bounds__(defer_eval_threads<SYS, PHYS>(), defer_eval_min_blocks<SYS, PHYS>())
+    defer_eval_kernel(DeferArgs a, TrajParams P, TrajIO io, const Co2arTablesGlobal *gtab) {
   using DS = DeferSys<SYS, PHYS, STG>;
   constexpr int NQ = DS::NQ;
   using Ctx = SampleCtx<STG, NQ>;
-  static_assert(SYS == SYS_N2AR, "CO2-Ar samples go through defer_eval_co2ar_kernel");
-  static_assert(sizeof(STG) == 4 && sizeof(PHYS) == 4 && NQ % 2 == 0 && sizeof(Ctx) % 16 == 0, "vector loads of the context");
+  static_assert(SYS == SYS_N2AR || sizeof(PHYS) == 8, "mixed CO2-Ar samples go through defer_eval_co2ar_kernel");
+  static_assert(sizeof(STG) == sizeof(PHYS) && NQ % 2 == 0 && sizeof(Ctx) % 16 == 0, "vector loads of the context");
   constexpr unsigned FULL = 0xffffffffu;
   extern __shared__ __align__(16) unsigned char df_smem[];
   DS ds;
@@ -322,6 +609,7 @@ __global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs 
       PHYS v = PHYS(0);
       bool nan = false;
       int kk = 0, item = 0, nn = 0;
+      double q[NQ] = {0.0, 0.0, 20.0, 0.0, 0.0, 1.0};
       if (valid) {
         double qo[NQ];
         double2 th;
@@ -333,9 +621,7 @@ __global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs 
         kk = hd.y + jj;
         const double x = (double(kk) * P.dt - th.x) * th.y;
         const STG xs = STG(x), x1 = STG(1) - STG(x);
-        PHYS d[3];
         // the trajectory kernel's interpolation (hh_traj.cuh) in its order
-        double q[NQ];
 #pragma unroll
         for (int cq = 0; cq < NQ; ++cq) {
           STG w = F[6 * NQ + cq] * xs;
@@ -347,10 +633,12 @@ __global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs 
           w = (w + F[0 * NQ + cq]) * xs;
           q[cq] = qo[cq] + double(w);
         }
-        ds.dipole(q, d);
+      }
+      PHYS d[3];
+      if (DS::WARP || valid) ds.dipole(q, d);
+      if (valid) {
         nan = isnan(d[0]) || isnan(d[1]) || isnan(d[2]);
-        const float4 m = *reinterpret_cast<const float4 *>(mu0s + (size_t)item * 4);
-        v = m.x * d[0] + m.y * d[1] + m.z * d[2];
+        v = load_mu0v(mu0s + (size_t)item * 4, d);
       }
       // the previous sample of the same context: lane - 1, or the last of the
       // previous round (jj == 0 is the cross-context case of defer_jump_kernel)
@@ -361,7 +649,7 @@ __global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs 
         const unsigned code =
             sample_code(v, nan, kk, item + 2 * a.traj_base == P.inject_item && kk == P.inject_k, jj > 0 && kk > 1, pv);
         if (code != 0xffffffffu) atomicMin(&a.item_fail[item], code);
-        if (!isnan(v) && !isinf(v)) atomicAdd(&crln_slice(a, P, item)[kk], P.weight * double(v));
+        if (sample_finite(v)) atomicAdd(&crln_slice(a, P, item)[kk], P.weight * double(v));
         if (jj == 0) first_v[base + o] = v;
         if (jj == nn - 1) last_v[base + o] = v;
       }
@@ -378,7 +666,7 @@ __global__ void __launch_bounds__(DEFER_THREADS, 1) defer_eval_kernel(DeferArgs 
 // pair is computed but neither tested nor accumulated.  20 warps per SM (96 registers a
 // thread, no spills) ran faster than 16 (128) and than 24 or 32 (80 or 64, with spills).
 template <typename PHYS, typename STG>
-__global__ void __launch_bounds__(defer_eval_threads<SYS_CO2AR>(), 20 * 32 / defer_eval_threads<SYS_CO2AR>())
+__global__ void __launch_bounds__(defer_eval_threads<SYS_CO2AR, float>(), 20 * 32 / defer_eval_threads<SYS_CO2AR, float>())
     defer_eval_co2ar_kernel(DeferArgs a, TrajParams P, TrajIO io, const Co2arTablesGlobal *gtab) {
   using DS = DeferSys<SYS_CO2AR, float, float>;
   constexpr int NQ = DS::NQ;
