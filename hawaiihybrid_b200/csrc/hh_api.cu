@@ -80,7 +80,8 @@ template <typename T> struct DevBuf {
 
 struct TrajTune {
   int warps;        // bulk kernel warps per block
-  int handoff_div;  // hand-off when at most (solo warp slots) / handoff_div items are open
+  int handoff_div;  // hand-off when at most (solo warp slots) * handoff_mul / handoff_div items are open
+  int handoff_mul;  // (more than the slots: the solo kernel's warps take the stored items in turn)
 };
 
 struct Ctx {
@@ -413,11 +414,11 @@ int g_defer_overlap = [] {
 }();
 
 // One trajectory launch: the bulk kernel (WARPS warps per block) until at most
-// cap / handoff_div items are open, then the solo kernel for the rest, where cap is
+// cap * handoff_mul / handoff_div items are open, then the solo kernel for the rest, where cap is
 // the solo kernel's warp slots.  With ev_split, events ev[4] (start), ev[5] (after the
 // bulk kernel) and ev[7] (end) are recorded for the autotuner.
 template <int SYS, typename PHYS, typename STG, bool COMP, int WARPS, bool REQ = false>
-int launch_traj_w(const TrajParams &P, const TrajIO &io, int handoff_div, bool ev_split) {
+int launch_traj_w(const TrajParams &P, const TrajIO &io, int handoff_div, int handoff_mul, bool ev_split) {
   auto kern = traj_kernel<SYS, PHYS, STG, COMP, false, WARPS, REQ>;
   const size_t smem = traj_smem_bytes<SYS, PHYS, STG, WARPS>();
   if (smem > 48 * 1024) CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -439,7 +440,8 @@ int launch_traj_w(const TrajParams &P, const TrajIO &io, int handoff_div, bool e
   const int solo_grid = std::max(1, per_sm_solo) * g.num_sms;
   const unsigned cap = (unsigned)solo_grid * (SOLO_THREADS / 32);
   constexpr int NS = SYS == SYS_HEAR ? 6 : SYS == SYS_CH4CO2 ? 19 : 12;
-  CK(g.handoff.ensure((size_t)cap * sizeof(HandoffState<NS, PHYS, STG>)));
+  const unsigned mul = (unsigned)std::max(1, handoff_mul);
+  CK(g.handoff.ensure((size_t)cap * mul * sizeof(HandoffState<NS, PHYS, STG>)));
   CK(g.hcount.ensure(4));
   CK(cudaMemsetAsync(g.hcount.p, 0, 4 * sizeof(unsigned int), g.st));
   TrajIO io2 = io;
@@ -447,10 +449,10 @@ int launch_traj_w(const TrajParams &P, const TrajIO &io, int handoff_div, bool e
   io2.n_handoff = g.hcount.p;
   io2.solo_cursor = g.hcount.p + 1;
   io2.done = g.hcount.p + 2;
-  io2.handoff_at = std::max(1u, cap / (unsigned)std::max(1, handoff_div));
+  io2.handoff_at = std::max(1u, cap * mul / (unsigned)std::max(1, handoff_div));
   if (ev_split) CK(cudaEventRecord(g.ev[4], g.st));
   g.bulk_snap = false;
-  if ((unsigned)io.n_items > cap) {
+  if ((unsigned)io.n_items > cap * mul) {
     kt_begin();
     kern<<<grid, THREADS, smem, g.st>>>(P, io2, g.d_tab);
     CK(cudaGetLastError());
@@ -477,10 +479,10 @@ int launch_traj_w(const TrajParams &P, const TrajIO &io, int handoff_div, bool e
 }
 
 template <int SYS, typename PHYS, typename STG, bool COMP>
-int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int handoff_div, bool ev_split) {
+int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int div, int mul, bool ev_split) {
   if (warps == TRAJ_WARPS_CANDIDATES[0])
-    return launch_traj_w<SYS, PHYS, STG, COMP, TRAJ_WARPS_CANDIDATES[0]>(P, io, handoff_div, ev_split);
-  return launch_traj_w<SYS, PHYS, STG, COMP, TRAJ_WARPS_CANDIDATES[1]>(P, io, handoff_div, ev_split);
+    return launch_traj_w<SYS, PHYS, STG, COMP, TRAJ_WARPS_CANDIDATES[0]>(P, io, div, mul, ev_split);
+  return launch_traj_w<SYS, PHYS, STG, COMP, TRAJ_WARPS_CANDIDATES[1]>(P, io, div, mul, ev_split);
 }
 
 // Autotuner of the trajectory launch (first large plain-C(t) call per system and
@@ -489,7 +491,12 @@ int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int hando
 // trajectories per warp to one).  Timed on the launch's first items, into scratch
 // C(t) and counters, so the call's own results are untouched:
 //   1. each warps-per-block candidate with the full hand-off threshold: bulk kernel time;
-//   2. with the faster shape, thresholds cap / 2 and cap / 4 against cap: launch time.
+//   2. with the faster shape, the launch time at thresholds of 2 cap and, if that is
+//      faster than cap, 4 cap; otherwise cap / 2 and, if faster, cap / 4.  More than cap:
+//      the solo kernel's warps take several stored items in turn, which pays where few of
+//      the bulk kernel's lanes are left busy long before the end (N2-Ar FP64, 20,011
+//      trajectories: 10 % of the lanes from a fifth of the launch on; bulk launch 82 ms
+//      with a threshold of cap, 49 with 4 cap, the call 142 and 117).
 // HH_TRAJ_WARPS (4 or 8) and HH_TRAJ_HANDOFF_DIV (1, 2 or 4) fix a choice instead.
 constexpr int TRAJ_TUNE_MIN_ITEMS = 16384;  // smaller launches use the defaults, untuned
 constexpr int TRAJ_TUNE_ITEMS = 32768;      // items the timing runs integrate
@@ -519,11 +526,11 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
   t.item_trace = nullptr;
   TrajParams Pt = P;
   Pt.inject_item = -1;
-  auto run = [&](int w, int d, float *bulk_ms, float *all_ms) -> int {
+  auto run = [&](int w, int d, int mul, float *bulk_ms, float *all_ms) -> int {
     CK(cudaMemsetAsync(g.tune_cnt.p, 0, (16 + 2 * HH_ST_COUNT + 1) * sizeof(double), g.st));
     if (t.ctx_count) CK(cudaMemsetAsync(t.ctx_count, 0, sizeof(unsigned long long), g.st));
     CK(cudaMemsetAsync(g.tune_crln.p, 0, (size_t)P.N * nsl * sizeof(double), g.st));
-    int rc = launch_traj_pick<SYS, PHYS, STG, COMP>(Pt, t, w, d, true);
+    int rc = launch_traj_pick<SYS, PHYS, STG, COMP>(Pt, t, w, d, mul, true);
     if (rc) return rc;
     CK(cudaEventSynchronize(g.ev[7]));
     CK(cudaEventElapsedTime(bulk_ms, g.ev[4], g.ev[5]));
@@ -536,7 +543,7 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
     float best = 0.f;
     for (int c = 0; c < 2; ++c) {
       const int w = TRAJ_WARPS_CANDIDATES[c];
-      int rc = run(w, 1, &bulk, &all);
+      int rc = run(w, 1, 1, &bulk, &all);
       if (rc) return rc;
       if (c == 0 || bulk < best) {
         best = bulk;
@@ -544,22 +551,32 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
       }
     }
   }
-  int d_best = fixed_d ? fixed_d : 1;
+  int d_best = fixed_d ? fixed_d : 1, m_best = 1;
   if (!fixed_d) {
-    float best = 0.f;
-    for (int d : {1, 2, 4}) {
-      int rc = run(w_best, d, &bulk, &all);
+    int rc = run(w_best, 1, 1, &bulk, &all);
+    if (rc) return rc;
+    float best = all;
+    for (int m : {2, 4}) {
+      rc = run(w_best, 1, m, &bulk, &all);
       if (rc) return rc;
-      if (d == 1 || all < best) {
-        best = all;
-        d_best = d;
-      }
+      if (!(all < best)) break;
+      best = all;
+      m_best = m;
+    }
+    for (int d : {2, 4}) {
+      if (m_best > 1) break;
+      rc = run(w_best, d, 1, &bulk, &all);
+      if (rc) return rc;
+      if (!(all < best)) break;
+      best = all;
+      d_best = d;
     }
   }
   // the timing runs' sample contexts are scratch
   if (t.ctx_count) CK(cudaMemsetAsync(t.ctx_count, 0, sizeof(unsigned long long), g.st));
   out->warps = w_best;
   out->handoff_div = d_best;
+  out->handoff_mul = m_best;
   return HH_OK;
 }
 
@@ -574,7 +591,8 @@ int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
   }
   const int w = tt.warps ? tt.warps : traj_warps<PHYS>();
   const int d = tt.handoff_div ? tt.handoff_div : 1;
-  return launch_traj_pick<SYS, PHYS, STG, COMP>(P, io, w, d, false);
+  const int m = tt.handoff_mul ? tt.handoff_mul : 1;
+  return launch_traj_pick<SYS, PHYS, STG, COMP>(P, io, w, d, m, false);
 }
 
 // PR_MU with requantization: the REQ kernels of the linear-monomer systems
@@ -585,12 +603,12 @@ int run_traj_dispatch_req(int precision, const TrajParams &P, const TrajIO &io) 
     io2.dipnet = g.d_n2ar_fold;
     io2.pesnet = mixed ? (const void *)g.d_n2ar_pes_f : (const void *)g.d_n2ar_pes_d;
     io2.diptab = mixed ? g.d_n2ar_tab : nullptr;
-    return mixed ? launch_traj_w<SYS_N2AR, float, float, false, traj_warps<float>(), true>(P, io2, 1, false)
-                 : launch_traj_w<SYS_N2AR, double, double, false, traj_warps<double>(), true>(P, io2, 1, false);
+    return mixed ? launch_traj_w<SYS_N2AR, float, float, false, traj_warps<float>(), true>(P, io2, 1, 1, false)
+                 : launch_traj_w<SYS_N2AR, double, double, false, traj_warps<double>(), true>(P, io2, 1, 1, false);
   }
   if (g.sys == SYS_CO2AR)
-    return mixed ? launch_traj_w<SYS_CO2AR, float, float, false, traj_warps<float>(), true>(P, io, 1, false)
-                 : launch_traj_w<SYS_CO2AR, double, double, false, traj_warps<double>(), true>(P, io, 1, false);
+    return mixed ? launch_traj_w<SYS_CO2AR, float, float, false, traj_warps<float>(), true>(P, io, 1, 1, false)
+                 : launch_traj_w<SYS_CO2AR, double, double, false, traj_warps<double>(), true>(P, io, 1, 1, false);
   return HH_E_UNSUPPORTED_SYSTEM;
 }
 
@@ -2383,7 +2401,7 @@ int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div,
   if (precision != HH_PRECISION_FP64 && precision != HH_PRECISION_MIXED) return HH_E_INVALID_ARGUMENT;
   TrajTune &tt = g.traj_tune[g.sys][precision == HH_PRECISION_MIXED ? 1 : 0];
   if (set_warps < 0 || set_handoff_div < 0) {
-    tt.warps = tt.handoff_div = 0;
+    tt.warps = tt.handoff_div = tt.handoff_mul = 0;
   } else if (set_warps > 0 || set_handoff_div > 0) {
     if (set_warps > 0 && set_warps != TRAJ_WARPS_CANDIDATES[0] && set_warps != TRAJ_WARPS_CANDIDATES[1])
       return HH_E_INVALID_ARGUMENT;
@@ -2392,6 +2410,7 @@ int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div,
     const int dw = precision == HH_PRECISION_MIXED ? traj_warps<float>() : traj_warps<double>();
     tt.warps = set_warps > 0 ? set_warps : (tt.warps ? tt.warps : dw);
     tt.handoff_div = set_handoff_div > 0 ? set_handoff_div : (tt.handoff_div ? tt.handoff_div : 1);
+    if (set_handoff_div > 0) tt.handoff_mul = 1;
   }
   if (warps) *warps = tt.warps;
   if (handoff_div) *handoff_div = tt.handoff_div;

@@ -274,39 +274,193 @@ __device__ __noinline__ N2arGrad<T> n2ar_pes_grad(const N2arPesNet<T> *net, T d1
   return {n2_mul(n2_mul(a1, dy1), s), n2_mul(n2_mul(a2, dy2), s)};
 }
 
-// n2ar_pes_grad with the 32 lanes of a warp on one (d1, d2), bit for bit: every
-// lane forms the network inputs, lane j evaluates hidden unit j (the same sum over
-// the 17 inputs, in the same order), lane i < 17 forms a_i = sum_j W0[i][j] g_j
-// over the units in the order of the per-lane loop from values shuffled out of the
-// other lanes, and every lane sums j1_i a_i / xscale_i and j2_i a_i / xscale_i over
-// i in order from the a_i shuffled out of lanes 0..16.  A trajectory therefore
-// takes the same steps in the solo kernel as in the bulk kernel.  All 32 lanes
-// call it with the same arguments.
-template <typename T>
-__device__ __noinline__ N2arGrad<T> n2ar_pes_grad_coop(const N2arPesNet<T> *net, T d1, T d2) {
-  static_assert(N2AR_PES_NH == 32 && N2AR_PES_NP <= 32, "one hidden unit per lane");
-  constexpr unsigned FULL = 0xffffffffu;
-  constexpr int NP = N2AR_PES_NP;
-  T ptr[NP], j1[NP], j2[NP], dy1, dy2;
-  n2ar_grad_inputs(net, d1, d2, ptr, j1, j2, dy1, dy2);
+// the variables of the monomials of PIP i, two bits each (monomial 0 in bits 0..7, 1 in
+// bits 8..15): 0, 1, 2 = y_k, 3 = absent; a PIP with one monomial has bit 16 clear
+struct N2arPipCodes {
+  unsigned c[32];
+};
+constexpr N2arPipCodes n2ar_pip_codes() {
+  N2arPipCodes t{};
+  int n[32] = {};
+  for (int i = 0; i < 32; ++i) t.c[i] = 0xffffu;
+  for (int m = 0; m < HH_N2AR_PES_NMONO; ++m) {
+    const int i = hh_n2ar_pes_poly[m], q = n[i]++;
+    unsigned v = 0;
+    for (int k = 0; k < 4; ++k) v |= (hh_n2ar_pes_var[m][k] < 0 ? 3u : unsigned(hh_n2ar_pes_var[m][k])) << (2 * k);
+    t.c[i] = (t.c[i] & ~(0xffu << (8 * q))) | (v << (8 * q));
+    if (q == 1) t.c[i] |= 1u << 16;
+    if (q > 1) t.c[i] = 0;  // more monomials than the code holds (checked below)
+  }
+  return t;
+}
+__constant__ N2arPipCodes c_n2ar_pip = n2ar_pip_codes();
+static_assert([] {
+  for (int i = 0; i < N2AR_PES_NP; ++i)
+    if (n2ar_pip_codes().c[i] == 0) return false;
+  return true;
+}(), "at most two monomials per PIP");
+
+// the code of this lane's PIP
+__device__ __forceinline__ unsigned n2ar_pip_code() {
   const int lane = threadIdx.x & 31;
-  const T *wt = net->w0t[lane];
-  T h = net->b0[lane];
+  return c_n2ar_pip.c[lane < N2AR_PES_NP ? lane : N2AR_PES_NP - 1];
+}
+
+// n values (16-byte aligned) by 16-byte loads
+template <int N> __device__ __forceinline__ void n2_load_row(float *d, const float *s) {
 #pragma unroll
-  for (int i = 0; i < NP; ++i) h = n2_fma(ptr[i], wt[i], h);
-  const T g = n2ar_unit_grad(h, net->w1[lane]);
+  for (int i = 0; i < N / 4; ++i) {
+    const float4 v = reinterpret_cast<const float4 *>(s)[i];
+    d[4 * i] = v.x;
+    d[4 * i + 1] = v.y;
+    d[4 * i + 2] = v.z;
+    d[4 * i + 3] = v.w;
+  }
+}
+template <int N> __device__ __forceinline__ void n2_load_row(double *d, const double *s) {
+#pragma unroll
+  for (int i = 0; i < N / 2; ++i) {
+    const double2 v = reinterpret_cast<const double2 *>(s)[i];
+    d[2 * i] = v.x;
+    d[2 * i + 1] = v.y;
+  }
+}
+
+// Shared memory of the cooperative gradient: the first-layer weights with one hidden unit
+// per lane (wf, once per block) and a warp's exchange buffer.
+template <typename T> struct N2arCoopWeights {
+  T wf[N2AR_PES_NP][32];  // wf[i][j] = W0[i][j]
+};
+template <typename T> struct alignas(16) N2arCoopScratch {
+  T y[4];                 // y0, y1, y2, 1 (the first and last set once, n2ar_coop_init)
+  T dy[2], pad[2];
+  T ptr[N2AR_PES_ROW];    // (rows start on 16 bytes)
+  T g[32];
+  T out[N2AR_PES_NP][4];  // a_i / xscale_i, dp_i/dy_1, dp_i/dy_2
+};
+
+template <typename T>
+__device__ __forceinline__ void n2ar_coop_init(N2arCoopWeights<T> *cw, N2arCoopScratch<T> *sc,
+                                               const N2arPesNet<T> *net) {
+  for (int i = threadIdx.x; i < N2AR_PES_NP * 32; i += blockDim.x) cw->wf[i / 32][i % 32] = net->w0t[i % 32][i / 32];
+  if ((threadIdx.x & 31) == 0) {
+    sc->y[0] = exp(-T(N2AR_L) / T(2));
+    sc->y[3] = T(1);
+  }
+  __syncthreads();
+}
+
+// n2ar_pes_grad with the 32 lanes of a warp on one (d1, d2), bit for bit: the pair
+// functions of d1 on even lanes and d2 on odd ones, PIP i with its Jacobian on lane i
+// (absent variables are exact factors of 1), hidden unit j on lane j (the same sum over
+// the 17 inputs, in the same order), a_i = sum_j W0[i][j] g_j on lane i over the units in
+// the order of the per-lane loop, and the sums of j1_i a_i / xscale_i and j2_i a_i /
+// xscale_i over i in order on every lane.  The values pass through shared memory.  A
+// trajectory therefore takes the same steps in the solo kernel as in the bulk kernel.  All
+// 32 lanes call it with the same arguments but code (n2ar_pip_code).  Latency bounds it (one right-hand side: 3,700 cycles in FP64): with every
+// lane forming all the inputs and values passed by shuffles the solo launch took, in FP64
+// (20,011 x 5,000), 60.7 ms, so 42 to 47; on the mixed path (131,072 x 16,384) 41.5 and 39.7.
+template <typename T>
+__device__ __noinline__ N2arGrad<T> n2ar_pes_grad_coop(const N2arPesNet<T> *net, const N2arCoopWeights<T> *cw,
+                                                       N2arCoopScratch<T> *sc, unsigned code, T d1, T d2) {
+  static_assert(N2AR_PES_NH == 32 && N2AR_PES_NP <= 32, "one hidden unit per lane");
+  constexpr int NP = N2AR_PES_NP;
+  const int lane = threadIdx.x & 31;
   const int ir = lane < NP ? lane : NP - 1;
-  T a = T(0);
+  {
+    T y, dy;
+    n2ar_pair_y_rn((lane & 1) ? d2 : d1, y, dy);
+    if (lane < 2) {
+      sc->y[1 + lane] = y;
+      sc->dy[lane] = dy;
+    }
+  }
+  __syncwarp();
+  T p, j1, j2;
+  {
+    // both monomials side by side; the second one's terms are dropped where it is absent
+    T pr[2], s1[2][4], s2[2][4];
+    unsigned v[2][4];
+    T x[2][4];
 #pragma unroll
-  for (int j = 0; j < N2AR_PES_NH; ++j) a = n2_fma(net->w0t[j][ir], __shfl_sync(FULL, g, j), a);
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        v[m][k] = (code >> (8 * m + 2 * k)) & 3u;
+        x[m][k] = sc->y[v[m][k]];
+      }
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      const T x01 = n2_mul(x[m][0], x[m][1]), x012 = n2_mul(x01, x[m][2]);
+      pr[m] = n2_mul(x012, x[m][3]);
+      const T d[4] = {n2_mul(n2_mul(x[m][1], x[m][2]), x[m][3]), n2_mul(n2_mul(x[m][0], x[m][2]), x[m][3]),
+                      n2_mul(x01, x[m][3]), x012};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        s1[m][k] = v[m][k] == 1u ? d[k] : T(0);
+        s2[m][k] = v[m][k] == 2u ? d[k] : T(0);
+      }
+    }
+    // (all terms are positive, so adding a zero is exact)
+    p = pr[0];
+    j1 = n2_add(n2_add(n2_add(s1[0][0], s1[0][1]), s1[0][2]), s1[0][3]);
+    j2 = n2_add(n2_add(n2_add(s2[0][0], s2[0][1]), s2[0][2]), s2[0][3]);
+    const T q = n2_add(p, pr[1]);
+    T q1 = j1, q2 = j2;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      q1 = n2_add(q1, s1[1][k]);
+      q2 = n2_add(q2, s2[1][k]);
+    }
+    if (code >> 16) {
+      p = q;
+      j1 = q1;
+      j2 = q2;
+    }
+  }
+  if (lane < NP) sc->ptr[lane] = n2_mul(n2_sub(p, net->xmean[ir]), net->ixscale[ir]);
+  __syncwarp();
+  T h = net->b0[lane];
+  {
+    T w[NP], q[N2AR_PES_ROW];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) w[i] = cw->wf[i][lane];
+    n2_load_row<N2AR_PES_ROW>(q, sc->ptr);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) h = n2_fma(q[i], w[i], h);
+  }
+  sc->g[lane] = n2ar_unit_grad(h, net->w1[lane]);
+  __syncwarp();
+  T a = T(0);
+  {
+    // loads ahead of the chain (one at a time they cost 31 cycles per unit)
+    T g[32], w[16];
+    n2_load_row<32>(g, sc->g);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) w[j] = net->w0t[16 * b + j][ir];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) a = n2_fma(w[j], g[16 * b + j], a);
+    }
+  }
+  if (lane < NP) {
+    sc->out[lane][0] = n2_mul(a, net->ixscale[ir]);
+    sc->out[lane][1] = j1;
+    sc->out[lane][2] = j2;
+  }
+  __syncwarp();
   T a1 = T(0), a2 = T(0);
 #pragma unroll
   for (int i = 0; i < NP; ++i) {
-    const T ai = n2_mul(__shfl_sync(FULL, a, i), net->ixscale[i]);
-    a1 = n2_fma(j1[i], ai, a1);
-    a2 = n2_fma(j2[i], ai, a2);
+    T o[4];
+    n2_load_row<4>(o, sc->out[i]);
+    a1 = n2_fma(o[1], o[0], a1);
+    a2 = n2_fma(o[2], o[0], a2);
   }
   const T s = n2_mul(net->yscale, T(1.0 / HH_HTOCM));
+  const T dy1 = sc->dy[0], dy2 = sc->dy[1];
+  __syncwarp();  // the next evaluation writes the buffer again
   return {n2_mul(n2_mul(a1, dy1), s), n2_mul(n2_mul(a2, dy2), s)};
 }
 

@@ -565,6 +565,16 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct Co2
 // maps body z to r^ and body x to the in-plane normal to r^ on the N1 side.
 // SOLO_: the solo kernel's instance (one trajectory per warp), whose right-hand side
 // the 32 lanes evaluate cooperatively (n2ar_pes_grad_coop)
+template <typename PHYS, typename STG, bool COMP> struct N2ArSoloArgs {
+  const N2arPesNet<PHYS> *pes;
+  const N2arCoopWeights<PHYS> *coop;
+  N2arCoopScratch<PHYS> *scr;
+  unsigned pip;
+  double inv_mu, inv_II;
+};
+template <typename PHYS, typename STG, bool COMP>
+__device__ STG n2ar_rhs_out_of_line(N2ArSoloArgs<PHYS, STG, COMP> a, STG ysc, int c);
+
 template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2ArSys {
   static constexpr bool SOLO = SOLO_;
   static constexpr int N = 12;
@@ -578,6 +588,9 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
   const N2arDipFold *fold;      // shared-memory copies
   const N2arPesNet<PHYS> *pes;
   const float4 *dtab;           // mixed path: the dipole table (hh_n2ar.cuh), global memory
+  const N2arCoopWeights<PHYS> *coop;  // solo kernel: shared memory of n2ar_pes_grad_coop
+  N2arCoopScratch<PHYS> *scr;         // (this warp's)
+  unsigned pip;                       // (this lane's PIP)
   template <typename YT> __device__ void rhs(const YT *y, STG *f) const {
     const PHYS r[3] = {PHYS(y[0]), PHYS(y[1]), PHYS(y[2])};
     const PHYS u[3] = {PHYS(y[6]), PHYS(y[7]), PHYS(y[8])};
@@ -594,7 +607,7 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     const PHYS i2 = inv_sqrt(e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
     N2arGrad<PHYS> g;
     if constexpr (SOLO)
-      g = n2ar_pes_grad_coop<PHYS>(pes, PHYS(1) / i1, PHYS(1) / i2);
+      g = n2ar_pes_grad_coop<PHYS>(pes, coop, scr, pip, PHYS(1) / i1, PHYS(1) / i2);
     else
       g = n2ar_pes_grad<PHYS>(pes, PHYS(1) / i1, PHYS(1) / i2);
     const PHYS a1 = g.g1 * i1, a2 = g.g2 * i2;
@@ -621,14 +634,9 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     f[10] = STG(-(uh[2] * Gu[0] - uh[0] * Gu[2]));
     f[11] = STG(-(uh[0] * Gu[1] - uh[1] * Gu[0]));
   }
-  // component c of f (solo kernel): the full stage point gathered from the lanes, the
-  // right-hand side on every lane
+  // component c of f (solo kernel), the values those of rhs
   __device__ __forceinline__ STG rhs_c(STG ysc, int c) const {
-    STG ys[N], f[N];
-#pragma unroll
-    for (int i = 0; i < N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
-    rhs(ys, f);
-    return pick_component<N>(f, c);
+    return n2ar_rhs_out_of_line<PHYS, STG, COMP>({pes, coop, scr, pip, inv_mu, inv_II}, ysc, c);
   }
   // q = (r[3], u[3]); the body-frame dipole is the FP64 network on the FP64 path and
   // the FP32 table of hh_n2ar.cuh (the network outside its R range) on the mixed path
@@ -651,6 +659,26 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     for (int c = 0; c < 3; ++c) d[c] = PHYS(b.dz * rh[c] + b.dx * e[c] * ie);
   }
 };
+
+// Component c of the N2-Ar right-hand side for the solo kernel: the full stage point
+// gathered from the lanes, N2ArSys::rhs around the shared gradient on every lane; out of
+// line, one copy for all stages.
+template <typename PHYS, typename STG, bool COMP>
+__device__ __noinline__ STG n2ar_rhs_out_of_line(N2ArSoloArgs<PHYS, STG, COMP> a, STG ysc, int c) {
+  using Sys = N2ArSys<PHYS, STG, COMP, true>;
+  Sys sys;
+  sys.inv_mu = a.inv_mu;
+  sys.inv_II = a.inv_II;
+  sys.pes = a.pes;
+  sys.coop = a.coop;
+  sys.scr = a.scr;
+  sys.pip = a.pip;
+  STG ys[Sys::N], f[Sys::N];
+#pragma unroll
+  for (int i = 0; i < Sys::N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
+  sys.rhs(ys, f);
+  return pick_component<Sys::N>(f, c);
+}
 
 // find_closest_integer / find_closest_half_integer (src/hawaii.c:360-393): the
 // requantized |j| of the linear monomer.  The half-integer rule returns 0 below 0.25,
@@ -1993,6 +2021,14 @@ __global__ void __launch_bounds__(32 * WARPS, TRAJ_MIN_BLOCKS)
     sys.fold = fold;
     sys.pes = pes;
     sys.dtab = static_cast<const float4 *>(io.diptab);
+    if constexpr (SOLO) {
+      __shared__ N2arCoopWeights<PHYS> coop_w;
+      __shared__ N2arCoopScratch<PHYS> coop_s[WARPS];
+      sys.coop = &coop_w;
+      sys.scr = &coop_s[threadIdx.x >> 5];
+      sys.pip = n2ar_pip_code();
+      n2ar_coop_init(&coop_w, sys.scr, pes);
+    }
     auto *ws = reinterpret_cast<WarpSamples<STG, PHYS, Sys::NQ> *>(smem_raw + sizeof(N2arDipFold) +
                                                                    sizeof(N2arPesNet<PHYS>));
     traj_body<Sys, PHYS, STG, REQ>(sys, P, io, ws);

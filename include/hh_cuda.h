@@ -366,7 +366,8 @@ int hh_cuda_debug_kernel_ms(int enable, double *ms, uint64_t *launches, int n);
 /* Tuning knob (no counterpart in the reference): the trajectory launch's block
  * shape (bulk kernel warps per block, 4 or 8) and hand-off threshold (the launch
  * switches from 32 trajectories per warp to one when at most (solo warp slots) /
- * handoff_div items are open; 1, 2 or 4) for the bound system and `precision`.  The
+ * handoff_div items are open; 1, 2 or 4; with 1 the tuner may also pick two or four
+ * times the slots) for the bound system and `precision`.  The
  * library times the candidates on the first plain-C(t) launch of at least 16,384
  * half-trajectories per system and precision (environment HH_TRAJ_WARPS,
  * HH_TRAJ_HANDOFF_DIV fix them instead).  set_* > 0 fixes a value, set_* < 0
