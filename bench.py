@@ -338,7 +338,8 @@ def bench_ch4co2(args, hh, H, peaks):
     out["dipole_records_per_lane"] = {"fp64": s64.value, "mixed": s32.value,
                                       "how": "timed per precision on the first call's records (the warm-up)"}
     nb, ng = _lib.ch4co2_fold_shape()
-    fl = flops.ch4_dipole_flops(4 * nb, ng)
+    coupled = s64.value == -2
+    stream_fl = flops.ch4_dipole_flops(4 * nb, ng)
     for name, st in (("mixed", sm), ("fp64", sp)):
         dms = kt[name]["ch4_dipole"]["ms"]
         if name == "mixed" and s32.value == -1 and dms > 0:
@@ -357,12 +358,17 @@ def bench_ch4co2(args, hh, H, peaks):
                         "(Blackwell dense TF32 is half its bf16 rate)"}
             continue
         if dms > 0:
+            in_coupled = coupled and name == "fp64"
+            fl = flops.CH4_COUPLED_FLOPS if in_coupled else stream_fl
             work = {"fp32": float(fl * st["n_samples"]) if name == "mixed" else 0.0,
                     "fp64": 0.0 if name == "mixed" else float(fl * st["n_samples"])}
             out.setdefault("roofline", {})[name] = _roof(
-                work, dms / 1e3, *peaks, f"ch4_dipole_kernel<{'float' if name == 'mixed' else 'double'}>",
-                note=f"{fl} flops per record ({4 * nb} padded coefficient entries, {ng} groups) x the call's "
-                     f"records; time from a per-kernel timed call")
+                work, dms / 1e3, *peaks,
+                "ch4_dipole_coupled_kernel" if in_coupled else
+                f"ch4_dipole_kernel<{'float' if name == 'mixed' else 'double'}>",
+                note=(f"{fl} flops per record (591 cubics, 156 groups)" if in_coupled else
+                      f"{fl} flops per record ({4 * nb} padded coefficient entries, {ng} groups)")
+                     + " x the call's records; time from a per-kernel timed call")
     if not args.no_accuracy:
         out["accuracy"] = [dict(T=w["Ts"][i], **_ct_errors(cm[i], cp[i])) for i in range(len(w["Ts"]))]
     return out

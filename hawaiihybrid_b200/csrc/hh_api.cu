@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/hh_cuda.h"
+#include "hh_ch4co2_coupled.cuh"
 #include "hh_ch4co2_dip.cuh"
 #include "hh_ch4co2_tc.cuh"
 #include "hh_ch4co2_fold.h"
@@ -119,6 +120,10 @@ struct Ctx {
   unsigned int *d_ch4_meta = nullptr;
   int ch4_B = 0;
   int ch4_groups = 0;  // (Y1, component, cos/sin) groups of the batch stream
+  // coupled form (FP64): cubics, group descriptors
+  double2 *d_ch4_cc = nullptr;
+  unsigned short *d_ch4_cd2 = nullptr;
+  Ch4CoupledArgs ch4_cpl{};  // its fixed arguments
   unsigned char *d_ch4_tc = nullptr;  // coefficient images of the tensor-core dipole kernel
   int *d_ch4_tc_err = nullptr;        // set by that kernel when an mbarrier wait gave up
   int ch4_dip_s[2] = {0, 0};  // records per lane of the dipole kernel [FP64, mixed]; 0: not tuned yet
@@ -822,15 +827,24 @@ int zimm_fft(const ZimmArgs &za) {
 
 // one launchable variant of the CH4-CO2 dipole kernel (S records per lane)
 // S: records per lane of ch4_dipole_kernel, or CH4_DIP_TC for the tensor-core kernel
-// (hh_ch4co2_tc.cuh: tasks of 128 records, one CTA per SM)
-constexpr int CH4_DIP_TC = -1;
+// (hh_ch4co2_tc.cuh: tasks of 128 records, one CTA per SM), or CH4_DIP_COUPLED for the
+// coupled-form kernel (hh_ch4co2_coupled.cuh: FP64, tasks of 32 records)
+constexpr int CH4_DIP_TC = -1, CH4_DIP_COUPLED = -2;
 struct Ch4DipVariant {
   void (*kern)(Ch4DipArgs);
   int S;
   size_t smem;
   int grid;
-  int task() const { return S == CH4_DIP_TC ? CH4TC_M : 32 * S; }
+  int task() const { return S == CH4_DIP_TC ? CH4TC_M : S == CH4_DIP_COUPLED ? 32 : 32 * S; }
 };
+int ch4_dip_coupled_variant(Ch4DipVariant *v) {
+  v->kern = nullptr;
+  v->S = CH4_DIP_COUPLED;
+  v->smem = ch4c_smem();
+  CK(cudaFuncSetAttribute(ch4_dipole_coupled_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)v->smem));
+  v->grid = g.num_sms;  // one block fills an SM's shared memory
+  return HH_OK;
+}
 
 int ch4_dip_tc_variant(Ch4DipVariant *v) {
   v->kern = nullptr;
@@ -853,8 +867,8 @@ template <typename PHYS, int S> int ch4_dip_variant(Ch4DipVariant *v) {
   return HH_OK;
 }
 
-// the dipole kernel's candidates per precision: S = 1, 2, 4 and the tensor-core
-// kernel (FP32), S = 1, 2 (FP64)
+// the dipole kernel's variants per precision: S = 1, 2, 4 and the tensor-core kernel
+// (FP32); S = 1, 2 and the coupled form (FP64)
 template <typename PHYS> int ch4_dip_candidates(Ch4DipVariant *v, int *n) {
   int rc = ch4_dip_variant<PHYS, 1>(&v[0]);
   if (!rc) rc = ch4_dip_variant<PHYS, 2>(&v[1]);
@@ -863,6 +877,9 @@ template <typename PHYS> int ch4_dip_candidates(Ch4DipVariant *v, int *n) {
     if (!rc) rc = ch4_dip_variant<PHYS, 4>(&v[2]);
     if (!rc) rc = ch4_dip_tc_variant(&v[3]);
     *n = 4;
+  } else {
+    if (!rc) rc = ch4_dip_coupled_variant(&v[2]);
+    *n = 3;
   }
   return rc;
 }
@@ -915,6 +932,9 @@ int run_records_t(const TrajParams &P, const double *d_ic, uint64_t n, uint64_t 
     const int want = env ? (strcmp(env, "tc") == 0 ? CH4_DIP_TC : atoi(env)) : 0;
     for (int c = 0; c < ncand; ++c)
       if (cand[c].S == want) tuned_s = want;
+    // FP64: the coupled form takes a tenth of the entry stream's arithmetic, so it is not
+    // timed against the others (4 x 25,013 trajectories: 2.98 ms against 70.3)
+    if (tuned_s == 0 && sizeof(PHYS) == 8) tuned_s = CH4_DIP_COUPLED;
   }
   for (uint64_t base = 0; base < n; base += chunk) {
     const uint64_t nc = std::min<uint64_t>(chunk, n - base);
@@ -989,6 +1009,15 @@ int run_records_t(const TrajParams &P, const double *d_ic, uint64_t n, uint64_t 
           ta.task_step = step;
           ta.err = g.d_ch4_tc_err;
           ch4_dipole_tc_kernel<<<v.grid, CH4TC_THREADS, v.smem, g.st>>>(ta);
+        }
+      } else if (v.S == CH4_DIP_COUPLED) {
+        if constexpr (sizeof(PHYS) == 8) {
+          Ch4CoupledArgs cpl = g.ch4_cpl;
+          cpl.records = g.rec.p;
+          cpl.sorted = g.rec_sorted.p;
+          cpl.warp0 = g.seg_w0.p;
+          cpl.mu = g.rec_mu.p;
+          ch4_dipole_coupled_kernel<<<v.grid, 32 * CH4C_WARPS, v.smem, g.st>>>(cpl);
         }
       } else {
         da.max_tasks = max_tasks;
@@ -1660,6 +1689,21 @@ int hh_cuda_init(int device, const hh_system_desc *sys) {
     CK(cudaMemcpy(g.d_ch4_cf, cf.data(), cf.size() * sizeof(float4), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.d_ch4_y2, f.by2.data(), 4 * B, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(g.d_ch4_meta, f.bmeta.data(), B * sizeof(unsigned int), cudaMemcpyHostToDevice));
+    {
+      Ch4Co2CoupledHost c;
+      if (ch4co2_build_coupled(&c) != 0) return HH_E_UNSUPPORTED_SYSTEM;
+      CK(cudaMalloc(&g.d_ch4_cc, c.coef.size() * sizeof(double)));
+      CK(cudaMalloc(&g.d_ch4_cd2, c.desc.size() * sizeof(unsigned short)));
+      CK(cudaMemcpy(g.d_ch4_cc, c.coef.data(), c.coef.size() * sizeof(double), cudaMemcpyHostToDevice));
+      CK(cudaMemcpy(g.d_ch4_cd2, c.desc.data(), c.desc.size() * sizeof(unsigned short), cudaMemcpyHostToDevice));
+      Ch4CoupledArgs &a = g.ch4_cpl;
+      a.coef = g.d_ch4_cc;
+      a.desc = g.d_ch4_cd2;
+      a.n_coef = c.n_coef;
+      a.n_group = c.n_group;
+      memcpy(a.count, c.count, sizeof a.count);
+      for (int i = 0; i < CH4_NSEG; ++i) a.centre[i] = hh_ch4co2_centre[i];
+    }
     std::vector<float> tc_blob;
     if (ch4co2_build_tc_blob(f, &tc_blob) != 0) return HH_E_UNSUPPORTED_SYSTEM;
     CK(cudaMalloc(&g.d_ch4_tc, tc_blob.size() * sizeof(float)));
@@ -2436,7 +2480,8 @@ int hh_cuda_debug_set_ch4_dipole(int precision, int variant) {
   if (!g.init) return HH_E_NOT_INITIALIZED;
   if (precision != HH_PRECISION_FP64 && precision != HH_PRECISION_MIXED) return HH_E_INVALID_ARGUMENT;
   const bool mixed = precision == HH_PRECISION_MIXED;
-  const bool ok = variant == 0 || variant == 1 || variant == 2 || (mixed && (variant == 4 || variant == CH4_DIP_TC));
+  const bool ok = variant == 0 || variant == 1 || variant == 2 ||
+                  (mixed ? variant == 4 || variant == CH4_DIP_TC : variant == CH4_DIP_COUPLED);
   if (!ok) return HH_E_INVALID_ARGUMENT;
   g.ch4_dip_s[mixed ? 1 : 0] = variant;
   return HH_OK;
@@ -2631,6 +2676,8 @@ void hh_cuda_shutdown(void) {
   if (g.d_ch4_cf) cudaFree(g.d_ch4_cf);
   if (g.d_ch4_y2) cudaFree(g.d_ch4_y2);
   if (g.d_ch4_meta) cudaFree(g.d_ch4_meta);
+  if (g.d_ch4_cc) cudaFree(g.d_ch4_cc);
+  if (g.d_ch4_cd2) cudaFree(g.d_ch4_cd2);
   if (g.d_ch4_tc) cudaFree(g.d_ch4_tc);
   if (g.d_ch4_tc_err) cudaFree(g.d_ch4_tc_err);
   if (g.d_mt) cudaFree(g.d_mt);

@@ -2,11 +2,13 @@
 // expanded reference tables of hh_ch4co2_tables.h, in FP64.
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <cstdint>
 #include <cstring>
 #include <map>
 #include <tuple>
 
+#include "hh_ch4co2_coupled.h"
 #include "hh_ch4co2_fold.h"
 #include "hh_ch4co2_tables.h"
 #include "hh_ch4co2_tc_layout.h"
@@ -173,5 +175,238 @@ int ch4co2_build_tc_blob(const Ch4Co2FoldHost &f, std::vector<float> *blob) {
         }
       }
     }
+  return 0;
+}
+
+// ---------------------------------------------------------------------------
+// coupled form (hh_ch4co2_coupled.h)
+// ---------------------------------------------------------------------------
+namespace {
+using cplx = std::complex<double>;
+
+// a tensor of l1 x l2 x vector over (m1, m2, q), spherical components
+struct Tensor {
+  int l1, l2;
+  std::vector<cplx> v;
+  Tensor(int a, int b) : l1(a), l2(b), v((size_t)(2 * a + 1) * (2 * b + 1) * 3, 0.0) {}
+  cplx &at(int m1, int m2, int q) { return v[((size_t)(m1 + l1) * (2 * l2 + 1) + (m2 + l2)) * 3 + (q + 1)]; }
+  cplx get(int m1, int m2, int q) const {
+    if (std::abs(m1) > l1 || std::abs(m2) > l2 || std::abs(q) > 1) return 0.0;
+    return v[((size_t)(m1 + l1) * (2 * l2 + 1) + (m2 + l2)) * 3 + (q + 1)];
+  }
+};
+template <class F> void each(const Tensor &t, F f) {
+  for (int a = -t.l1; a <= t.l1; ++a)
+    for (int b = -t.l2; b <= t.l2; ++b)
+      for (int q = -1; q <= 1; ++q) f(a, b, q);
+}
+double ladder(int l, int m, int s) { return std::sqrt(double(l * (l + 1) - m * (m + s))); }  // m -> m + s
+// J_s T, s = +1 or -1: the sum of the three ladder operators
+Tensor shift(const Tensor &t, int s) {
+  Tensor o(t.l1, t.l2);
+  each(t, [&](int a, int b, int q) {
+    cplx x = 0.0;
+    if (std::abs(a - s) <= t.l1) x += ladder(t.l1, a - s, s) * t.get(a - s, b, q);
+    if (std::abs(b - s) <= t.l2) x += ladder(t.l2, b - s, s) * t.get(a, b - s, q);
+    if (std::abs(q - s) <= 1) x += ladder(1, q - s, s) * t.get(a, b, q - s);
+    o.at(a, b, q) = x;
+  });
+  return o;
+}
+Tensor slice(const Tensor &t, int K) {
+  Tensor o(t.l1, t.l2);
+  each(t, [&](int a, int b, int q) {
+    if (a + b + q == K) o.at(a, b, q) = t.get(a, b, q);
+  });
+  return o;
+}
+double norm2(const Tensor &t) {
+  double n = 0.0;
+  for (const cplx &x : t.v) n += std::norm(x);
+  return n;
+}
+// P_l^m(cos theta) cos or sin (m phi) (Condon-Shortley) over the complex harmonics
+void real_harmonic(int l, int m, int cs, std::vector<cplx> &v) {
+  v.assign(2 * l + 1, 0.0);
+  double r = 1.0;  // (l + m)! / (l - m)!
+  for (int k = l - m + 1; k <= l + m; ++k) r *= k;
+  const double n = std::sqrt((2 * l + 1) / (4.0 * M_PI) / r), sg = (m & 1) ? -1.0 : 1.0;
+  if (m == 0) {
+    v[l] = 1.0 / n;
+  } else if (cs == 0) {
+    v[l + m] = 0.5 / n;
+    v[l - m] = 0.5 * sg / n;
+  } else {
+    v[l + m] = cplx(0.0, -0.5) / n;
+    v[l - m] = cplx(0.0, 0.5) * sg / n;
+  }
+}
+using Poly = std::vector<cplx>;  // coefficients K = -J..J
+Poly mul(const Poly &a, const Poly &b) {
+  Poly o(a.size() + b.size() - 1, 0.0);
+  for (size_t i = 0; i < a.size(); ++i)
+    for (size_t j = 0; j < b.size(); ++j) o[i + j] += a[i] * b[j];
+  return o;
+}
+Poly comb(const Poly &a, double x, const Poly &b) {
+  Poly o(a);
+  for (size_t i = 0; i < o.size(); ++i) o[i] += x * b[i];
+  return o;
+}
+// the invariants' coefficients in the body frame itself (e1 = x, e2 = y, n1 = z)
+void invariants(Poly (&I)[hh::CH4C_NJ]) {
+  const cplx i1(0.0, 1.0);
+  const Poly ux = {1.0, 0.0, -1.0}, uy = {i1, 0.0, i1}, uz = {0.0, 2.0, 0.0};
+  const Poly xy = mul(ux, uy), zz = mul(uz, uz);
+  I[0] = {1.0};
+  I[1] = mul(xy, uz);
+  I[2] = mul(comb(zz, -1.0, xy), comb(zz, 1.0, xy));
+  I[3] = mul(I[1], I[1]);
+  Poly d = mul(comb(mul(ux, ux), -1.0, mul(uy, uy)), comb(mul(xy, xy), 2.0, mul(zz, zz)));
+  for (cplx &x : d) x *= i1;
+  I[4] = d;
+  I[5] = mul(I[1], I[2]);
+  I[6] = mul(I[2], I[2]);
+  I[7] = mul(I[1], I[3]);
+  I[8] = mul(I[2], I[3]);
+}
+double sqrt_binom(int J, int K) {  // sqrt((2J)! / ((J+K)! (J-K)!))
+  double b = 1.0;
+  for (int k = 1; k <= J - K; ++k) b = b * (J + K + k) / k;
+  return std::sqrt(b);
+}
+}  // namespace
+
+int ch4co2_build_coupled(Ch4Co2CoupledHost *out) {
+  using namespace hh;
+  Poly I[CH4C_NJ];
+  invariants(I);
+  // basis functions from the term list
+  std::map<int, std::vector<int>> terms;
+  for (int t = 0; t < HH_CH4CO2_NTERM; ++t) terms[hh_ch4co2_tidx[t][0]].push_back(t);
+  const double s2 = std::sqrt(0.5);
+  const cplx cart[3][3] = {{s2, 0.0, -s2}, {cplx(0.0, s2), 0.0, cplx(0.0, s2)}, {0.0, 1.0, 0.0}};  // e_x, e_y, e_z over q
+  // g[(jx, m2, q)][l2][b]: the real coefficient of rad_b p_K P_l2^|m2|
+  std::map<std::tuple<int, int, int>, std::map<int, std::vector<std::pair<int, double>>>> G;
+  for (const auto &kv : terms) {
+    const int b = kv.first;
+    int l1, m1, c1, l2, m2, c2;
+    lm_of(hh_ch4co2_tidx[kv.second[0]][2], &l1, &m1, &c1);
+    lm_of(hh_ch4co2_tidx[kv.second[0]][3], &l2, &m2, &c2);
+    if (l2 > CH4C_LMAX || (l2 & 1)) return -1;
+    Tensor T(l1, l2);
+    std::vector<cplx> y1, y2;
+    for (int t : kv.second) {
+      const short *ix = hh_ch4co2_tidx[t];
+      int a, am, ac, e, em, ec;
+      lm_of(ix[2], &a, &am, &ac);
+      lm_of(ix[3], &e, &em, &ec);
+      if (a != l1 || e != l2) return -1;
+      real_harmonic(a, am, ac, y1);
+      real_harmonic(e, em, ec, y2);
+      for (int p = -l1; p <= l1; ++p)
+        if (y1[p + l1] != 0.0)
+          for (int r = -l2; r <= l2; ++r)
+            if (y2[r + l2] != 0.0)
+              for (int q = -1; q <= 1; ++q)
+                T.at(p, r, q) += hh_ch4co2_tcoef[t] * y1[p + l1] * y2[r + l2] * cart[ix[1]][q + 1];
+    }
+    const double n2 = norm2(T);
+    if (!(n2 > 0.0)) continue;
+    // J from <J^2> = |J_- T|^2 + <Jz^2 - Jz>
+    double jj = norm2(shift(T, -1)) / n2, kz = 0.0;
+    each(T, [&](int a, int e, int q) {
+      const int K = a + e + q;
+      kz += double(K) * (K - 1) * std::norm(T.get(a, e, q));
+    });
+    jj += kz / n2;
+    const double Jr = 0.5 * (std::sqrt(1.0 + 4.0 * jj) - 1.0);
+    const int J = (int)std::lround(Jr);
+    int jx = -1;
+    for (int k = 0; k < CH4C_NJ; ++k)
+      if (CH4C_J[k] == J && (k == 4) == (((l1 + l2 + 1 + J) & 1) != 0)) jx = k;
+    if (jx < 0 || std::abs(Jr - J) > 1e-6) return -1;
+    // the strongest K of the invariant, its slice, and the ladder from there to every K
+    int K0 = 0;
+    for (int K = 1; K <= J; ++K)
+      if (std::abs(I[jx][K + J]) / sqrt_binom(J, K) > 1.0001 * std::abs(I[jx][K0 + J]) / sqrt_binom(J, K0)) K0 = K;
+    const cplx alpha = sqrt_binom(J, K0) / I[jx][K0 + J];
+    std::map<int, Tensor> sl;
+    sl.emplace(K0, slice(T, K0));
+    for (int K = K0; K < J; ++K) {
+      Tensor n = shift(sl.at(K), 1);
+      for (cplx &x : n.v) x /= ladder(J, K, 1);
+      sl.emplace(K + 1, n);
+    }
+    for (int K = K0; K > -J; --K) {
+      Tensor n = shift(sl.at(K), -1);
+      for (cplx &x : n.v) x /= ladder(J, K, -1);
+      sl.emplace(K - 1, n);
+    }
+    // T = sum_K a_K |J K> with a_K = p_K / sqrt_binom(K) / alpha'
+    double off = 0.0;
+    each(T, [&](int a, int e, int q) {
+      const int K = a + e + q;
+      cplx x = T.get(a, e, q);
+      if (std::abs(K) <= J) x -= alpha * I[jx][K + J] / sqrt_binom(J, K) * sl.at(K).get(a, e, q);
+      off += std::norm(x);
+    });
+    if (!(off < 1e-18 * n2)) return -1;
+    const double yy = std::sqrt(double(2 * l1 + 1) * (2 * l2 + 1)) / (4.0 * M_PI);
+    for (int K = -J; K <= J; ++K)
+      for (int q = 0; q <= 1; ++q) {
+        const int mm = K - q;
+        if (std::abs(mm) > l2 || (q == 0 && mm < 0)) continue;
+        cplx gv = alpha * sl.at(K).get(0, mm, q) * yy / sqrt_binom(J, K);
+        if (mm < 0 && (mm & 1)) gv = -gv;       // P^{-m} = (-1)^m P^m in this normalisation
+        if (std::abs(gv.imag()) > 1e-10 * std::abs(gv) + 1e-14) return -1;
+        double gr = gv.real();
+        if (q == 0 && mm > 0) gr *= 2.0;        // m and -m add conjugate terms
+        // p_K of K < 0 from p_|K|
+        if (K < 0 && ((K & 1) != 0) != (jx == 4)) gr = -gr;
+        if (gr != 0.0) G[{jx, mm, q}][l2].push_back({b, gr});
+      }
+  }
+  // groups in the kernel's order
+  struct Grp {
+    int jx, mm, q, n;
+  };
+  std::vector<Grp> order;
+  for (int m = 0; m <= CH4C_LMAX; ++m) {
+    std::vector<Grp> at;
+    for (const auto &kv : G) {
+      int jx, mm, q;
+      std::tie(jx, mm, q) = kv.first;
+      if (std::abs(mm) != m) continue;
+      const int lmax = kv.second.rbegin()->first;
+      at.push_back({jx, mm, q, (lmax - ch4c_l0(m)) / 2 + 1});
+    }
+    std::stable_sort(at.begin(), at.end(), [](const Grp &x, const Grp &y) { return x.n > y.n; });
+    for (const Grp &x : at) {
+      if (x.n < 1 || x.n > ch4c_nl(m)) return -1;
+      out->count[m][x.n]++;
+      order.push_back(x);
+    }
+  }
+  out->n_group = (int)order.size();
+  out->n_coef = 0;
+  for (const Grp &x : order) out->n_coef += x.n;
+  if (out->n_coef > CH4C_MAXCOEF || out->n_group > CH4C_MAXGROUP) return -1;
+  out->desc.clear();
+  out->coef.assign((size_t)HH_CH4CO2_NSEG * out->n_coef * 4, 0.0);
+  int c = 0;
+  for (const Grp &x : order) {
+    const int K = x.mm + x.q;
+    out->desc.push_back((unsigned short)((CH4C_TAU[x.jx] + std::abs(K)) | (x.q << 8) | ((K < 0 ? 1 : 0) << 9)));
+    const auto &by_l = G[{x.jx, x.mm, x.q}];
+    for (int i = 0; i < x.n; ++i, ++c) {
+      const auto it = by_l.find(ch4c_l0(std::abs(x.mm)) + 2 * i);
+      if (it == by_l.end()) continue;
+      for (const auto &br : it->second)
+        for (int s = 0; s < HH_CH4CO2_NSEG; ++s)
+          for (int j = 0; j < 4; ++j)
+            out->coef[((size_t)s * out->n_coef + c) * 4 + j] += br.second * hh_ch4co2_rad[br.first][s][j];
+    }
+  }
   return 0;
 }

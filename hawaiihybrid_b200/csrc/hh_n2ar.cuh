@@ -357,7 +357,8 @@ __device__ __forceinline__ void n2ar_coop_init(N2arCoopWeights<T> *cw, N2arCoopS
 // the order of the per-lane loop, and the sums of j1_i a_i / xscale_i and j2_i a_i /
 // xscale_i over i in order on every lane.  The values pass through shared memory.  A
 // trajectory therefore takes the same steps in the solo kernel as in the bulk kernel.  All
-// 32 lanes call it with the same arguments but code (n2ar_pip_code).  Latency bounds it (one right-hand side: 3,700 cycles in FP64): with every
+// 32 lanes call it with the same arguments but code (n2ar_pip_code).  Latency bounds it
+// (one right-hand side: 3,700 cycles in FP64): with every
 // lane forming all the inputs and values passed by shuffles the solo launch took, in FP64
 // (20,011 x 5,000), 60.7 ms, so 42 to 47; on the mixed path (131,072 x 16,384) 41.5 and 39.7.
 template <typename T>

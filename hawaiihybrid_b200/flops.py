@@ -51,6 +51,11 @@ def ch4_dipole_flops(n_entries_padded: int, n_groups: int) -> int:
     return 8 * n_entries_padded + 10 * n_groups + 600
 
 
+# CH4-CO2 FP64 dipole in coupled form (ch4_dipole_coupled_kernel) per record: 591 cubics (4
+# FMA each), 156 group ends (about 1.6 FMA), 330 complex products of the rotated invariants
+# (4 FMA), the Legendre values (about 180) and the frame (about 260)
+CH4_COUPLED_FLOPS = 2 * (4 * 591 + 250 + 4 * 330) + 180 + 260
+
 # CH4-CO2 tensor-core dipole (ch4_dipole_tc_kernel): per 128-record task, pass 0 runs two
 # 208-column component tiles and pass 1 one, over K = 368 in chunks of 16, each MMA of
 # M = 128, N = 208, K = 8 issued three times (A_hi B_hi, A_hi B_lo, A_lo B_hi)

@@ -323,7 +323,8 @@ int hh_cuda_debug_n2ar_dipole(int precision, const double *R, const double *T, u
 /* Diagnostic (no counterpart in the reference): the CH4-CO2 dipole kernel variant
  * that the tuner picked for the FP64 and the mixed path on the first record-path call
  * of this context: records per lane (1, 2 or 4) of the CUDA-core kernel, -1 for the
- * tensor-core kernel (mixed path only), 0 before that call. */
+ * tensor-core kernel (mixed path only), -2 for the coupled-form kernel (FP64 path only,
+ * taken there without timing), 0 before that call. */
 int hh_cuda_debug_tuning(int *ch4_dip_s_fp64, int *ch4_dip_s_mixed);
 /* Tuning knob (no counterpart in the reference): fixes the CH4-CO2 dipole kernel
  * variant of `precision` (values as above; 0 lets the tuner time them again on the
