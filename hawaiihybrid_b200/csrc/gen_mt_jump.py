@@ -34,7 +34,7 @@ N, M = 624, 397
 MATRIX_A = np.uint32(0x9908B0DF)
 UPPER, LOWER = np.uint32(0x80000000), np.uint32(0x7FFFFFFF)
 DEG = 19937
-SEG_BLOCKS = 2048               # 624-word blocks per generated segment
+SEG_BLOCKS = 512                # 624-word blocks per generated segment
 SEG_WORDS = SEG_BLOCKS * N
 COARSE = 32                     # segments per coarse jump
 

@@ -144,7 +144,8 @@ struct Ctx {
   DevBuf<double> qp_cand, energy, qp0;
   DevBuf<unsigned int> block_counts;
   DevBuf<long long> cand_idx;
-  DevBuf<unsigned long long> scal;  // [0] first_irregular, [1] total
+  DevBuf<unsigned long long> scal;  // [0] first_irregular, [1] total, [2] prefilter list length
+  DevBuf<unsigned int> cand_list;   // CH4-CO2: candidates the prefilter leaves
   // trajectories
   DevBuf<double> crln;
   DevBuf<unsigned long long> counters;
@@ -264,7 +265,7 @@ int gen_blocks(uint32_t *out, long long nblk, cudaStream_t s) {
     const int nseg = (int)(nblk / MT_SEG_BLOCKS);
     CK(g.mt_seg_states.ensure((size_t)nseg * MT_N));
     CK(launch_mt_generate_segments(g.d_mt, out, nseg, g.mt_seg_states.p, g.d_mt_jump_seg, g.d_mt_jump_coarse, s));
-    g_launches += 4;
+    g_launches += 2 + (nseg - 1) / 32;  // coarse jumps one by one, fine jumps, words
   } else {
     CK(launch_mt_generate(g.d_mt, out, nblk, s));
     g_launches += 1;
@@ -352,21 +353,24 @@ int sample_into(const hh_calc_params *p, double T, uint64_t n, double *d_out, ui
   while (got < n) {
     long long remaining = (long long)(n - got);
     double pe = std::max(g.p_accept, 0.01);
+    // 4,096 candidates of headroom: a request for 64 trajectories makes 44 thousand words of
+    // the sequential stream (0.04 ms), not the 655 thousand of a minimum round of 65,536
     long long ncand = (long long)(remaining / pe * 1.15) + 4096;
-    ncand = std::min(std::max(ncand, 65536LL), 1LL << 23);
+    ncand = std::min(ncand, 1LL << 23);
     int rc = ensure_words(g.wpos + ncand * g.D + 4096);
     if (rc) return rc;
     CK(g.accept.ensure(ncand));
     CK(g.consumed.ensure(ncand));
     CK(g.qp_cand.ensure((size_t)ncand * g.QP));
     CK(g.energy.ensure(ncand));
+    if (g.sys == SYS_CH4CO2) CK(g.cand_list.ensure(ncand));
     CK(g.block_counts.ensure((ncand + 1023) / 1024 + 1));
     CK(cudaMemsetAsync(g.scal.p, 0xff, sizeof(unsigned long long), g.st));
     CK(launch_candidates(g.sys, g.mu, g.II, T, p->sampler_Rmin, p->sampler_Rmax, p->pesmin,
                          p->pair_state, g.d_tab, g.words[g.cur].p, g.wvalid, g.wpos - g.wbase, g.D,
                          ncand, g.accept.p, g.consumed.p, g.qp_cand.p, g.energy.p, g.scal.p,
-                         g.sx, g.st));
-    g_launches += 1;
+                         g.sx, g.sys == SYS_CH4CO2 ? g.cand_list.p : nullptr, g.scal.p + 2, g.st));
+    g_launches += g.sys == SYS_CH4CO2 ? 2 : 1;
     unsigned long long first_irr = 0;
     CK(cudaMemcpyAsync(&first_irr, g.scal.p, sizeof first_irr, cudaMemcpyDeviceToHost, g.st));
     CK(cudaStreamSynchronize(g.st));
@@ -2616,6 +2620,7 @@ void hh_cuda_shutdown(void) {
   g.consumed.release();
   g.qp_cand.release();
   g.energy.release();
+  g.cand_list.release();
   g.qp0.release();
   g.block_counts.release();
   g.cand_idx.release();

@@ -1,4 +1,6 @@
 // Sampler translation unit of libhh_cuda.so (built with -fmad=false).
+#include <algorithm>
+
 #include "hh_internal.h"
 #include "hh_sampler.cuh"
 
@@ -15,28 +17,32 @@ cudaError_t launch_mt_generate(uint32_t *state, uint32_t *out, long long n_block
   return cudaGetLastError();
 }
 
-size_t mt_jump_smem() { return MT_JUMP_WIN * sizeof(uint32_t) + 10240 * sizeof(unsigned short); }
+size_t mt_jump_smem() { return MT_JUMP_WIN * sizeof(uint32_t) + MT_JUMP_PART * sizeof(unsigned short); }
 
 cudaError_t launch_mt_generate_segments(uint32_t *state, uint32_t *out, int n_seg, uint32_t *seg_states,
                                         const unsigned short *jump_seg, const unsigned short *jump_coarse,
                                         cudaStream_t st) {
   static_assert(HH_MT_JUMP_SEG_N <= 10240 && HH_MT_JUMP_COARSE_N <= 10240, "jump tables exceed the buffer");
   const size_t smem = mt_jump_smem();
-  cudaError_t e = cudaFuncSetAttribute(mt_jump_chain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = cudaFuncSetAttribute(mt_jump_coarse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
-  // segment 0 starts from the current state
+  // segment 0 starts from the current state; the jumps add into zeros
+  e = cudaMemsetAsync(seg_states, 0, (size_t)n_seg * MT_N * sizeof(uint32_t), st);
+  if (e != cudaSuccess) return e;
   e = cudaMemcpyAsync(seg_states, state, MT_N * sizeof(uint32_t), cudaMemcpyDeviceToDevice, st);
   if (e != cudaSuccess) return e;
   const int n_coarse = (n_seg + HH_MT_COARSE - 1) / HH_MT_COARSE;
-  // coarse chain on one CTA: states 0, C, 2C, ...; then every other segment state
-  // by one jump from its interval's start (the fine tables follow the segment table
-  // in the same buffer: mt_jump_fine_tables)
-  mt_jump_chain_kernel<<<1, MT_JUMP_THREADS, smem, st>>>(seg_states, 0, HH_MT_COARSE, n_coarse - 1, n_seg,
-                                                         jump_coarse, HH_MT_JUMP_COARSE_N);
+  // states 0, C, 2C, ... one after the other; then every other segment state by one jump
+  // from its interval's start (the fine tables follow the segment table in the same
+  // buffer: mt_jump_fine_tables)
+  for (int k = 1; k < n_coarse; ++k)
+    mt_jump_coarse_kernel<<<MT_JUMP_SPLIT, MT_JUMP_THREADS, smem, st>>>(
+        seg_states, (k - 1) * HH_MT_COARSE, k * HH_MT_COARSE, jump_coarse, HH_MT_JUMP_COARSE_N);
   if (n_seg > 1) {
     e = cudaFuncSetAttribute(mt_jump_fine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    mt_jump_fine_kernel<<<n_coarse * (HH_MT_COARSE - 1), MT_JUMP_THREADS, smem, st>>>(
+    const int n_fine = std::min(n_coarse * (HH_MT_COARSE - 1), n_seg - 1);
+    mt_jump_fine_kernel<<<dim3(n_fine, MT_JUMP_SPLIT), MT_JUMP_THREADS, smem, st>>>(
         seg_states, n_seg, jump_seg + MT_FINE_OFFSET, jump_seg + MT_FINE_OFFSET + (HH_MT_COARSE - 1) * HH_MT_JUMP_FINE_MAX);
   }
   mt_generate_segments_kernel<<<n_seg, 256, 0, st>>>(seg_states, out, n_seg, state);
@@ -66,13 +72,24 @@ cudaError_t launch_candidates(int sys, double mu, double II, double T, double Rm
                               const uint32_t *words, long long n_words, long long word_base, int D,
                               long long n_cand, unsigned char *accept, unsigned char *consumed,
                               double *qp, double *energy, unsigned long long *first_irregular,
-                              const SamplerExtra &x, cudaStream_t st) {
+                              const SamplerExtra &x, unsigned *list, unsigned long long *n_list, cudaStream_t st) {
   SamplerArgs a{sys, mu, II, T, Rmin, Rmax, pesmin, pair_state, x};
   size_t smem = (sys == SYS_CO2AR) ? sizeof(Co2arTables<double>) : 0;
   long long blocks = (n_cand + 255) / 256;
+  const unsigned *cl = nullptr;
+  if (list && sys == SYS_CH4CO2 && D == 25) {
+    // the words of every candidate's regular window are there: n_words covers them
+    cudaError_t e = cudaMemsetAsync(n_list, 0, sizeof(unsigned long long), st);
+    if (e != cudaSuccess) return e;
+    ch4_prefilter_kernel<<<(unsigned)blocks, 256, 0, st>>>(a, words, word_base, n_cand, accept, consumed, list, n_list);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    cl = list;
+    blocks = blocks < 1184 ? blocks : 1184;
+  }
   candidate_kernel<<<(unsigned)blocks, 256, smem, st>>>(a, gtab, words, n_words, word_base, D,
                                                          n_cand, accept, consumed, qp, energy,
-                                                         first_irregular);
+                                                         first_irregular, cl, n_list);
   return cudaGetLastError();
 }
 

@@ -11,8 +11,8 @@
 // retries when its first word is exactly 0 (log(0) = -inf).
 //
 // GPU mapping:
-//  1. mt_generate: one CTA advances the MT state 624 words at a time with a
-//     three-phase parallel refresh and writes the tempered words to HBM;
+//  1. mt_generate: one CTA advances the stream 227 words at a time in a ring in shared
+//     memory and writes the tempered words to HBM;
 //  2. candidates: one thread per candidate c reads the words [c*D, (c+1)*D),
 //     restates q_generator/p_generator/Hamiltonian/reject/pair-state filter in
 //     FP64 with the reference's operation order, and flags acceptance;
@@ -25,9 +25,9 @@
 // Long requests of the stream (the 100 K rejection step of CH4-CO2 takes about
 // 1.5e9 words per call) are generated in segments of HH_MT_SEG_BLOCKS blocks, one
 // CTA each, from segment start states found by jumping ahead (hh_mt_jump.h):
-// a chain of coarse jumps (HH_MT_COARSE segments each) on one CTA, then the fine
-// jumps of every coarse interval in parallel.  The words are the same as those of
-// the sequential generator.
+// a chain of coarse jumps (HH_MT_COARSE segments each), then the fine jumps of every
+// coarse interval in parallel.  The words are the same as those of the sequential
+// generator.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -69,146 +69,117 @@ __global__ void mt_seed_kernel(uint32_t seed, uint32_t *state) {
   state[i] = p * seed;
 }
 
-// Advance the generator by n_blocks refreshes, writing 624 tempered words per
-// refresh to out.  One CTA of 256 threads; the state lives in shared memory.
-// one refresh of the 624 words in shared memory, in place (three dependency
-// phases); every thread of the CTA (>= 227 threads) calls it
-__device__ __forceinline__ void mt_refresh_smem(uint32_t *mt) {
-  const int tid = threadIdx.x;
-  uint32_t v;
-  if (tid < MT_N - MT_M) v = mt_twist(mt[tid], mt[tid + 1], mt[tid + MT_M]);
-  __syncthreads();
-  if (tid < MT_N - MT_M) mt[tid] = v;
-  __syncthreads();
-  {
-    int i = tid + (MT_N - MT_M);
-    if (tid < MT_N - MT_M) v = mt_twist(mt[i], mt[i + 1], mt[i - (MT_N - MT_M)]);
-    __syncthreads();
-    if (tid < MT_N - MT_M) mt[i] = v;
-    __syncthreads();
-  }
-  {
-    int i = tid + 2 * (MT_N - MT_M);
-    if (i < MT_N) v = mt_twist(mt[i], mt[(i + 1) % MT_N], mt[i - (MT_N - MT_M)]);
-    __syncthreads();
-    if (i < MT_N) mt[i] = v;
+// The stream word after word, 227 at a time: x_{n+624} depends on x_n, x_{n+1} and x_{n+397},
+// and x_{n+397} is the word that the same thread formed one step earlier, so it stays in a
+// register and only x_n and x_{n+1} are read, from words formed two or three steps earlier.
+// One barrier per two steps therefore orders the reads behind the writes; the ring of 2,048
+// words is long enough that a step overwrites only words last read six steps before.
+// 0.26 us per block of 624; a block-wise refresh in place (six barriers) took 0.51.
+//
+// mt_words: the words x_624 .. x_{n_words + 623} after the state x_0 .. x_623 in buf, where
+// x_n is at buf[n & mask]; every new word goes to emit(n - 624, x_n).  256 threads, all
+// calling; the caller's barrier follows the filling of buf, and one ends the call.
+constexpr int MT_RING = 2048;
+template <typename Emit>
+__device__ __forceinline__ void mt_words(uint32_t *buf, unsigned mask, long long n_words, const Emit &emit) {
+  constexpr unsigned W = MT_N - MT_M;
+  const unsigned tid = threadIdx.x;
+  const bool on = tid < W;
+  unsigned n = tid;
+  uint32_t prev = on ? buf[(n + MT_M) & mask] : 0u;
+  const long long turns = (n_words + 2 * W - 1) / (2 * W);
+  long long j = tid;
+  for (long long t = 0; t < turns; ++t) {
+    if (on) {
+      // both steps' words first: they were formed before the last barrier
+      const uint32_t a0 = buf[n & mask], b0 = buf[(n + 1) & mask];
+      const uint32_t a1 = buf[(n + W) & mask], b1 = buf[(n + W + 1) & mask];
+      const uint32_t x0 = mt_twist(a0, b0, prev), x1 = mt_twist(a1, b1, x0);
+      if (j < n_words) {
+        buf[(n + MT_N) & mask] = x0;
+        emit(j, x0);
+      }
+      if (j + W < n_words) {
+        buf[(n + W + MT_N) & mask] = x1;
+        emit(j + W, x1);
+      }
+      prev = x1;
+      n += 2 * W;
+      j += 2 * W;
+    }
     __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(256) mt_generate_kernel(uint32_t *state, uint32_t *out,
-                                                          long long n_blocks) {
-  __shared__ uint32_t mt[MT_N];
-  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) mt[i] = state[i];
-  __syncthreads();
+// n_words of the stream after the block state `from` (global memory), tempered, to out, by
+// one CTA; the 624 words that end the stream to `to` unless null.
+__device__ __forceinline__ void mt_stream(const uint32_t *from, uint32_t *out, long long n_words, uint32_t *to,
+                                          uint32_t *ring) {
   const int tid = threadIdx.x;
-  for (long long b = 0; b < n_blocks; ++b) {
-    uint32_t v;
-    // phase A: i in [0, 227) depends on old words only
-    if (tid < MT_N - MT_M) v = mt_twist(mt[tid], mt[tid + 1], mt[tid + MT_M]);
-    __syncthreads();
-    if (tid < MT_N - MT_M) mt[tid] = v;
-    __syncthreads();
-    // phase B: i in [227, 454) uses new words i-227 from phase A
-    {
-      int i = tid + (MT_N - MT_M);
-      if (tid < MT_N - MT_M) v = mt_twist(mt[i], mt[i + 1], mt[i - (MT_N - MT_M)]);
-      __syncthreads();
-      if (tid < MT_N - MT_M) mt[i] = v;
-      __syncthreads();
-    }
-    // phase C: i in [454, 624); the last word wraps to the new mt[0]
-    {
-      int i = tid + 2 * (MT_N - MT_M);
-      if (i < MT_N) v = mt_twist(mt[i], mt[(i + 1) % MT_N], mt[i - (MT_N - MT_M)]);
-      __syncthreads();
-      if (i < MT_N) mt[i] = v;
-      __syncthreads();
-    }
-    uint32_t *o = out + b * MT_N;
-    for (int i = tid; i < MT_N; i += blockDim.x) o[i] = mt_temper(mt[i]);
-  }
+  for (int i = tid; i < MT_N; i += blockDim.x) ring[i] = from[i];
   __syncthreads();
-  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) state[i] = mt[i];
+  mt_words(ring, MT_RING - 1, n_words, [&](long long j, uint32_t x) { out[j] = mt_temper(x); });
+  if (to) {
+    for (int i = tid; i < MT_N; i += blockDim.x) to[i] = ring[(unsigned)(n_words + i) & (MT_RING - 1)];
+  }
 }
 
-// Chains of jumps: CTA c starts from states[c * chain_stride] (a 624-word block
-// state) and writes the states `step`, 2 step, ... n_jumps * step segments later to
-// states[c * chain_stride + k * step], k = 1..n_jumps, stopping before index n_states.
-// One jump of J words (bits: set-bit positions of x^J mod phi) XORs windows of the
-// 19,937 + 623 stream words after the state, which are generated in shared memory.
+// Advance the generator by n_blocks refreshes, writing 624 tempered words per refresh to out.
+__global__ void __launch_bounds__(256) mt_generate_kernel(uint32_t *state, uint32_t *out, long long n_blocks) {
+  __shared__ uint32_t ring[MT_RING];
+  mt_stream(state, out, n_blocks * MT_N, state, ring);
+}
+
+// One jump of J words: the state J words after `src` is the XOR of the windows, at the
+// set-bit positions of x^J mod phi, of the 19,937 + 623 stream words after src, which each
+// CTA generates in shared memory.  MT_JUMP_SPLIT CTAs share the positions and XOR their
+// parts into dst (zero before): the windows' reads, about 9,950 x 624 words, bound a jump
+// (0.24 ms in one CTA, 0.03 so).
 constexpr int MT_JUMP_WIN = 33 * MT_N;  // the state and the 32 blocks after it
 constexpr int MT_JUMP_THREADS = 640;
-__global__ void __launch_bounds__(MT_JUMP_THREADS) mt_jump_chain_kernel(uint32_t *states, int chain_stride,
-                                                                       int step, int n_jumps, int n_states,
-                                                                       const unsigned short *bits, int n_bits) {
-  extern __shared__ uint32_t jsm[];
-  uint32_t *win = jsm;                                         // MT_JUMP_WIN words
-  unsigned short *bs = reinterpret_cast<unsigned short *>(jsm + MT_JUMP_WIN);
-  for (int i = threadIdx.x; i < n_bits; i += blockDim.x) bs[i] = bits[i];
-  const long long base = (long long)blockIdx.x * chain_stride;
-  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) win[i] = states[base * MT_N + i];
+constexpr int MT_JUMP_SPLIT = 8;
+constexpr int MT_JUMP_PART = (10240 + MT_JUMP_SPLIT - 1) / MT_JUMP_SPLIT;
+__device__ __forceinline__ void mt_jump(const uint32_t *src, uint32_t *dst, const unsigned short *bits, int n_bits,
+                                        int part, uint32_t *win, unsigned short *bs) {
+  const int lo = part * MT_JUMP_PART, hi = min(n_bits, lo + MT_JUMP_PART);
+  if (lo >= hi) return;  // the whole block
+  for (int i = lo + threadIdx.x; i < hi; i += blockDim.x) bs[i - lo] = bits[i];
+  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) win[i] = src[i];
   __syncthreads();
-  for (int k = 1; k <= n_jumps; ++k) {
-    const long long dst = base + (long long)k * step;
-    if (dst >= n_states) break;
-    // the 32 blocks after the state: block b + 1 from block b, refreshed in place in
-    // a copy at its own position
-    for (int b = 0; b < 32; ++b) {
-      uint32_t *cur = win + (b + 1) * MT_N;
-      for (int i = threadIdx.x; i < MT_N; i += blockDim.x) cur[i] = win[b * MT_N + i];
-      __syncthreads();
-      mt_refresh_smem(cur);
-    }
+  mt_words(win, 0xffffffffu, MT_JUMP_WIN - MT_N, [](long long, uint32_t) {});
+  if (threadIdx.x < MT_N) {
+    const int j = threadIdx.x;
     uint32_t acc = 0;
-    if (threadIdx.x < MT_N) {
-      const int j = threadIdx.x;
-#pragma unroll 4
-      for (int t = 0; t < n_bits; ++t) acc ^= win[bs[t] + j];
-    }
-    __syncthreads();
-    if (threadIdx.x < MT_N) {
-      win[threadIdx.x] = acc;
-      states[dst * MT_N + threadIdx.x] = acc;
-    }
-    __syncthreads();
+#pragma unroll 8
+    for (int t = 0; t < hi - lo; ++t) acc ^= win[bs[t] + j];
+    atomicXor(&dst[j], acc);
   }
 }
 
-// Fine jumps: CTA b computes segment s = (b / 31) * 32 + b % 31 + 1 (skipping the
-// coarse states, which the chain made) by one jump of k = s % 32 segments from
-// states[s - k] with the table of x^(k J) mod phi, so every segment state of a round
-// is one jump deep instead of a chain of up to 31.
+// The jump from states[base] to states[dst]: grid MT_JUMP_SPLIT.
+__global__ void __launch_bounds__(MT_JUMP_THREADS) mt_jump_coarse_kernel(uint32_t *states, int base, int dst,
+                                                                        const unsigned short *bits, int n_bits) {
+  extern __shared__ uint32_t jsm[];
+  mt_jump(states + (size_t)base * MT_N, states + (size_t)dst * MT_N, bits, n_bits, blockIdx.x, jsm,
+          reinterpret_cast<unsigned short *>(jsm + MT_JUMP_WIN));
+}
+
+// Fine jumps: CTA (b, part) adds its part of segment s = (b / 31) * 32 + b % 31 + 1 (skipping
+// the coarse states, which the chain made), one jump of k = s % 32 segments from
+// states[s - k] with the table of x^(k J) mod phi, so every segment state of a round is one
+// jump deep instead of a chain of up to 31.
 constexpr size_t MT_FINE_OFFSET = 10240;  // the fine tables' offset in the segment-table buffer
 static_assert(HH_MT_JUMP_FINE_MAX <= 10240, "fine jump table exceeds the buffer");
 __global__ void __launch_bounds__(MT_JUMP_THREADS) mt_jump_fine_kernel(uint32_t *states, int n_seg,
                                                                       const unsigned short *fine,
                                                                       const unsigned short *fine_n) {
   extern __shared__ uint32_t jsm[];
-  uint32_t *win = jsm;                                         // MT_JUMP_WIN words
-  unsigned short *bs = reinterpret_cast<unsigned short *>(jsm + MT_JUMP_WIN);
   constexpr int PER = HH_MT_COARSE - 1;
   const long long s = (long long)(blockIdx.x / PER) * HH_MT_COARSE + (blockIdx.x % PER) + 1;
   if (s >= n_seg) return;  // the whole block
   const int k = (int)(s % HH_MT_COARSE);
-  const int n_bits = fine_n[k - 1];
-  for (int i = threadIdx.x; i < n_bits; i += blockDim.x) bs[i] = fine[(size_t)(k - 1) * HH_MT_JUMP_FINE_MAX + i];
-  const long long base = s - k;
-  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) win[i] = states[base * MT_N + i];
-  __syncthreads();
-  for (int b = 0; b < 32; ++b) {
-    uint32_t *cur = win + (b + 1) * MT_N;
-    for (int i = threadIdx.x; i < MT_N; i += blockDim.x) cur[i] = win[b * MT_N + i];
-    __syncthreads();
-    mt_refresh_smem(cur);
-  }
-  if (threadIdx.x < MT_N) {
-    const int j = threadIdx.x;
-    uint32_t acc = 0;
-#pragma unroll 4
-    for (int t = 0; t < n_bits; ++t) acc ^= win[bs[t] + j];
-    states[s * MT_N + j] = acc;
-  }
+  mt_jump(states + (s - k) * MT_N, states + s * MT_N, fine + (size_t)(k - 1) * HH_MT_JUMP_FINE_MAX, fine_n[k - 1],
+          blockIdx.y, jsm, reinterpret_cast<unsigned short *>(jsm + MT_JUMP_WIN));
 }
 
 // Segment s: HH_MT_SEG_BLOCKS blocks from states[s], tempered words to
@@ -216,18 +187,10 @@ __global__ void __launch_bounds__(MT_JUMP_THREADS) mt_jump_fine_kernel(uint32_t 
 // generator state.
 __global__ void __launch_bounds__(256) mt_generate_segments_kernel(const uint32_t *states, uint32_t *out,
                                                                    int n_seg, uint32_t *final_state) {
-  __shared__ uint32_t mt[MT_N];
+  __shared__ uint32_t ring[MT_RING];
   const int s = blockIdx.x;
-  for (int i = threadIdx.x; i < MT_N; i += blockDim.x) mt[i] = states[(size_t)s * MT_N + i];
-  __syncthreads();
-  uint32_t *o = out + (size_t)s * HH_MT_SEG_BLOCKS * MT_N;
-  for (int b = 0; b < HH_MT_SEG_BLOCKS; ++b) {
-    mt_refresh_smem(mt);
-    for (int i = threadIdx.x; i < MT_N; i += blockDim.x) o[(size_t)b * MT_N + i] = mt_temper(mt[i]);
-  }
-  __syncthreads();
-  if (s == n_seg - 1)
-    for (int i = threadIdx.x; i < MT_N; i += blockDim.x) final_state[i] = mt[i];
+  mt_stream(states + (size_t)s * MT_N, out + (size_t)s * HH_MT_SEG_BLOCKS * MT_N, (long long)HH_MT_SEG_BLOCKS * MT_N,
+            s == n_seg - 1 ? final_state : nullptr, ring);
 }
 
 // reference operation order is kept; FP contraction is disabled for this code
@@ -248,17 +211,91 @@ __device__ __forceinline__ double bm_normal(const uint32_t *w, long long &pos, l
   }
 }
 
-// one thread per candidate; words of candidate c start at word_base + c*D
+// Rejection ahead of the momenta (CH4-CO2, whose 100 K step accepts one candidate in 200).
+// reject() compares exp(-V / kT) / M with the candidate's last uniform u; V depends on the
+// positions alone, which are the first eight words.  One thread per candidate evaluates V
+// in FP32 and rejects at once where the comparison is decided by more than a bound on its
+// error, in the exponent 0.01 + (1e-4 |V| + 1e-7 Hartree) / kT: the FP32 site sum is good to
+// 1e-6 of its terms.  The others, and candidates with a zero word at a Box-Muller
+// position (whose draw is retried), go on the list for candidate_kernel, which decides
+// them as it would have decided all.  14.8e6 candidates: 6.6 ms with all in FP64, so 1.1 ms
+// (bound by reading the words) and 0.8 ms for those left.
+__global__ void __launch_bounds__(256) ch4_prefilter_kernel(SamplerArgs a, const uint32_t *words, long long word_base,
+                                                            long long n_cand, unsigned char *accept,
+                                                            unsigned char *consumed, unsigned *list,
+                                                            unsigned long long *n_list) {
+  constexpr int D = 25;
+  __shared__ uint32_t w_s[256 * D];
+  const long long c0 = blockIdx.x * 256ll;
+  const int m = (int)min(256ll, n_cand - c0);
+  const uint32_t *src = words + word_base + c0 * D;
+  for (int i = threadIdx.x; i < m * D; i += 256) w_s[i] = src[i];
+  __syncthreads();
+  bool keep = false;
+  if (threadIdx.x < m) {
+    const uint32_t *w = w_s + threadIdx.x * D;
+    constexpr float k = 1.f / 4294967296.f;
+#pragma unroll
+    for (int j = 8; j < 24; j += 2) keep = keep || w[j] == 0u;
+    const float rmin3 = float(a.Rmin) * float(a.Rmin) * float(a.Rmin), rmax3 = float(a.Rmax) * float(a.Rmax) * float(a.Rmax);
+    const float R = cbrtf(float(w[0]) * k * (rmax3 - rmin3) + rmin3);
+    // r, the CH4 quaternion and the CO2 axis of ch4co2_qp_to_state
+    float sP, cP, s1, c1, s3, c3, s2, c2;
+    sincospif(2.f * float(w[1]) * k, &sP, &cP);
+    sincospif(float(w[3]) * k, &s1, &c1);   // phi / 2
+    sincospif(float(w[5]) * k, &s3, &c3);   // psi / 2
+    sincospif(2.f * float(w[6]) * k, &s2, &c2);
+    const float cT = 2.f * (float(w[2]) * k) - 1.f, ct = 2.f * (float(w[4]) * k) - 1.f, cu = 2.f * (float(w[7]) * k) - 1.f;
+    const float sT = sqrtf(fmaxf(0.f, (1.f - cT) * (1.f + cT))), su = sqrtf(fmaxf(0.f, (1.f - cu) * (1.f + cu)));
+    const float cb = sqrtf(fmaxf(0.f, 0.5f * (1.f + ct))), sb = sqrtf(fmaxf(0.f, 0.5f * (1.f - ct)));
+    const float r[3] = {-R * sT * cP, -R * sT * sP, R * cT}, u[3] = {-su * c2, -su * s2, cu};
+    const float t0 = c1 * cb, t1 = c1 * sb, t2 = s1 * sb, t3 = s1 * cb;
+    const float q[4] = {t0 * c3 - t3 * s3, t1 * c3 + t2 * s3, t2 * c3 - t1 * s3, t0 * s3 + t3 * c3};
+    float M[3][3];
+    quat_matrix<float>(q, M);
+    const float V = ch4co2_lj<float>(a.x.lj, M, r, u).V;
+    const float ikT = float(HH_HKT / a.T);
+    // ln(exp(-V / kT) / M) against ln u, M = 1.5 exp(-pesmin / kT); a NaN keeps the candidate
+    const float lw = (float(a.pesmin) - V) * ikT - 0.405465f;
+    const float err = 0.01f + (1e-4f * fabsf(V) + 1e-7f) * ikT;
+    keep = keep || !(lw + err < logf(float(w[24]) * k));
+    if (!keep) {
+      accept[c0 + threadIdx.x] = 0;
+      consumed[c0 + threadIdx.x] = D;
+    }
+  }
+  const unsigned bal = __ballot_sync(0xffffffffu, keep);
+  const int lane = threadIdx.x & 31;
+  unsigned base = 0;
+  if (bal && lane == 0) base = (unsigned)atomicAdd(n_list, (unsigned long long)__popc(bal));
+  base = __shfl_sync(0xffffffffu, base, 0);
+  if (keep) list[base + __popc(bal & ((1u << lane) - 1u))] = (unsigned)(c0 + threadIdx.x);
+}
+
+// one thread per candidate (of the list, when there is one: *n_list candidates); words of
+// candidate c start at word_base + c*D
+__device__ __forceinline__ void candidate_at(
+    const SamplerArgs &a, const Co2arTables<double> *tb, const uint32_t *words, long long n_words,
+    long long word_base, int D, long long c, unsigned char *accept, unsigned char *consumed,
+    double *qp_out, double *energy_out, unsigned long long *first_irregular);
 __global__ void __launch_bounds__(256) candidate_kernel(
     SamplerArgs a, const Co2arTablesGlobal *gtab, const uint32_t *words, long long n_words,
     long long word_base, int D, long long n_cand, unsigned char *accept, unsigned char *consumed,
-    double *qp_out, double *energy_out, unsigned long long *first_irregular) {
+    double *qp_out, double *energy_out, unsigned long long *first_irregular, const unsigned *list,
+    const unsigned long long *n_list) {
   extern __shared__ unsigned char smem_raw[];
   Co2arTables<double> *tb = reinterpret_cast<Co2arTables<double> *>(smem_raw);
   if (a.sys == SYS_CO2AR) load_tables<double>(tb, gtab);
   __syncthreads();
-  long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (c >= n_cand) return;
+  const long long n = list ? (long long)*n_list : n_cand;
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    candidate_at(a, tb, words, n_words, word_base, D, list ? (long long)list[i] : i, accept, consumed, qp_out,
+                 energy_out, first_irregular);
+}
+__device__ __forceinline__ void candidate_at(
+    const SamplerArgs &a, const Co2arTables<double> *tb, const uint32_t *words, long long n_words,
+    long long word_base, int D, long long c, unsigned char *accept, unsigned char *consumed,
+    double *qp_out, double *energy_out, unsigned long long *first_irregular) {
   long long pos = word_base + c * D;
   const long long limit = n_words;
   int retries = 0;
