@@ -1448,13 +1448,32 @@ int run_trajectories(const hh_calc_params *p, const double *d_ic, uint64_t n, ui
   return HH_OK;
 }
 
+// the FP64 M0 kernel of system SYS for the launch's temperatures (TP: the power of two at
+// or above nT)
+template <int SYS> int launch_m0_fp64(const M0Args &a, int grid, size_t smem, double *partials) {
+  auto k = a.nT > 8   ? m0_fp64_kernel<SYS, 16>
+           : a.nT > 4 ? m0_fp64_kernel<SYS, 8>
+           : a.nT > 2 ? m0_fp64_kernel<SYS, 4>
+           : a.nT > 1 ? m0_fp64_kernel<SYS, 2>
+                      : m0_fp64_kernel<SYS, 1>;
+  if (smem > 32 * 1024) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  k<<<grid, 256, smem, g.st>>>(a, g.d_tab, g.d_n2ar_fold, partials);
+  return HH_OK;
+}
+
+// blocks of the bound system's moment kernels: whole waves of what is resident at a time
+int moment_grid(int moment, bool mixed) {
+  return g.num_sms * (moment == 0 && !mixed && g.sys != SYS_N2AR ? M0_FP64_BLOCKS : 4);
+}
+
 // launches the M0 kernel of the bound system over `grid` blocks; allocates nothing
 int launch_m0(const M0Args &a, int grid, bool mixed, double *partials) {
   const int block = 256;
   kt_begin();
+  int rc = HH_OK;
   if (g.sys == SYS_HEAR) {
     if (mixed) m0_kernel<SYS_HEAR, float, true><<<grid, block, 0, g.st>>>(a, g.d_tab, nullptr, partials);
-    else m0_kernel<SYS_HEAR, double, false><<<grid, block, 0, g.st>>>(a, g.d_tab, nullptr, partials);
+    else rc = launch_m0_fp64<SYS_HEAR>(a, grid, 0, partials);
   } else if (g.sys == SYS_N2AR) {
     const size_t smem = sizeof(N2arDipFold);
     if (mixed) {
@@ -1462,18 +1481,16 @@ int launch_m0(const M0Args &a, int grid, bool mixed, double *partials) {
       CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       k<<<grid, block, smem, g.st>>>(a, g.d_tab, g.d_n2ar_fold, partials);
     } else {
-      auto k = m0_kernel<SYS_N2AR, double, false>;
-      CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k<<<grid, block, smem, g.st>>>(a, g.d_tab, g.d_n2ar_fold, partials);
+      rc = launch_m0_fp64<SYS_N2AR>(a, grid, smem, partials);
     }
   } else {
     if (mixed)
       m0_kernel<SYS_CO2AR, float, true><<<grid, block, sizeof(Co2arTables<float>), g.st>>>(
           a, g.d_tab, nullptr, partials);
     else
-      m0_kernel<SYS_CO2AR, double, false><<<grid, block, sizeof(Co2arTables<double>), g.st>>>(
-          a, g.d_tab, nullptr, partials);
+      rc = launch_m0_fp64<SYS_CO2AR>(a, grid, sizeof(Co2arTables<double>), partials);
   }
+  if (rc) return rc;
   CK(cudaGetLastError());
   kt_end(HH_KT_MOMENT);
   return HH_OK;
@@ -2160,7 +2177,7 @@ int hh_cuda_moment_sums(const hh_calc_params *p, const double *T, int nT, uint64
   for (int t = 0; t < nT; ++t)
     if (!(T[t] > 0)) return HH_E_INVALID_ARGUMENT;
   CK(cudaSetDevice(g.device));
-  const int grid = g.num_sms * 4;
+  const int grid = moment_grid(moment, precision_mode == HH_PRECISION_MIXED);
   CK(g.m0_partials.ensure((size_t)grid * M0_MAXT * 2));
   CK(g.m0_out.ensure(M0_MAXT * 2));
   for (int t0 = 0; t0 < nT; t0 += M0_MAXT) {
@@ -2576,7 +2593,7 @@ int hh_cuda_m0_noalloc(const hh_calc_params *p, const double *T, int nT, uint64_
   int rc = m0_noalloc_scratch(g.device, &scratch);
   if (rc) return rc;
   double *partials = scratch, *res = scratch + M0_NOALLOC_PARTIALS;
-  const int grid = std::min(g.num_sms * 4, M0_NOALLOC_MAX_BLOCKS);
+  const int grid = std::min(moment_grid(0, precision_mode == HH_PRECISION_MIXED), M0_NOALLOC_MAX_BLOCKS);
   const int n_chunks = (nT + M0_MAXT - 1) / M0_MAXT;
   CK(cudaMemsetAsync(res, 0, sizeof(double) * 2 * M0_MAXT * n_chunks, g.st));
   for (int c = 0; c < n_chunks; ++c) {
