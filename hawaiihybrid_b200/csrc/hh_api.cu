@@ -79,6 +79,24 @@ template <typename T> struct DevBuf {
   }
 };
 
+template <typename T> struct PinBuf {  // page-locked host memory
+  T *p = nullptr;
+  size_t cap = 0;
+  cudaError_t ensure(size_t n) {
+    if (n <= cap) return cudaSuccess;
+    release();
+    const cudaError_t e = cudaMallocHost(&p, n * sizeof(T));
+    if (e == cudaSuccess) cap = n;
+    else p = nullptr;
+    return e;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    cap = 0;
+  }
+};
+
 struct TrajTune {
   int warps;        // bulk kernel warps per block
   int handoff_div;  // hand-off when at most (solo warp slots) * handoff_mul / handoff_div items are open
@@ -175,18 +193,15 @@ struct Ctx {
   // PR_MU: complex series (two buffers) and the spectrum
   DevBuf<double2> pm_a, pm_b;
   DevBuf<double2> zf_a, zf_b;   // Zimmermann FFT workspace
-  DevBuf<double> pm_sf;
+  DevBuf<double> pm_sf, pm_w, pm_part;  // spectrum, trajectory weights, sums per block
   // M0
   DevBuf<double> m0_partials, m0_out;
   // VEGAS: grid edges, block sums, per-bin sums of F^2
   DevBuf<double> vg_edges, vg_sums, vg_hist;
   // FFT, and the CUDA graph of its kernel sequence for the current (N, dt, buffers)
-  DevBuf<double> f_cf, f_nu, f_sf;
+  DevBuf<double> f_cf, f_sf;
   DevBuf<double2> f_a, f_b;
-  cudaGraphExec_t idct_exec = nullptr;
-  size_t idct_N = 0;
-  double idct_dt = 0.0;
-  const void *idct_bufs[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
+  PinBuf<double> f_pin;
 };
 
 Ctx g;
@@ -800,32 +815,55 @@ int zimm_fft(const ZimmArgs &za) {
   const int N = za.N;
   int L = 1;
   while (L < 2 * N - 1) L <<= 1;
+  const int logL = __builtin_ctz((unsigned)L), passes = fft_passes(logL);
   const size_t per = 3 * (size_t)L * sizeof(double2);
   const long long m = std::max<long long>(1, std::min<long long>(za.n_traj, (long long)(ZIMM_FFT_BUDGET / (2 * per))));
   CK(g.zf_a.ensure(3 * (size_t)m * L));
   CK(g.zf_b.ensure(3 * (size_t)m * L));
-  const int passes = __builtin_ctz((unsigned)L);
   for (long long t0 = 0; t0 < za.n_traj; t0 += m) {
     const long long mm = std::min<long long>(m, za.n_traj - t0);
-    zimm_pack_kernel<PHYS><<<(unsigned)((3 * mm * L + 255) / 256), 256, 0, g.st>>>(za, L, t0, mm, g.zf_a.p);
-    CK(cudaGetLastError());
-    double2 *x = g.zf_a.p, *y = g.zf_b.p;
-    for (long long s = 1; s < L; s *= 2) {
-      stockham_batch_kernel<<<(unsigned)((3 * mm * (L / 2) + 255) / 256), 256, 0, g.st>>>(x, y, L, s, 3 * mm);
-      std::swap(x, y);
-    }
-    zimm_cross_kernel<<<(unsigned)((mm * L + 255) / 256), 256, 0, g.st>>>(x, L, mm, y);
-    CK(cudaGetLastError());
-    std::swap(x, y);
-    for (long long s = 1; s < L; s *= 2) {
-      stockham_batch_kernel<<<(unsigned)((mm * (L / 2) + 255) / 256), 256, 0, g.st>>>(x, y, L, s, mm);
-      std::swap(x, y);
-    }
+    // the first transform ends in x (fft_run: by the parity of its passes); the second one
+    // reads x and ends in y, its first pass writing the other workspace
+    double2 *x = (passes & 1) ? g.zf_a.p : g.zf_b.p, *y = g.zf_b.p, *o = (passes & 1) ? g.zf_b.p : g.zf_a.p;
+    CK(fft_run(ZimmPack<PHYS>{za, t0}, FftTo{x, logL}, logL, 3 * mm, g.zf_a.p, g.zf_b.p, g.st));
+    CK(fft_run(ZimmCross{x, logL}, FftTo{y, logL}, logL, mm, o, x, g.st));
     const dim3 agrid((unsigned)((N + 255) / 256), (unsigned)((mm + 255) / 256));
-    zimm_accum_kernel<<<agrid, 256, 0, g.st>>>(x, L, N, mm, za.traj_base + t0, za.traj_per_iter, za.w / L, za.crln);
+    zimm_accum_kernel<<<agrid, 256, 0, g.st>>>(y, L, N, mm, za.traj_base + t0, za.traj_per_iter, za.w / L, za.crln);
     CK(cudaGetLastError());
-    g_launches += 3 + 2 * (unsigned long long)passes;
+    g_launches += 1 + 2 * (unsigned long long)passes;
   }
+  return HH_OK;
+}
+
+// adds the spectra of a chunk of trajectories to g.pm_sf
+template <typename PHYS>
+int prmu_spectra(const PrmuPackArgs &pa, int logN, int L) {
+  const PrmuPack<PHYS> in{pa};
+  const long long pairs = (pa.n_traj + 1) / 2;
+  int rows;
+  if (logN >= FFT_MIN_LOG_TILE && logN <= FFT_MAX_LOG_TILE) {
+    const size_t smem = fft_smem(logN) + (size_t)L * sizeof(double);
+    auto k = prmu_spectrum_kernel<PHYS>;
+    if (smem > 48 * 1024) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 1 << (logN - 3), smem));
+    rows = (int)std::min<long long>(pairs, (long long)std::max(1, per_sm) * g.num_sms);
+    CK(g.pm_part.ensure((size_t)rows * L));
+    k<<<rows, 1 << (logN - 3), smem, g.st>>>(in, logN, L, g.pm_part.p);
+    g_launches += 3;  // weights, spectra, reduction
+  } else {
+    const long long B = 3 * pairs;
+    const int np = fft_passes(logN), gx = (L + 255) / 256;
+    double2 *out = (np & 1) && np > 1 ? g.pm_a.p : g.pm_b.p;
+    CK(fft_run(in, FftTo{out, logN}, logN, B, g.pm_a.p, g.pm_b.p, g.st));
+    rows = (int)std::min<long long>(B, std::max(1, 8 * g.num_sms / gx));
+    CK(g.pm_part.ensure((size_t)rows * L));
+    prmu_accum_kernel<<<dim3(gx, rows), 256, 0, g.st>>>(out, B, 1ll << logN, L, g.pm_part.p);
+    g_launches += 3 + (unsigned long long)np;  // weights, passes, accumulate, reduction
+  }
+  CK(cudaGetLastError());
+  prmu_reduce_kernel<<<(L + 31) / 32, 256, 0, g.st>>>(g.pm_part.p, rows, L, g.pm_sf.p);
+  CK(cudaGetLastError());
   return HH_OK;
 }
 
@@ -1970,13 +2008,18 @@ int hh_cuda_prmu(const hh_calc_params *p, double T, double R0, double approx_fre
   }
   const int stride = (int)N + 1;
   const size_t ps = (precision_mode == HH_PRECISION_MIXED) ? sizeof(float) : sizeof(double);
-  const size_t per_traj = (size_t)stride * 4 * ps + 2 * 2 * N * sizeof(double2) + 4 * sizeof(int);
+  const int logN = __builtin_ctzll((unsigned long long)N);
+  const bool fused = logN >= FFT_MIN_LOG_TILE && logN <= FFT_MAX_LOG_TILE;
+  const size_t per_traj = (size_t)stride * 4 * ps + (fused ? 0 : 2 * 2 * N * sizeof(double2)) + 4 * sizeof(int);
   const uint64_t chunk = std::min<uint64_t>(n_traj, std::max<uint64_t>(1, CH4_RECORD_BUDGET / per_traj));
   CK(g.rec_mu.ensure((size_t)chunk * stride * 4 * ps));
   CK(g.rec_len.ensure(2 * chunk));
   CK(g.rec_status.ensure(2 * chunk));
-  CK(g.pm_a.ensure(2 * chunk * N));
-  CK(g.pm_b.ensure(2 * chunk * N));
+  if (!fused) {  // three series per pair of trajectories
+    CK(g.pm_a.ensure(3 * ((chunk + 1) / 2) * N));
+    CK(g.pm_b.ensure(3 * ((chunk + 1) / 2) * N));
+  }
+  CK(g.pm_w.ensure(chunk));
   CK(g.pm_sf.ensure(L));
   CK(g.counters.ensure(16));
   CK(g.status_hist.ensure(2 * HH_ST_COUNT));
@@ -2022,23 +2065,12 @@ int hh_cuda_prmu(const hh_calc_params *p, double T, double R0, double approx_fre
     pa.stride = stride;
     pa.allow_trunc = allow_truncating ? 1 : 0;
     pa.coeff = sf_coeff / g.mu;
-    pa.z = g.pm_a.p;
+    pa.w = g.pm_w.p;
     pa.counted = g.rec_nfail.p;
-    const long long tot = (long long)nc * (long long)N;
-    if (precision_mode == HH_PRECISION_MIXED)
-      prmu_pack_kernel<float><<<(unsigned)((tot + 255) / 256), 256, 0, g.st>>>(pa);
-    else
-      prmu_pack_kernel<double><<<(unsigned)((tot + 255) / 256), 256, 0, g.st>>>(pa);
+    prmu_weight_kernel<<<(unsigned)((nc + 255) / 256), 256, 0, g.st>>>(pa);
     CK(cudaGetLastError());
-    const long long B = 2 * (long long)nc;
-    double2 *x = g.pm_a.p, *y = g.pm_b.p;
-    for (long long s = 1; s < (long long)N; s *= 2) {
-      stockham_batch_kernel<<<(unsigned)((B * ((long long)N / 2) + 255) / 256), 256, 0, g.st>>>(x, y, (long long)N, s, B);
-      std::swap(x, y);
-    }
-    prmu_accum_kernel<<<(unsigned)((L + 255) / 256), 256, 0, g.st>>>(x, B, (int)N, (int)L, g.pm_sf.p);
-    CK(cudaGetLastError());
-    g_launches += 2 + (unsigned long long)__builtin_ctzll((unsigned long long)N);  // pack, accumulate, passes
+    rc = precision_mode == HH_PRECISION_MIXED ? prmu_spectra<float>(pa, logN, (int)L) : prmu_spectra<double>(pa, logN, (int)L);
+    if (rc) return rc;
   }
   CK(cudaEventRecord(g.ev[3], g.st));
   unsigned long long counted = 0;
@@ -2321,60 +2353,74 @@ int hh_cuda_vegas(const hh_calc_params *p, int integrand, double T, uint64_t nit
   return HH_OK;
 }
 
-// the transform's kernels on g.st: pack, log2(2N) Stockham passes, finish
-void idct_enqueue(size_t N, double dt) {
-  const long long L = 2 * (long long)N;
-  const int tb = 256;
-  idct_pack_kernel<<<(unsigned)((L + tb - 1) / tb), tb, 0, g.st>>>(g.f_cf.p, (long long)N, dt, g.f_a.p);
-  idct_pack2_kernel<<<(unsigned)((N + tb - 1) / tb), tb, 0, g.st>>>(g.f_cf.p, (long long)N, g.f_a.p);
-  double2 *x = g.f_a.p, *y = g.f_b.p;
-  for (long long s = 1; s < L; s *= 2) {
-    stockham_pass_kernel<<<(unsigned)((L / 2 + tb - 1) / tb), tb, 0, g.st>>>(x, y, L, s);
-    std::swap(x, y);
-  }
-  idct_finish_kernel<<<(unsigned)((N + tb - 1) / tb), tb, 0, g.st>>>(x, (long long)N, dt, g.f_nu.p,
-                                                                      g.f_sf.p);
-}
+// page-locked staging of the CF -> SF transform, up to IDCT_PIN_MAX samples (8 MB each way,
+// kept until shutdown); a longer C(t), or one for which there is no page-locked memory, is
+// copied from and to the caller's.  What is left of a call is the host's reading and writing
+// of the caller's arrays (65,536 samples: 51 us of 140 are the read of the device's output).
+// 65,536 samples: 0.36 ms with 21 kernels and four copies of pageable memory -> 0.17 ms;
+// 2,048: 38 us with the two copies, 35 without
+constexpr size_t IDCT_PIN_MAX = size_t(1) << 20;
 
 int hh_cuda_idct_cf_to_sf(double *cf, size_t N, double dt, double *nu, double *sf) {
   if (!g.init) return HH_E_NOT_INITIALIZED;
   if (!cf || !nu || !sf || !(dt > 0)) return HH_E_INVALID_ARGUMENT;
   if (N == 0 || (N & (N - 1))) return HH_E_NOT_POWER_OF_TWO;
-  for (size_t i = 0; i < N; ++i)
-    if (cf[i] != cf[i]) return HH_E_INVALID_ARGUMENT;  // the reference exits on NaN input
   CK(cudaSetDevice(g.device));
-  long long L = 2 * (long long)N;
-  CK(g.f_cf.ensure(N));
-  CK(g.f_nu.ensure(N));
-  CK(g.f_sf.ensure(N));
-  CK(g.f_a.ensure(L));
-  CK(g.f_b.ensure(L));
-  // the ~log2(2N) + 3 small kernels are launch-bound: they are captured once per
-  // (N, dt, buffers) into a CUDA graph and replayed
-  const void *bufs[5] = {g.f_cf.p, g.f_nu.p, g.f_sf.p, g.f_a.p, g.f_b.p};
-  bool same = g.idct_exec && g.idct_N == N && g.idct_dt == dt;
-  for (int i = 0; i < 5; ++i) same = same && (g.idct_bufs[i] == bufs[i]);
-  if (!same) {
-    if (g.idct_exec) cudaGraphExecDestroy(g.idct_exec);
-    g.idct_exec = nullptr;
-    cudaGraph_t graph = nullptr;
-    CK(cudaStreamBeginCapture(g.st, cudaStreamCaptureModeThreadLocal));
-    idct_enqueue(N, dt);
-    CK(cudaStreamEndCapture(g.st, &graph));
-    const cudaError_t e = cudaGraphInstantiate(&g.idct_exec, graph, 0);
-    cudaGraphDestroy(graph);
-    CK(e);
-    g.idct_N = N;
-    g.idct_dt = dt;
-    for (int i = 0; i < 5; ++i) g.idct_bufs[i] = bufs[i];
+  bool pin = N <= IDCT_PIN_MAX;
+  if (pin && g.f_pin.ensure(2 * N) != cudaSuccess) {
+    cudaGetLastError();  // no page-locked memory to be had
+    pin = false;
   }
-  (void)L;
-  CK(cudaMemcpyAsync(g.f_cf.p, cf, N * sizeof(double), cudaMemcpyHostToDevice, g.st));
-  CK(cudaGraphLaunch(g.idct_exec, g.st));
-  CK(cudaMemcpyAsync(nu, g.f_nu.p, N * sizeof(double), cudaMemcpyDeviceToHost, g.st));
-  CK(cudaMemcpyAsync(sf, g.f_sf.p, N * sizeof(double), cudaMemcpyDeviceToHost, g.st));
-  CK(cudaMemcpyAsync(cf, g.f_cf.p, N * sizeof(double), cudaMemcpyDeviceToHost, g.st));
-  CK(cudaStreamSynchronize(g.st));
+  double *in = pin ? g.f_pin.p : cf, *out = pin ? g.f_pin.p + N : sf;
+  // a block at a time, so that the check and the copy are vector code
+  for (size_t i0 = 0; i0 < N; i0 += 512) {
+    const size_t i1 = std::min(N, i0 + 512);
+    int bad = 0;
+    for (size_t i = i0; i < i1; ++i) bad |= cf[i] != cf[i];
+    if (bad) return HH_E_INVALID_ARGUMENT;  // the reference exits on NaN input
+    if (pin) memcpy(in + i0, cf + i0, (i1 - i0) * sizeof(double));
+  }
+  const long long L = 2 * (long long)N;
+  const int logL = __builtin_ctzll((unsigned long long)L), np = fft_passes(logL);
+  if (!pin || np > 1) {
+    CK(g.f_cf.ensure(N));
+    CK(g.f_sf.ensure(N));
+  }
+  if (np > 1) CK(g.f_a.ensure(L));
+  if (np > 2) CK(g.f_b.ensure(L));
+  const double Xscale = 1.0 / HH_LIGHTSPEED_CM / HH_ATU / 2.0 / HH_PI;
+  const double Yscale = HH_ATU * HH_ADIPMOMU * HH_ADIPMOMU / (4.0 * HH_PI * HH_EPSILON0);
+  const double tmax = double(N) * dt;
+  // one pass reads and writes the staging itself: two copies less
+  const bool direct = pin && np == 1;
+  if (!direct) CK(cudaMemcpyAsync(g.f_cf.p, in, N * sizeof(double), cudaMemcpyHostToDevice, g.st));
+  CK(fft_run(IdctPack{direct ? in : g.f_cf.p, (long long)N},
+             IdctFinish{direct ? out : g.f_sf.p, (long long)N, tmax / HH_PI * Yscale}, logL, 1, g.f_a.p, g.f_b.p,
+             g.st));
+  if (!direct) CK(cudaMemcpyAsync(out, g.f_sf.p, N * sizeof(double), cudaMemcpyDeviceToHost, g.st));
+  // meanwhile the grid, the first touch of sf's pages, and, in place on the caller's C(t)
+  // like the reference, the apodization (from the staged copy; else once C(t) is read)
+  const double nu1 = HH_PI / tmax * Xscale, rN = 1.0 / double(N);
+  auto blocks = [&](auto &&f) {  // f(first, count): loops over a 32-bit index are vector code
+    for (size_t i0 = 0; i0 < N; i0 += 512) f(i0, (int)std::min<size_t>(512, N - i0));
+  };
+  auto apodize = [&](const double *src) {
+    blocks([&](size_t i0, int n) {
+      const double k0 = double((long long)i0);
+      for (int j = 0; j < n; ++j) cf[i0 + j] = src[i0 + j] * connes(k0 + j, rN);
+    });
+  };
+  blocks([&](size_t i0, int n) {
+    const double k0 = double((long long)i0);
+    for (int j = 0; j < n; ++j) nu[i0 + j] = (k0 + j) * nu1;
+    if (pin) sf[i0] = 0.0;
+  });
+  if (pin) apodize(in);
+  const cudaError_t e = cudaStreamSynchronize(g.st);
+  if (e != cudaSuccess && pin) memcpy(cf, in, N * sizeof(double));
+  CK(e);
+  if (pin) memcpy(sf, out, N * sizeof(double));
+  else apodize(cf);
   return HH_OK;
 }
 
@@ -2676,6 +2722,8 @@ void hh_cuda_shutdown(void) {
   g.pm_a.release();
   g.pm_b.release();
   g.pm_sf.release();
+  g.pm_w.release();
+  g.pm_part.release();
   g.m0_partials.release();
   g.m0_out.release();
   g.tune_crln.release();
@@ -2684,11 +2732,10 @@ void hh_cuda_shutdown(void) {
   g.vg_sums.release();
   g.vg_hist.release();
   g.f_cf.release();
-  g.f_nu.release();
   g.f_sf.release();
   g.f_a.release();
   g.f_b.release();
-  if (g.idct_exec) cudaGraphExecDestroy(g.idct_exec);
+  g.f_pin.release();
   if (g.d_tab) cudaFree(g.d_tab);
   if (g.d_n2ar_fold) cudaFree(g.d_n2ar_fold);
   if (g.d_n2ar_pes_d) cudaFree(g.d_n2ar_pes_d);

@@ -531,51 +531,48 @@ __device__ __forceinline__ void zimm_d(const PHYS *sv, int N, int lf, int lb, in
 // a = d[0..N-1] and b = d[0..2N-2], zero-padded to L >= 2N - 1 (a power of two),
 // C(s) = sum_c a[c] . b[c+s] is the circular cross-correlation of a and b for
 // s < N (no term wraps), so with the transform F[k] = sum_j x_j e^{+2 pi i jk/L} of
-// stockham_batch_kernel:
+// hh_fft.cuh:
 //   C(s) = (1/L) Re sum_k conj(P_k) e^{+2 pi i sk/L},  P_k = sum_comp conj(A_k) B_k.
-//   1. zimm_pack: per trajectory and component the complex series a_j + i b_j
-//      (zero for a dropped trajectory);
-//   2. log2 L Stockham passes over 3 series per trajectory;
-//   3. zimm_cross: A_k = (Z_k + conj Z_{L-k}) / 2, B_k = (Z_k - conj Z_{L-k}) / 2i, and
-//      conj(P_k) per trajectory;
-//   4. log2 L passes over one series per trajectory;
-//   5. zimm_accum: C(s) += w Re(.)/L into each trajectory's C(t) slice.
+//   1. the transform of three series per trajectory, read through ZimmPack: component by
+//      component a_j + i b_j (zero for a dropped trajectory);
+//   2. the transform of one series per trajectory, read through ZimmCross:
+//      A_k = (Z_k + conj Z_{L-k}) / 2, B_k = (Z_k - conj Z_{L-k}) / 2i, and conj(P_k);
+//   3. zimm_accum: C(s) += w Re(.)/L into each trajectory's C(t) slice.
 // All transforms are FP64 on both precision paths.
-template <typename PHYS>
-__global__ void __launch_bounds__(256) zimm_pack_kernel(ZimmArgs a, int L, long long t0, long long m, double2 *z) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= 3 * m * L) return;
-  const long long sr = i / L;
-  const int j = (int)(i - sr * L);
-  const long long t = t0 + sr / 3;
-  const int comp = (int)(sr % 3);
-  double av = 0.0, bv = 0.0;
-  if (!a.failed[t] && j <= 2 * a.N - 2) {
-    const PHYS *sv = static_cast<const PHYS *>(a.series) + (size_t)t * a.stride * 4;
-    double d[3];
-    zimm_d(sv, a.N, a.len[2 * t], a.len[2 * t + 1], j, d);
-    bv = d[comp];
-    if (j < a.N) av = d[comp];
+template <typename PHYS> struct ZimmPack {
+  ZimmArgs a;
+  long long t0;
+  __device__ double2 operator()(long long sr, long long j) const {
+    const long long t = t0 + sr / 3;
+    const int comp = (int)(sr % 3);
+    double av = 0.0, bv = 0.0;
+    if (!a.failed[t] && j <= 2 * a.N - 2) {
+      const PHYS *sv = static_cast<const PHYS *>(a.series) + (size_t)t * a.stride * 4;
+      double d[3];
+      zimm_d(sv, a.N, a.len[2 * t], a.len[2 * t + 1], (int)j, d);
+      bv = comp == 0 ? d[0] : comp == 1 ? d[1] : d[2];
+      if (j < a.N) av = bv;
+    }
+    return make_double2(av, bv);
   }
-  z[i] = make_double2(av, bv);
-}
+};
 
-__global__ void __launch_bounds__(256) zimm_cross_kernel(const double2 *Z, int L, long long m, double2 *pc) {
-  const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (i >= m * L) return;
-  const long long t = i / L;
-  const int k = (int)(i - t * L);
-  const int kr = (L - k) & (L - 1);
-  double pr = 0.0, pi = 0.0;
-  for (int c = 0; c < 3; ++c) {
-    const double2 zk = Z[(3 * t + c) * L + k], zm = Z[(3 * t + c) * L + kr];
-    const double ar = 0.5 * (zk.x + zm.x), ai = 0.5 * (zk.y - zm.y);
-    const double br = 0.5 * (zk.y + zm.y), bi = -0.5 * (zk.x - zm.x);
-    pr += ar * br + ai * bi;  // conj(A) B
-    pi += ar * bi - ai * br;
+struct ZimmCross {
+  const double2 *Z;
+  int logL;
+  __device__ double2 operator()(long long t, long long k) const {
+    const long long L = 1ll << logL, kr = (L - k) & (L - 1);
+    double pr = 0.0, pi = 0.0;
+    for (int c = 0; c < 3; ++c) {
+      const double2 zk = Z[((3 * t + c) << logL) + k], zm = Z[((3 * t + c) << logL) + kr];
+      const double ar = 0.5 * (zk.x + zm.x), ai = 0.5 * (zk.y - zm.y);
+      const double br = 0.5 * (zk.y + zm.y), bi = -0.5 * (zk.x - zm.x);
+      pr += ar * br + ai * bi;  // conj(A) B
+      pi += ar * bi - ai * br;
+    }
+    return make_double2(pr, -pi);
   }
-  pc[i] = make_double2(pr, -pi);
-}
+};
 
 // grid: x over s < N, y over groups of 256 trajectories
 __global__ void __launch_bounds__(256) zimm_accum_kernel(const double2 *R, int L, int N, long long m,
