@@ -1242,7 +1242,7 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       tr_launch = std::min<uint64_t>(n, it_launch * per_iter);
       if (!mixed) tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
       items_launch = 2 * tr_launch;
-      cap = (unsigned long long)(est * double(items_launch)) + 4096ull;
+      cap = (unsigned long long)(est * double(items_launch)) + 16384ull;  // and the solo warps' unused ones
       if (getenv("HH_DEFER_TRACE"))
         fprintf(stderr, "[defer] attempt %d est %.3f items %llu cap %llu (buffer %llu) launches of %llu trajectories, "
                 "budget %.2f GB, free %.2f GB\n", attempt, est, (unsigned long long)items_launch, cap,
@@ -1377,6 +1377,7 @@ int run_trajectories(const hh_calc_params *p, const double *d_ic, uint64_t n, ui
   P.mu = g.mu;
   P.II = g.II;
   P.dt = p->sampling_time;
+  P.inv_dt = 1.0 / P.dt;
   P.N = (int)N;
   P.Rcut = p->Rcut;
   double tol = (precision == HH_PRECISION_MIXED)
@@ -1988,6 +1989,7 @@ int hh_cuda_prmu(const hh_calc_params *p, double T, double R0, double approx_fre
   P.mu = g.mu;
   P.II = g.II;
   P.dt = dt;
+  P.inv_dt = 1.0 / dt;
   P.N = (int)N + 1;
   P.Rcut = R0;
   const double tol = (precision_mode == HH_PRECISION_MIXED)

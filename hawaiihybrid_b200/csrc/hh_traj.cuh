@@ -38,7 +38,7 @@ enum { SYS_HEAR = 1, SYS_CO2AR = 2, SYS_N2AR = 3, SYS_CH4CO2 = 4 };
 
 struct TrajParams {
   double mu, II;
-  double dt;
+  double dt, inv_dt;          // sampling interval; its reciprocal, for first guesses only
   int N;
   double Rcut;
   double rtol, atol;
@@ -361,9 +361,22 @@ template <typename T> __device__ __forceinline__ void legendre10_rn(T x, T (&P)[
   }
 }
 
+constexpr int SOLO_MAX_WARPS = 8;  // warps per block of the solo kernels
+
+// A warp's exchange of the radial functions and (FP64) of the stage point: a store and a few
+// broadcast loads where each shuffled double takes two instructions (44 of the 320 of a
+// CO2-Ar right-hand side were shuffles, which it issues one per 3.9 cycles)
+template <typename T> struct Co2arRhsScratch {
+  struct alignas(2 * sizeof(T)) Pair {
+    T c, dc;
+  };
+  Pair rad[CO2AR_NL];
+  alignas(16) T y[12];
+};
+
 template <typename T, bool EXP>
-__device__ __forceinline__ PesGrad<T> co2ar_pes_grad_lanes(const Co2arTables<T> *tb, T R, T iR, T x, int i, int li) {
-  constexpr unsigned FULL = 0xffffffffu;
+__device__ __forceinline__ PesGrad<T> co2ar_pes_grad_lanes(const Co2arTables<T> *tb, T R, T iR, T x, int i, int li,
+                                                           Co2arRhsScratch<T> &scr) {
   T P[11], dP[11], c, dc;
   const T t = R - tb->rlo[i];
   if constexpr (sizeof(T) == 4) {
@@ -397,13 +410,15 @@ __device__ __forceinline__ PesGrad<T> co2ar_pes_grad_lanes(const Co2arTables<T> 
     }
     radial<T>(row, R, t, iR, EXP ? 3 : 1, c, dc);
   }
+  if ((threadIdx.x & 31) < CO2AR_NL) scr.rad[li] = {c, dc};
+  __syncwarp();
   legendre10_rn(x, P, dP);
   T aR = T(0), ax = T(0);
 #pragma unroll
   for (int l = 0; l < CO2AR_NL; ++l) {
-    const T cl = __shfl_sync(FULL, c, l), dcl = __shfl_sync(FULL, dc, l);
-    aR = n2_fma(P[2 * l], dcl, aR);
-    ax = n2_fma(dP[2 * l], cl, ax);
+    const typename Co2arRhsScratch<T>::Pair v = scr.rad[l];
+    aR = n2_fma(P[2 * l], v.dc, aR);
+    ax = n2_fma(dP[2 * l], v.c, ax);
   }
   // (rounded here: the caller's expressions must not fuse with these products)
   const T sc = T(1.0 / HH_HTOCM);
@@ -443,24 +458,47 @@ __device__ __noinline__ T co2ar_rhs_lane(const Co2arTables<T> *tb, T ysc, T im, 
   constexpr unsigned FULL = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const T rb = tb->rbound[lane < CO2AR_NINT - 1 ? lane : CO2AR_NINT - 2];
-  T r[3], u[3];
+  __shared__ Co2arRhsScratch<T> scratch[SOLO_MAX_WARPS];
+  Co2arRhsScratch<T> &scr = scratch[threadIdx.x >> 5];
+  T r[3], u[3], v1, v2, v3, v4;
+  if constexpr (sizeof(T) == 8) {
+    // (the barrier below and the one behind the radial functions keep two calls apart)
+    if (lane < 12) scr.y[lane] = ysc;
+    __syncwarp();
+    const double2 r01 = *reinterpret_cast<const double2 *>(&scr.y[0]), u01 = *reinterpret_cast<const double2 *>(&scr.y[6]);
+    r[0] = r01.x;
+    r[1] = r01.y;
+    r[2] = scr.y[2];
+    u[0] = u01.x;
+    u[1] = u01.y;
+    u[2] = scr.y[8];
+    v1 = scr.y[L.s1];
+    v2 = scr.y[L.s2];
+    v3 = scr.y[L.s3];
+    v4 = scr.y[L.s4];
+  } else {
 #pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    r[i] = __shfl_sync(FULL, ysc, i);
-    u[i] = __shfl_sync(FULL, ysc, 6 + i);
+    for (int i = 0; i < 3; ++i) {
+      r[i] = __shfl_sync(FULL, ysc, i);
+      u[i] = __shfl_sync(FULL, ysc, 6 + i);
+    }
+    v1 = __shfl_sync(FULL, ysc, L.s1);
+    v2 = __shfl_sync(FULL, ysc, L.s2);
+    v3 = __shfl_sync(FULL, ysc, L.s3);
+    v4 = __shfl_sync(FULL, ysc, L.s4);
   }
-  const T v1 = __shfl_sync(FULL, ysc, L.s1), v2 = __shfl_sync(FULL, ysc, L.s2);
-  const T v3 = __shfl_sync(FULL, ysc, L.s3), v4 = __shfl_sync(FULL, ysc, L.s4);
   T R2 = r[0] * r[0] + r[1] * r[1] + r[2] * r[2];
-  T iR = inv_sqrt(R2);
+  const T U2 = u[0] * u[0] + u[1] * u[1] + u[2] * u[2];
+  // the two roots side by side
+  const T root = inv_sqrt(lane & 1 ? U2 : R2);
+  const T iR = __shfl_sync(FULL, root, 0), iu = __shfl_sync(FULL, root, 1);
   T R = R2 * iR;
-  T iu = inv_sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
   T rh[3] = {r[0] * iR, r[1] * iR, r[2] * iR};
   T uh[3] = {u[0] * iu, u[1] * iu, u[2] * iu};
   T x = rh[0] * uh[0] + rh[1] * uh[1] + rh[2] * uh[2];
   const int i = __popc(__ballot_sync(FULL, lane < CO2AR_NINT - 1 && R >= rb));
-  const PesGrad<T> G = tb->fpes[i] & 2 ? co2ar_pes_grad_lanes<T, true>(tb, R, iR, x, i, L.li)
-                                       : co2ar_pes_grad_lanes<T, false>(tb, R, iR, x, i, L.li);
+  const PesGrad<T> G = tb->fpes[i] & 2 ? co2ar_pes_grad_lanes<T, true>(tb, R, iR, x, i, L.li, scr)
+                                       : co2ar_pes_grad_lanes<T, false>(tb, R, iR, x, i, L.li, scr);
   const T VR = G.VR, Vx = G.Vx;
   T a = VR - Vx * x * iR;  // dV/dr = a r^ + (Vx/R) u^
   T b = Vx * iR;
@@ -894,8 +932,11 @@ __device__ __forceinline__ void dense_stages(const Sys &sys, STG (&K)[16][Sys::N
 // right-looking: once K_j is known, a_{S,j} K_j goes into the sums of the later stages, of
 // the solution, the error estimates and the dense output.  Each sum takes its terms in the
 // order j = 0, 1, .. of the per-lane code, but only its last term waits for K_{S-1}.
-// Measured, solo launch: He-Ar 10,240 x 65,536 FP64 80 -> 58 ms (12.0 -> 9.0 us per step),
-// CO2-Ar 102,400 x 32,768 FP64 229 -> 134 ms, PR_MU 4,096 x 4,096 FP64 26.3 -> 16.8 ms.  A
+// Measured, solo launch: He-Ar 10,240 x 65,536 FP64 80 -> 57 ms (12.0 -> 8.7 us per step),
+// CO2-Ar 102,400 x 32,768 FP64 229 -> 107 ms, PR_MU 4,096 x 4,096 FP64 26.3 -> 15.9 ms.  Of
+// the 18,500 cycles of a CO2-Ar FP64 step the 12 stages of the attempt are 13,400 and the
+// three of the dense output 3,200; square roots, divisions and an atomic's round trip
+// between them were 3,500 more.  A
 // rolled stage loop with the right-hand side inlined took 28 % (CO2-Ar) more per step.
 // rows: A[i] the sum of stage i + 1 (A[11]: the solution), X the stages 13..15, D the
 // dense-output rows
@@ -935,7 +976,7 @@ __device__ __forceinline__ void cp_stage(const Sys &sys, SysSums<Sys, STG> &s, S
 
 template <class Sys, typename STG>
 __device__ __forceinline__ double step_attempt_cp(const Sys &sys, const TrajParams &P, STG k0, double y, double h,
-                                                  double &y_new, STG &k12, SysSums<Sys, STG> &s) {
+                                                  double &y_new, STG &k12, SysSums<Sys, STG> &s, double &inv_h) {
   constexpr int N = Sys::N;
   const int lane = threadIdx.x & 31;
   const int c = lane < N ? lane : N - 1;
@@ -959,7 +1000,10 @@ __device__ __forceinline__ double step_attempt_cp(const Sys &sys, const TrajPara
   solo_add<12>(s, k12);
   double sc = P.atol + fmax(fabs(y), fabs(y_new)) * P.rtol;
   if (sizeof(STG) == 4) sc += fabs(h) * P.noise_floor * double(s.m5);
-  const double isc = 1.0 / sc;
+  // one division for the components' scales and, on the last lane, the dense output's 1 / h
+  static_assert(N < 32, "lane 31 holds no component");
+  const double isc = 1.0 / (lane == 31 ? h : sc);
+  inv_h = __shfl_sync(0xffffffffu, isc, 31);
   const double q5 = double(s.a5) * isc, q3 = double(s.a3) * isc;
   double e5 = 0.0, e3 = 0.0;
 #pragma unroll
@@ -1014,25 +1058,45 @@ __device__ __forceinline__ void dense_eval(const double *y_old, const STG (&F)[7
 // Whether |r(x)| of the dense-output polynomial y = y_old + F0 x + F1 x(1-x) + F2 x^2(1-x)
 // + ... + F6 x^4(1-x)^3 stays below Rcut on [0, 1], with a margin for the evaluation in
 // the stage precision: |r(x)| <= max(|r_old|, |r_old + F0|) + sum_i c_i |F_i|, c_i the
-// maxima of its basis (|r_old + F0 x| is convex in x).  f(r, c): component c of F_r.
+// maxima of its basis (|r_old + F0 x| is convex in x).  |F_i| is bounded by its 1-norm and
+// the sum taken to the right-hand side, so that no square root is left (eight of them in a
+// chain were 1,900 of the 24,600 cycles of a CO2-Ar FP64 solo step); a step that the looser
+// bound misses has its samples tested one by one.  f(r, c): component c of F_r.
 template <typename FF>
 __device__ __forceinline__ bool dense_stays_inside(const FF &f, const double *q, double Rcut) {
   constexpr double cb[7] = {0.0, 0.25, 4.0 / 27.0, 1.0 / 16.0, 108.0 / 3125.0, 1.0 / 64.0, 6912.0 / 823543.0};
-  double ro2 = 0.0, rn2 = 0.0, f02 = 0.0, tail = 0.0;
+  double ro2 = 0.0, rn2 = 0.0, f0s = 0.0, tail = 0.0;
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double qo = q[c], f0 = f(0, c);
     ro2 += qo * qo;
     rn2 += (qo + f0) * (qo + f0);
-    f02 += f0 * f0;
+    f0s += fabs(f0);
   }
 #pragma unroll
-  for (int r = 1; r < 7; ++r) {
-    const double a0 = f(r, 0), a1 = f(r, 1), a2 = f(r, 2);
-    tail += cb[r] * sqrt(a0 * a0 + a1 * a1 + a2 * a2);
+  for (int r = 1; r < 7; ++r) tail += cb[r] * ((fabs(f(r, 0)) + fabs(f(r, 1))) + fabs(f(r, 2)));
+  const double lim = Rcut * (1.0 - 1e-12) - tail - 1e-5 * (f0s + tail);
+  return lim > 0.0 && ro2 < lim * lim && rn2 < lim * lim;
+}
+
+// the same with component c of r and of the F_r on lane c (c < 3)
+template <typename STG> __device__ __forceinline__ bool dense_stays_inside_cp(const STG (&F)[7], double q, double Rcut) {
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr double cb[7] = {0.0, 0.25, 4.0 / 27.0, 1.0 / 16.0, 108.0 / 3125.0, 1.0 / 64.0, 6912.0 / 823543.0};
+  const double f0 = double(F[0]), qn = q + f0;
+  double m = 1e-5 * fabs(f0);  // this component's share of tail and margin
+#pragma unroll
+  for (int r = 1; r < 7; ++r) m += (cb[r] * (1.0 + 1e-5)) * fabs(double(F[r]));
+  double ro2 = 0.0, rn2 = 0.0, ms = 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double a = __shfl_sync(FULL, q, c), b = __shfl_sync(FULL, qn, c);
+    ro2 += a * a;
+    rn2 += b * b;
+    ms += __shfl_sync(FULL, m, c);
   }
-  const double bound = fmax(sqrt(ro2), sqrt(rn2)) + tail;
-  return bound + 1e-5 * (sqrt(f02) + tail) + 1e-12 * bound < Rcut;
+  const double lim = Rcut * (1.0 - 1e-12) - ms;
+  return lim > 0.0 && ro2 < lim * lim && rn2 < lim * lim;
 }
 
 // Per-item set-up, out of line (once per half-trajectory): Cartesian initial
@@ -1259,7 +1323,11 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
   auto item_of = [&](unsigned idx) {
     return io.items ? io.items[idx] : (io.fwd_only ? 2 * (int)idx : (int)idx);
   };
-  unsigned long long ctx_slot = ~0ull;  // solo mode, deferred samples: lane 0's reserved context
+  // solo mode, deferred samples: the warp's reserved contexts (one atomic for CTX_BATCH; its
+  // round trip was 900 cycles of every step)
+  constexpr int CTX_BATCH = 8;
+  unsigned long long ctx_next = 0;
+  int ctx_left = 0;
   bool handing = false;  // bulk mode: this warp hands its open items to the solo kernel
   unsigned round = 0;
   int sync_round = 0;    // bulk mode: rounds since the last block barrier
@@ -1369,6 +1437,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
     bool accepted = false;
     bool landed = false;  // REQ: the step ends exactly at sample time k dt
     double h_taken = 0.0;
+    double inv_h = 0.0;  // solo mode: 1 / h_att
     if (active) {
       // 10 * spacing of doubles above t (t >= 0 and finite)
       const double min_step = 10.0 * (__longlong_as_double(__double_as_longlong(t) + 1) - t);
@@ -1386,7 +1455,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
       } else {
         double err;
         if constexpr (Sys::SOLO)
-          err = step_attempt_cp<Sys, STG>(sys, P, K[0][0], y[0], h_att, y_new[0], K[12][0], dsum);
+          err = step_attempt_cp<Sys, STG>(sys, P, K[0][0], y[0], h_att, y_new[0], K[12][0], dsum, inv_h);
         else
           err = step_attempt<Sys, STG>(sys, P, K, y, h_att, y_new);
         nrhs += 12;
@@ -1420,7 +1489,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
     // the last sample time the step passed
     auto last_k = [&]() {
       const double t_new = t + h_taken;
-      int kl = (int)fmin(floor(t_new / dt), double(P.N - 1));
+      int kl = (int)fmin(floor(t_new * P.inv_dt), double(P.N - 1));  // a guess, made exact below
       while (kl + 1 <= P.N - 1 && double(kl + 1) * dt <= t_new) ++kl;
       while (kl > k && double(kl) * dt > t_new) --kl;
       return REQ && landed ? k : kl;
@@ -1457,20 +1526,21 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
         constexpr int NQ = Sys::NQ;
         STG *sF = &ws->F[0][0][0];       // [7][NQ]
         double *sq = &ws->qold[0][0];    // [NQ]
+        // (qidx skips one block of momenta at most: component 3 on is lane - (qidx(3) - 3))
+        constexpr int SKIP = NQ > 3 ? Sys::qidx(NQ - 1) - (NQ - 1) : 0;
+        const int cq = lane < 3 ? lane : lane - SKIP;
+        if (lane < 3 || (lane >= 3 + SKIP && lane < NQ + SKIP)) {
 #pragma unroll
-        for (int cq = 0; cq < NQ; ++cq)
-          if (Sys::qidx(cq) == lane) {
-#pragma unroll
-            for (int r = 0; r < 7; ++r) sF[r * NQ + cq] = Fc[r];
-            sq[cq] = y[0];
-          }
-        const int cnt = last_k() - k + 1;
-        const double inv_h = 1.0 / h_taken;
+          for (int r = 0; r < 7; ++r) sF[r * NQ + cq] = Fc[r];
+          sq[cq] = y[0];
+        }
+        // lane i: does the step pass sample k + i?
+        int cnt = __popc(__ballot_sync(FULL, k + lane < P.N && double(k + lane) * dt <= t + h_taken));
+        if (cnt == 32 || REQ) cnt = last_k() - k + 1;
         __syncwarp();
         bool safe = false;  // deferred samples: no sample of the step passes R > Rcut
         if constexpr (!Sys::RECORDS)
-          if (defer && cnt > 0)
-            safe = dense_stays_inside([&](int r, int c) { return double(sF[r * NQ + c]); }, sq, P.Rcut);
+          if (defer && cnt > 0) safe = dense_stays_inside_cp(Fc, y[0], P.Rcut);
         unsigned cut = 0xffffffffu;
         PHYS tail = curr;
         if (safe) {
@@ -1531,7 +1601,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
               } else if (nan) code = (unsigned(j) << 3) | 1u;
               else if (item == P.inject_item && kk == P.inject_k) code = (unsigned(j) << 3) | 4u;
               else if (fabs(double(val)) > 1e100) code = (unsigned(j) << 3) | 2u;
-              else if (kk > 1 && fabs(double(val) / double(pv)) > 1e10) code = (unsigned(j) << 3) | 3u;
+              else if (kk > 1 && fabs(double(val)) > 1e10 * fabs(double(pv))) code = (unsigned(j) << 3) | 3u;
               else if (out) code = (unsigned(j + 1) << 3);  // stored, then the branch ends
             }
             cut = __reduce_min_sync(FULL, code);
@@ -1556,9 +1626,13 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
         const int nc = cut == 0xffffffffu ? cnt : min(cnt, int(cut >> 3));
         if constexpr (!Sys::RECORDS) {
           if (defer && nc > 0) {
-            // the context's slot was reserved a step ago, so the atomic's latency is hidden
-            if (lane == 0 && ctx_slot == ~0ull) ctx_slot = atomicAdd(io.ctx_count, 1ull);
-            const unsigned long long idx = __shfl_sync(FULL, ctx_slot, 0);
+            if (ctx_left == 0) {
+              if (lane == 0) ctx_next = atomicAdd(io.ctx_count, (unsigned long long)CTX_BATCH);
+              ctx_next = __shfl_sync(FULL, ctx_next, 0);
+              ctx_left = CTX_BATCH;
+            }
+            const unsigned long long idx = ctx_next++;
+            --ctx_left;
             if (idx < io.ctx_cap) {
               auto *cx = static_cast<SampleCtx<STG, NQ> *>(io.ctx) + idx;
               for (int e = lane; e < 7 * NQ; e += 32) (&cx->F[0][0])[e] = sF[e];
@@ -1574,7 +1648,6 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
             }
             // past the capacity the host repeats the call with a larger buffer
             last_ctx = (int)idx;
-            if (lane == 0) ctx_slot = atomicAdd(io.ctx_count, 1ull);
           }
         }
         if (nc > 0) {
@@ -1729,7 +1802,7 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
             else if (fabs(double(val)) > 1e100) code = (unsigned(j) << 3) | 2u;
             else {
               const PHYS pv = (j == ws->off[o]) ? ws->prev[o] : (jj == 0 ? ws->tail[o] : ws->res[jj - 1]);
-              if (kks[u] > 1 && fabs(double(val) / double(pv)) > 1e10) code = (unsigned(j) << 3) | 3u;
+              if (kks[u] > 1 && fabs(double(val)) > 1e10 * fabs(double(pv))) code = (unsigned(j) << 3) | 3u;
               else if (out_[u]) code = (unsigned(j + 1) << 3);  // stored, then the branch ends
             }
             if (code != 0xffffffffu) atomicMin(&ws->cut[o], code);
@@ -1933,9 +2006,9 @@ __device__ __forceinline__ void traj_body(const Sys &sys, const TrajParams &P, c
     }
   }
   if constexpr (Sys::SOLO && !Sys::RECORDS) {
-    // a reserved context that was not used holds no samples
-    if (defer && ctx_slot < io.ctx_cap) {
-      auto *cx = static_cast<SampleCtx<STG, Sys::NQ> *>(io.ctx) + ctx_slot;
+    // reserved contexts that were not used hold no samples
+    if (defer && lane < ctx_left && ctx_next + lane < io.ctx_cap) {
+      auto *cx = static_cast<SampleCtx<STG, Sys::NQ> *>(io.ctx) + ctx_next + lane;
       cx->item = 0;
       cx->k0 = 0;
       cx->n = 0;
@@ -1990,6 +2063,7 @@ template <int SYS, typename PHYS, typename STG, bool COMP, bool SOLO = false, in
           bool REQ = false>
 __global__ void __launch_bounds__(32 * WARPS, TRAJ_MIN_BLOCKS)
     traj_kernel(TrajParams P, TrajIO io, const Co2arTablesGlobal *gtab) {
+  static_assert(!SOLO || WARPS <= SOLO_MAX_WARPS, "scratch of the solo right-hand sides");
   static_assert(!REQ || SYS == SYS_CO2AR || SYS == SYS_N2AR, "requantization of a linear monomer");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   if constexpr (SYS == SYS_HEAR) {
