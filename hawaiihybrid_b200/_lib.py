@@ -190,9 +190,9 @@ def ch4co2_fold_shape() -> tuple[int, int]:
 
 
 def defer_samples(mode: int = -1) -> int:
-    """Placement of the mixed path's sample dipoles (hh_cuda_debug_set_defer): 0 in the
-    trajectory kernel, 1 CO2-Ar deferred to the sample kernels, 2 CO2-Ar and N2-Ar;
-    -1 only reads it.  Returns the mode before the call."""
+    """Placement of the sample dipoles (hh_cuda_debug_set_defer): 0 in the trajectory
+    kernel, 1 deferred to the sample kernels except in small mixed N2-Ar calls, 2 in all
+    CO2-Ar and N2-Ar calls; -1 only reads it.  Returns the mode before the call."""
     prev = C.c_int(0)
     check(load().hh_cuda_debug_set_defer(int(mode), C.byref(prev)))
     return prev.value

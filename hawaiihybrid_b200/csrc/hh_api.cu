@@ -665,20 +665,25 @@ int run_traj_dispatch(int precision, const TrajParams &P, const TrajIO &io) {
 // plain C(t) of the systems with a surface dipole; records, series, satellite
 // temperatures, PR_MU and a failure injection with a soft status keep in-kernel samples.
 // g_defer (hh_cuda_debug_set_defer; environment HH_DEFER_SAMPLES, default 1): 0 in-kernel
-// samples for every call; 1 deferred for CO2-Ar on both paths and for N2-Ar in FP64, whose
-// samples are the FP64 network (the mixed N2-Ar dipole is a table lookup, which gains
-// nothing: 365 against 368 ms per iteration); 2 also mixed N2-Ar.  In FP64 (ms per call,
-// samples in the kernel / deferred): CO2-Ar 102,400 x 32,768 222 / 172, its bulk launch
-// 88 / 41; N2-Ar 20,011 x 5,000 205 / 142, its bulk launch 145 / 82.
+// samples for every call; 1 deferred for CO2-Ar on both paths, for N2-Ar in FP64, whose
+// samples are the FP64 network, and for mixed N2-Ar calls of N2AR_DEFER_SAMPLES sample
+// times or more; 2 all of mixed N2-Ar.  Samples in the kernel / deferred, ms per call: FP64
+// CO2-Ar 102,400 x 32,768 222 / 172, its bulk launch 88 / 41; N2-Ar 20,011 x 5,000 205 / 142,
+// its bulk launch 145 / 82.  Mixed N2-Ar (a table lookup of 800 bytes per sample and lane):
+// 131,072 x 16,384 119 / 94, its bulk launch 74 / 35; 20,000 x 512 12.2 / 10.3; 64 x 16,384
+// 11.0 / 10.3; 500 x 512 3.26 / 3.28; 64 x 2,048 2.31 / 2.47, where the item starts and the
+// sample kernels' launches are not made up for.
+constexpr uint64_t N2AR_DEFER_SAMPLES = 1u << 19;
 int g_defer = [] {
   const char *e = getenv("HH_DEFER_SAMPLES");
   return e ? atoi(e) : 1;
 }();
-bool defer_eligible(int precision, const TrajParams &P, const TrajIO &io) {
+bool defer_eligible(int precision, const TrajParams &P, const TrajIO &io, uint64_t n) {
   // the CO2-Ar sample kernels evaluate dipole intervals without exponential terms
   const bool sys_ok = g.sys == SYS_CO2AR
                           ? g_defer >= 1 && !g_co2ar_dip_exp
-                          : (g.sys == SYS_N2AR && g_defer >= (precision == HH_PRECISION_MIXED ? 2 : 1));
+                          : (g.sys == SYS_N2AR &&
+                             g_defer >= (precision == HH_PRECISION_MIXED && n * (uint64_t)P.N < N2AR_DEFER_SAMPLES ? 2 : 1));
   return sys_ok && io.n_sat == 0 && !io.series && !io.records && !P.prmu &&
          (P.inject_item < 0 || P.inject_status >= HH_ST_NAN_DIPOLE);
 }
@@ -1200,15 +1205,15 @@ int traj_block_sync() {
 // (the reference drops a trajectory whose correlation_eval returns 1 while still
 // counting it: both branches are replayed with the opposite weight).  With deferred
 // samples the iterations go in launches whose sample contexts fit the buffer (at most
-// 32 GiB and 40 % of the free memory, or HH_DEFER_BUDGET_MB; in FP64, whose contexts are
-// larger, an iteration that does not fit goes in several launches); a launch that wrote
+// 32 GiB and 40 % of the free memory, or HH_DEFER_BUDGET_MB; an iteration that does not
+// fit goes in several launches); a launch that wrote
 // more contexts than the buffer holds repeats the call with a larger estimate of
 // contexts per item (HH_DEFER_EST sets the first one), and a second overflow with
 // in-kernel samples.
 int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n, uint64_t per_iter,
               uint64_t n_iter, int *nfail_out) {
   const size_t N = (size_t)P.N;
-  const bool eligible = defer_eligible(precision, P, io0);
+  const bool eligible = defer_eligible(precision, P, io0, n);
   const bool mixed = precision == HH_PRECISION_MIXED;
   const size_t vb = mixed ? sizeof(float) : sizeof(double);
   const size_t ctx_b = mixed ? sizeof(SampleCtx<float, 6>) : sizeof(SampleCtx<double, 6>);
@@ -1240,7 +1245,7 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       const uint64_t max_items = (uint64_t)std::max(1.0, budget / per_item);
       it_launch = std::min<uint64_t>(n_iter, std::max<uint64_t>(1, max_items / (2 * per_iter)));
       tr_launch = std::min<uint64_t>(n, it_launch * per_iter);
-      if (!mixed) tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
+      tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
       items_launch = 2 * tr_launch;
       cap = (unsigned long long)(est * double(items_launch)) + 16384ull;  // and the solo warps' unused ones
       if (getenv("HH_DEFER_TRACE"))
@@ -1281,7 +1286,7 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     } else {
       uint64_t t1 = 0;
       for (uint64_t t0 = 0; t0 < n; t0 = t1) {
-        // whole iterations, or (FP64) a part of one
+        // whole iterations, or a part of one
         const uint64_t i0 = t0 / per_iter;
         const bool part = tr_launch < per_iter;
         t1 = part ? std::min({n, (i0 + 1) * per_iter, t0 + tr_launch}) : std::min(n, (i0 + it_launch) * per_iter);

@@ -334,9 +334,10 @@ int hh_cuda_debug_set_ch4_dipole(int precision, int variant);
 
 /* Diagnostic (no counterpart in the reference): where the plain C(t) evaluates the
  * dipoles at the sample times.  mode 0: inside the trajectory kernel; 1 (the default, or
- * the environment variable HH_DEFER_SAMPLES): CO2-Ar on both paths and N2-Ar in FP64
- * deferred to the sample kernels (the trajectory kernel writes one dense-output context
- * per step and tests only R > Rcut); 2: mixed N2-Ar too; -1 leaves the mode as it is.
+ * the environment variable HH_DEFER_SAMPLES): CO2-Ar and N2-Ar deferred to the sample
+ * kernels (the trajectory kernel writes one dense-output context per step and tests only
+ * R > Rcut), but for mixed N2-Ar calls of fewer than 2^19 trajectories x sample times; 2:
+ * these too; -1 leaves the mode as it is.
  * *previous (if not NULL) receives the mode before the call.  Both placements give the
  * same samples and C(t) up to the order of the FP64 sums. */
 int hh_cuda_debug_set_defer(int mode, int *previous);
