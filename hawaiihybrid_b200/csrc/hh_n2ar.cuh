@@ -149,15 +149,30 @@ __device__ __forceinline__ float n2_div(float a, float b) { return __fdiv_rn(a, 
 __device__ __forceinline__ double n2_div(double a, double b) { return __ddiv_rn(a, b); }
 
 // y(d) of an N-Ar pair and dy/dd as n2ar_pair_y, with fixed rounding
-template <typename T> __device__ __forceinline__ void n2ar_pair_y_rn(T d, T &y, T &dy) {
+// LANES (solo kernel): the two quotients side by side on lanes 2 apart, which hold the same d
+template <typename T, bool LANES = false> __device__ __forceinline__ void n2ar_pair_y_rn(T d, T &y, T &dy) {
   const T e = exp(-n2_mul(d, T(0.5)));
-  if (d < T(6)) {
+  if (!LANES && d < T(6)) {
     y = e;
     dy = -n2_mul(e, T(0.5));
     return;
   }
   const T d2 = n2_mul(d, d), d6 = n2_mul(n2_mul(d2, d2), d2), d7 = n2_mul(d6, d);
-  const T a6 = n2_div(T(1e4), d6), a7 = n2_div(T(6e4), d7);
+  T a6, a7;
+  if constexpr (LANES) {
+    const bool second = (threadIdx.x & 2) != 0;
+    const T q = n2_div(second ? T(6e4) : T(1e4), second ? d7 : d6), o = __shfl_xor_sync(0xffffffffu, q, 2);
+    a6 = second ? o : q;
+    a7 = second ? q : o;
+  } else {
+    a6 = n2_div(T(1e4), d6);
+    a7 = n2_div(T(6e4), d7);
+  }
+  if (LANES && d < T(6)) {
+    y = e;
+    dy = -n2_mul(e, T(0.5));
+    return;
+  }
   if (d < T(20)) {
     const T w = T(14), r = n2_div(n2_sub(d, T(6)), w);
     const T r2 = n2_mul(r, r), r3 = n2_mul(r2, r), r4 = n2_mul(r3, r), r5 = n2_mul(r4, r);
@@ -222,7 +237,7 @@ template <typename T> __device__ __forceinline__ T n2ar_unit_grad(T h, T w1) {
 // the weights of `net` (shared memory in the kernels), so the code stays small.
 // FP32: two hidden units per iteration with the paired FP32 instructions of sm_100,
 // each half the scalar loop's fma chain in the same order (h_j over i, a_i over j), so
-// the values are bit for bit those of the scalar loop and of n2ar_pes_grad_coop.
+// the values are bit for bit those of the scalar loop and of n2ar_pes_grad_lanes.
 template <typename T>
 __device__ __noinline__ N2arGrad<T> n2ar_pes_grad(const N2arPesNet<T> *net, T d1, T d2) {
   constexpr int NP = N2AR_PES_NP;
@@ -326,17 +341,18 @@ template <int N> __device__ __forceinline__ void n2_load_row(double *d, const do
   }
 }
 
-// Shared memory of the cooperative gradient: the first-layer weights with one hidden unit
-// per lane (wf, once per block) and a warp's exchange buffer.
-template <typename T> struct N2arCoopWeights {
-  T wf[N2AR_PES_NP][32];  // wf[i][j] = W0[i][j]
+// Shared memory of the cooperative gradient: the first-layer weights with one input per
+// lane (wf, once per block; rows 16 bytes apart modulo the banks, so that the lanes' 16-byte
+// loads meet different ones) and a warp's exchange buffer.
+template <typename T> struct alignas(16) N2arCoopWeights {
+  T wf[N2AR_PES_NP][32 + 16 / sizeof(T)];  // wf[i][j] = W0[i][j]
 };
 template <typename T> struct alignas(16) N2arCoopScratch {
   T y[4];                 // y0, y1, y2, 1 (the first and last set once, n2ar_coop_init)
-  T dy[2], pad[2];
+  T yx[12];               // the stage point
   T ptr[N2AR_PES_ROW];    // (rows start on 16 bytes)
   T g[32];
-  T out[N2AR_PES_NP][4];  // a_i / xscale_i, dp_i/dy_1, dp_i/dy_2
+  T a[N2AR_PES_ROW], j[2][N2AR_PES_ROW];  // a_i / xscale_i; dp_i/dy_1 and dp_i/dy_2
 };
 
 template <typename T>
@@ -350,32 +366,26 @@ __device__ __forceinline__ void n2ar_coop_init(N2arCoopWeights<T> *cw, N2arCoopS
   __syncthreads();
 }
 
-// n2ar_pes_grad with the 32 lanes of a warp on one (d1, d2), bit for bit: the pair
-// functions of d1 on even lanes and d2 on odd ones, PIP i with its Jacobian on lane i
-// (absent variables are exact factors of 1), hidden unit j on lane j (the same sum over
+// n2ar_pes_grad with the 32 lanes of a warp on one (d1, d2), bit for bit: end lane % 2 of the
+// molecule's pair function, distance d, and sum on each lane, PIP i with its Jacobian on lane
+// i (absent variables are exact factors of 1), hidden unit j on lane j (the same sum over
 // the 17 inputs, in the same order), a_i = sum_j W0[i][j] g_j on lane i over the units in
-// the order of the per-lane loop, and the sums of j1_i a_i / xscale_i and j2_i a_i /
-// xscale_i over i in order on every lane.  The values pass through shared memory.  A
-// trajectory therefore takes the same steps in the solo kernel as in the bulk kernel.  All
-// 32 lanes call it with the same arguments but code (n2ar_pip_code).  Latency bounds it
-// (one right-hand side: 3,700 cycles in FP64): with every
-// lane forming all the inputs and values passed by shuffles the solo launch took, in FP64
-// (20,011 x 5,000), 60.7 ms, so 42 to 47; on the mixed path (131,072 x 16,384) 41.5 and 39.7.
+// the order of the per-lane loop, and the sum of j_i a_i / xscale_i over i in order.  The
+// values pass through shared memory.  A trajectory therefore takes the same steps in the
+// solo kernel as in the bulk kernel.  All 32 lanes call it; returns dV/dd of the lane's end.
+// Latency bounds it: the 32 and the two 17 term chains alone are 570 cycles in FP64 and 270 in
+// FP32; the rows are 16-byte loads ahead of them.  Part of the solo right-hand side
+// (n2ar_rhs_lane).
 template <typename T>
-__device__ __noinline__ N2arGrad<T> n2ar_pes_grad_coop(const N2arPesNet<T> *net, const N2arCoopWeights<T> *cw,
-                                                       N2arCoopScratch<T> *sc, unsigned code, T d1, T d2) {
+__device__ __forceinline__ T n2ar_pes_grad_lanes(const N2arPesNet<T> *net, const N2arCoopWeights<T> *cw,
+                                                 N2arCoopScratch<T> *sc, unsigned code, T d) {
   static_assert(N2AR_PES_NH == 32 && N2AR_PES_NP <= 32, "one hidden unit per lane");
   constexpr int NP = N2AR_PES_NP;
   const int lane = threadIdx.x & 31;
   const int ir = lane < NP ? lane : NP - 1;
-  {
-    T y, dy;
-    n2ar_pair_y_rn((lane & 1) ? d2 : d1, y, dy);
-    if (lane < 2) {
-      sc->y[1 + lane] = y;
-      sc->dy[lane] = dy;
-    }
-  }
+  T yd, dy;
+  n2ar_pair_y_rn<T, true>(d, yd, dy);
+  if (lane < 2) sc->y[1 + lane] = yd;
   __syncwarp();
   T p, j1, j2;
   {
@@ -423,9 +433,8 @@ __device__ __noinline__ N2arGrad<T> n2ar_pes_grad_coop(const N2arPesNet<T> *net,
   __syncwarp();
   T h = net->b0[lane];
   {
-    T w[NP], q[N2AR_PES_ROW];
-#pragma unroll
-    for (int i = 0; i < NP; ++i) w[i] = cw->wf[i][lane];
+    T w[N2AR_PES_ROW], q[N2AR_PES_ROW];
+    n2_load_row<N2AR_PES_ROW>(w, net->w0t[lane]);
     n2_load_row<N2AR_PES_ROW>(q, sc->ptr);
 #pragma unroll
     for (int i = 0; i < NP; ++i) h = n2_fma(q[i], w[i], h);
@@ -435,34 +444,30 @@ __device__ __noinline__ N2arGrad<T> n2ar_pes_grad_coop(const N2arPesNet<T> *net,
   T a = T(0);
   {
     // loads ahead of the chain (one at a time they cost 31 cycles per unit)
-    T g[32], w[16];
-    n2_load_row<32>(g, sc->g);
 #pragma unroll
     for (int b = 0; b < 2; ++b) {
+      T g[16], w[16];
+      n2_load_row<16>(g, sc->g + 16 * b);
+      n2_load_row<16>(w, &cw->wf[ir][16 * b]);
 #pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = net->w0t[16 * b + j][ir];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) a = n2_fma(w[j], g[16 * b + j], a);
+      for (int j = 0; j < 16; ++j) a = n2_fma(w[j], g[j], a);
     }
   }
   if (lane < NP) {
-    sc->out[lane][0] = n2_mul(a, net->ixscale[ir]);
-    sc->out[lane][1] = j1;
-    sc->out[lane][2] = j2;
+    sc->a[lane] = n2_mul(a, net->ixscale[ir]);
+    sc->j[0][lane] = j1;
+    sc->j[1][lane] = j2;
   }
   __syncwarp();
-  T a1 = T(0), a2 = T(0);
+  T sum = T(0);
+  {
+    T ai[N2AR_PES_ROW], ji[N2AR_PES_ROW];
+    n2_load_row<N2AR_PES_ROW>(ai, sc->a);
+    n2_load_row<N2AR_PES_ROW>(ji, sc->j[lane & 1]);
 #pragma unroll
-  for (int i = 0; i < NP; ++i) {
-    T o[4];
-    n2_load_row<4>(o, sc->out[i]);
-    a1 = n2_fma(o[1], o[0], a1);
-    a2 = n2_fma(o[2], o[0], a2);
+    for (int i = 0; i < NP; ++i) sum = n2_fma(ji[i], ai[i], sum);
   }
-  const T s = n2_mul(net->yscale, T(1.0 / HH_HTOCM));
-  const T dy1 = sc->dy[0], dy2 = sc->dy[1];
-  __syncwarp();  // the next evaluation writes the buffer again
-  return {n2_mul(n2_mul(a1, dy1), s), n2_mul(n2_mul(a2, dy2), s)};
+  return n2_mul(n2_mul(sum, dy), n2_mul(net->yscale, T(1.0 / HH_HTOCM)));
 }
 
 // V (Hartree) for d1 = |N1-Ar|, d2 = |N2-Ar| (pes_xyz, ai_pes_n2_ar_pip_nn.cpp:127-132)

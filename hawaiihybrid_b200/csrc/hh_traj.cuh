@@ -602,16 +602,45 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct Co2
 // (R, x = r^.u^): the Euler-angle rotation of the reference (examples/correlation_n2_ar.cpp:52-76)
 // maps body z to r^ and body x to the in-plane normal to r^ on the N1 side.
 // SOLO_: the solo kernel's instance (one trajectory per warp), whose right-hand side
-// the 32 lanes evaluate cooperatively (n2ar_pes_grad_coop)
-template <typename PHYS, typename STG, bool COMP> struct N2ArSoloArgs {
-  const N2arPesNet<PHYS> *pes;
-  const N2arCoopWeights<PHYS> *coop;
-  N2arCoopScratch<PHYS> *scr;
-  unsigned pip;
-  double inv_mu, inv_II;
-};
-template <typename PHYS, typename STG, bool COMP>
-__device__ STG n2ar_rhs_out_of_line(N2ArSoloArgs<PHYS, STG, COMP> a, STG ysc, int c);
+// the 32 lanes evaluate together (n2ar_rhs_lane)
+//
+// Component c of the right-hand side with the 32 lanes of a warp on one stage point, bit for
+// bit as N2ArSys::rhs rounds it; out of line, one copy for the stages.  Lane parity is the end
+// of the molecule: a lane forms its end's vector, distance, pair function and sum; then lane
+// c its own component (LinearLane).  FP64 5,500 -> 3,400 cycles and FP32 2,330 -> 2,040 against
+// every lane forming both ends and all twelve components around the shared gradient.
+template <typename T>
+__device__ __noinline__ T n2ar_rhs_lane(const N2arPesNet<T> *net, const N2arCoopWeights<T> *cw, N2arCoopScratch<T> *scr,
+                                        unsigned code, T ysc, T im, T iI, LinearLane L) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  if (lane < 12) scr->yx[lane] = ysc;  // (the barriers of the gradient keep two calls apart)
+  __syncwarp();
+  const T *y = scr->yx;
+  const T r[3] = {y[0], y[1], y[2]}, u[3] = {y[6], y[7], y[8]};
+  const T v1 = y[L.s1], v2 = y[L.s2], v3 = y[L.s3], v4 = y[L.s4];
+  auto norm2 = [](const T *v) { return n2_fma(v[2], v[2], n2_fma(v[0], v[0], n2_mul(v[1], v[1]))); };
+  const T iu = inv_sqrt(norm2(u));
+  const T h = T(N2AR_L / 2.0), hs = (lane & 1) ? h : -h;
+  T e[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) e[c] = n2_fma(hs, n2_mul(u[c], iu), r[c]);
+  const T ie = inv_sqrt(norm2(e));
+  const T a = n2_mul(n2ar_pes_grad_lanes<T>(net, cw, scr, code, T(1) / ie), ie);
+  const T a1 = __shfl_sync(FULL, a, 0), a2 = __shfl_sync(FULL, a, 1);
+  // components: p = v1; force -(a1 e1_k + a2 e2_k) of r_k = v1, u_k = v2; axis j_k1 u_k2 -
+  // j_k2 u_k1; torque -(u^_k1 G_k2 - u^_k2 G_k1), G_m = h (a2 e2_m - a1 e1_m), of
+  // r_k2 = v1, u_k1 = v2, u_k2 = v3, r_k1 = v4
+  const T s = L.g == 2 ? T(1) : iu, p = n2_mul(v2, s), q = n2_mul(v3, s);
+  const T ra = L.g == 1 ? v1 : v4;
+  const T e1a = n2_fma(-h, p, ra), e2a = n2_fma(h, p, ra), e1b = n2_fma(-h, q, v1), e2b = n2_fma(h, q, v1);
+  const T x = n2_mul(a2, e2a), fr = n2_fma(a1, e1a, x);
+  const T ga = n2_mul(h, n2_fma(-a1, e1a, x)), gb = n2_mul(h, n2_fma(-a1, e1b, n2_mul(a2, e2b)));
+  // the axis and the torque: the first product fused
+  const T X = L.g == 2 ? v1 : p, Y = L.g == 2 ? p : gb, Z = L.g == 2 ? -v4 : -q, W = L.g == 2 ? q : ga;
+  const T cr = n2_fma(X, Y, n2_mul(Z, W));
+  return L.g == 0 ? n2_mul(v1, im) : L.g == 1 ? -fr : L.g == 2 ? n2_mul(cr, iI) : -cr;
+}
 
 template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2ArSys {
   static constexpr bool SOLO = SOLO_;
@@ -626,10 +655,20 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
   const N2arDipFold *fold;      // shared-memory copies
   const N2arPesNet<PHYS> *pes;
   const float4 *dtab;           // mixed path: the dipole table (hh_n2ar.cuh), global memory
-  const N2arCoopWeights<PHYS> *coop;  // solo kernel: shared memory of n2ar_pes_grad_coop
+  const N2arCoopWeights<PHYS> *coop;  // solo kernel: shared memory of n2ar_pes_grad_lanes
   N2arCoopScratch<PHYS> *scr;         // (this warp's)
   unsigned pip;                       // (this lane's PIP)
   template <typename YT> __device__ void rhs(const YT *y, STG *f) const {
+    if constexpr (SOLO) {
+      STG ys[N];
+#pragma unroll
+      for (int i = 0; i < N; ++i) ys[i] = STG(y[i]);
+      const int lane = threadIdx.x & 31, c = lane < N ? lane : N - 1;
+      const STG fc = rhs_c(pick_component<N>(ys, c), c);
+#pragma unroll
+      for (int i = 0; i < N; ++i) f[i] = __shfl_sync(0xffffffffu, fc, i);
+      return;
+    }
     const PHYS r[3] = {PHYS(y[0]), PHYS(y[1]), PHYS(y[2])};
     const PHYS u[3] = {PHYS(y[6]), PHYS(y[7]), PHYS(y[8])};
     const PHYS iu = inv_sqrt(u[0] * u[0] + u[1] * u[1] + u[2] * u[2]);
@@ -643,11 +682,7 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     }
     const PHYS i1 = inv_sqrt(e1[0] * e1[0] + e1[1] * e1[1] + e1[2] * e1[2]);
     const PHYS i2 = inv_sqrt(e2[0] * e2[0] + e2[1] * e2[1] + e2[2] * e2[2]);
-    N2arGrad<PHYS> g;
-    if constexpr (SOLO)
-      g = n2ar_pes_grad_coop<PHYS>(pes, coop, scr, pip, PHYS(1) / i1, PHYS(1) / i2);
-    else
-      g = n2ar_pes_grad<PHYS>(pes, PHYS(1) / i1, PHYS(1) / i2);
+    const N2arGrad<PHYS> g = n2ar_pes_grad<PHYS>(pes, PHYS(1) / i1, PHYS(1) / i2);
     const PHYS a1 = g.g1 * i1, a2 = g.g2 * i2;
     PHYS Gr[3], Gu[3];
 #pragma unroll
@@ -674,7 +709,7 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
   }
   // component c of f (solo kernel), the values those of rhs
   __device__ __forceinline__ STG rhs_c(STG ysc, int c) const {
-    return n2ar_rhs_out_of_line<PHYS, STG, COMP>({pes, coop, scr, pip, inv_mu, inv_II}, ysc, c);
+    return n2ar_rhs_lane<PHYS>(pes, coop, scr, pip, ysc, STG(inv_mu), STG(inv_II), LinearLane(threadIdx.x & 31));
   }
   // q = (r[3], u[3]); the body-frame dipole is the FP64 network on the FP64 path and
   // the FP32 table of hh_n2ar.cuh (the network outside its R range) on the mixed path
@@ -697,26 +732,6 @@ template <typename PHYS, typename STG, bool COMP, bool SOLO_ = false> struct N2A
     for (int c = 0; c < 3; ++c) d[c] = PHYS(b.dz * rh[c] + b.dx * e[c] * ie);
   }
 };
-
-// Component c of the N2-Ar right-hand side for the solo kernel: the full stage point
-// gathered from the lanes, N2ArSys::rhs around the shared gradient on every lane; out of
-// line, one copy for all stages.
-template <typename PHYS, typename STG, bool COMP>
-__device__ __noinline__ STG n2ar_rhs_out_of_line(N2ArSoloArgs<PHYS, STG, COMP> a, STG ysc, int c) {
-  using Sys = N2ArSys<PHYS, STG, COMP, true>;
-  Sys sys;
-  sys.inv_mu = a.inv_mu;
-  sys.inv_II = a.inv_II;
-  sys.pes = a.pes;
-  sys.coop = a.coop;
-  sys.scr = a.scr;
-  sys.pip = a.pip;
-  STG ys[Sys::N], f[Sys::N];
-#pragma unroll
-  for (int i = 0; i < Sys::N; ++i) ys[i] = __shfl_sync(0xffffffffu, ysc, i);
-  sys.rhs(ys, f);
-  return pick_component<Sys::N>(f, c);
-}
 
 // find_closest_integer / find_closest_half_integer (src/hawaii.c:360-393): the
 // requantized |j| of the linear monomer.  The half-integer rule returns 0 below 0.25,
