@@ -515,14 +515,25 @@ int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int div, 
 // trajectories per warp to one).  Timed on the launch's first items, into scratch
 // C(t) and counters, so the call's own results are untouched:
 //   1. each warps-per-block candidate with the full hand-off threshold: bulk kernel time;
-//   2. with the faster shape, the launch time at thresholds of 2 cap and, if that is
-//      faster than cap, 4 cap; otherwise cap / 2 and, if faster, cap / 4.  More than cap:
+//   2. with the faster shape, the launch time at thresholds of 2 cap, 4 cap and 8 cap as long
+//      as each is faster; otherwise cap / 2 and, if faster, cap / 4.  More than cap:
 //      the solo kernel's warps take several stored items in turn, which pays where few of
 //      the bulk kernel's lanes are left busy long before the end (N2-Ar FP64, 20,011
-//      trajectories: 10 % of the lanes from a fifth of the launch on; bulk launch 82 ms
-//      with a threshold of cap, 49 with 4 cap, the call 142 and 117).
+//      trajectories: 10 % of the lanes from a fifth of the launch on; the call 135 ms with a
+//      threshold of cap, 122 with 2, 109 with 4, 102 with 8 and 108 with 16; mixed,
+//      131,072 x 16,384: 97, 92, 89, 87 and 87).
+// Before that, and in smaller launches, the threshold is default_handoff_mul x cap: at that
+// many items or fewer all run in the solo kernel.  A warp per trajectory is the faster form
+// far beyond one item per warp slot, since the bulk kernel's rounds last as long for few open
+// lanes as for many.  ms per call at thresholds of 1, 2, 4, 8 and 16 cap, FP64, N = 4,096:
+//   CO2-Ar 1,000   14.9 13.7 13.6 13.5 13.4      N2-Ar 1,000   32.9 22.1 22.3 21.9 21.9
+//   CO2-Ar 4,000   18.5 17.0 15.9 14.7 14.7      N2-Ar 4,000   71.2 78.3 50.1 43.9 42.0
+//   CO2-Ar 16,000  29.5 26.1 22.9 23.7 27.3      N2-Ar 16,000  110 97.6 87.2 81.8 89.5
+//   He-Ar 1,000    1.77 1.32 1.32 1.32 1.33      PR_MU CO2-Ar 4,096  22.8 19.8 17.8 17.8 17.7
+// (mixed path: CO2-Ar 1,000 2.71 2.32 2.34, PR_MU 4,096 5.23 4.77 3.66).  CH4-CO2, whose
+// trajectories are all about as long, gains nothing.
 // HH_TRAJ_WARPS (4 or 8) and HH_TRAJ_HANDOFF_DIV (1, 2 or 4) fix a choice instead.
-constexpr int TRAJ_TUNE_MIN_ITEMS = 16384;  // smaller launches use the defaults, untuned
+constexpr int TRAJ_TUNE_MIN_ITEMS = 16384;  // smaller launches use the defaults
 constexpr int TRAJ_TUNE_ITEMS = 32768;      // items the timing runs integrate
 
 template <int SYS, typename PHYS, typename STG, bool COMP>
@@ -580,7 +591,7 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
     int rc = run(w_best, 1, 1, &bulk, &all);
     if (rc) return rc;
     float best = all;
-    for (int m : {2, 4}) {
+    for (int m : {2, 4, 8}) {
       rc = run(w_best, 1, m, &bulk, &all);
       if (rc) return rc;
       if (!(all < best)) break;
@@ -604,6 +615,8 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
   return HH_OK;
 }
 
+constexpr int default_handoff_mul(int sys) { return sys == SYS_CH4CO2 ? 1 : sys == SYS_N2AR ? 8 : 4; }
+
 template <int SYS, typename PHYS, typename STG, bool COMP>
 int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
   (void)grid_out;
@@ -615,7 +628,7 @@ int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
   }
   const int w = tt.warps ? tt.warps : traj_warps<PHYS>();
   const int d = tt.handoff_div ? tt.handoff_div : 1;
-  const int m = tt.handoff_mul ? tt.handoff_mul : 1;
+  const int m = tt.handoff_mul ? tt.handoff_mul : default_handoff_mul(SYS);
   return launch_traj_pick<SYS, PHYS, STG, COMP>(P, io, w, d, m, false);
 }
 
