@@ -1214,6 +1214,9 @@ int traj_block_sync() {
   return e ? std::max(0, atoi(e)) : 1;
 }
 
+// contexts beyond the estimate: the solo warps' unused reservations
+constexpr size_t DEFER_HEADROOM = 16384;
+
 // The plain C(t) launches of run_trajectories, then the replay of failed trajectories
 // (the reference drops a trajectory whose correlation_eval returns 1 while still
 // counting it: both branches are replayed with the opposite weight).  With deferred
@@ -1248,24 +1251,30 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     unsigned long long cap = 0;
     uint64_t it_launch = n_iter, tr_launch = n, items_launch = 2 * n;
     if (defer) {
-      size_t free_b = 0, total_b = 0;
-      CK(cudaMemGetInfo(&free_b, &total_b));
-      double budget = std::min(32.0 * double(1ull << 30), 0.4 * double(free_b + g.dctx.cap + g.dvals.cap));
-      if (const char *eb = getenv("HH_DEFER_BUDGET_MB")) budget = std::max(1.0, atof(eb)) * double(1 << 20);
       if (attempt == 0)
         if (const char *ee = getenv("HH_DEFER_EST")) est = std::max(0.01, atof(ee));
-      const double per_item = est * double(ctx_b + 2 * vb);
-      const uint64_t max_items = (uint64_t)std::max(1.0, budget / per_item);
-      it_launch = std::min<uint64_t>(n_iter, std::max<uint64_t>(1, max_items / (2 * per_iter)));
-      tr_launch = std::min<uint64_t>(n, it_launch * per_iter);
-      tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
+      const char *eb = getenv("HH_DEFER_BUDGET_MB");
+      const size_t want = (size_t)(est * double(2 * n)) + DEFER_HEADROOM;
+      size_t free_b = 0, total_b = 0;
+      // the whole call's contexts fit the buffers of an earlier one: no need to know the free
+      // memory, a query of the driver that takes 0.13 ms, 10 at the 99th percentile and 80 at
+      // times (CO2-Ar mixed, 4 x 102,400 x 32,768: one call in five took 80 to 140 ms, not 58)
+      if (eb || g.dctx.cap < want * ctx_b || g.dvals.cap < want * 2 * vb) {
+        CK(cudaMemGetInfo(&free_b, &total_b));
+        double budget = std::min(32.0 * double(1ull << 30), 0.4 * double(free_b + g.dctx.cap + g.dvals.cap));
+        if (eb) budget = std::max(1.0, atof(eb)) * double(1 << 20);
+        const double per_item = est * double(ctx_b + 2 * vb);
+        const uint64_t max_items = (uint64_t)std::max(1.0, budget / per_item);
+        it_launch = std::min<uint64_t>(n_iter, std::max<uint64_t>(1, max_items / (2 * per_iter)));
+        tr_launch = std::min<uint64_t>(n, it_launch * per_iter);
+        tr_launch = std::min<uint64_t>(tr_launch, std::max<uint64_t>(1, max_items / 2));
+      }
       items_launch = 2 * tr_launch;
-      cap = (unsigned long long)(est * double(items_launch)) + 16384ull;  // and the solo warps' unused ones
+      cap = (unsigned long long)(est * double(items_launch)) + DEFER_HEADROOM;
       if (getenv("HH_DEFER_TRACE"))
         fprintf(stderr, "[defer] attempt %d est %.3f items %llu cap %llu (buffer %llu) launches of %llu trajectories, "
-                "budget %.2f GB, free %.2f GB\n", attempt, est, (unsigned long long)items_launch, cap,
-                (unsigned long long)(g.dctx.cap / ctx_b), (unsigned long long)tr_launch, budget / 1e9,
-                free_b / 1e9);
+                "free %.2f GB\n", attempt, est, (unsigned long long)items_launch, cap,
+                (unsigned long long)(g.dctx.cap / ctx_b), (unsigned long long)tr_launch, free_b / 1e9);
       // 10 % headroom: the estimate moves a little from call to call, and a larger
       // buffer would otherwise be reallocated (cudaFree and cudaMalloc of gigabytes)
       // inside a call
