@@ -32,6 +32,7 @@
 #include <math.h>
 #include <stdint.h>
 
+#include "hh_interval.h"
 #include "hh_traj.cuh"
 
 namespace hh {
@@ -108,7 +109,7 @@ struct DeferCo2arDip {
   float4 row[CO2AR_NINT][CO2AR_NL][4];  // [interval][l / 2][16 words]
   float rlo[CO2AR_NINT];
   int fdip[CO2AR_NINT];
-  unsigned char ivl[164];               // interval of R in [j / 4, (j + 1) / 4), j <= 160
+  unsigned char ivl[R_SLOTS];           // interval of the R of slot j (r_slot)
 };
 template <> struct DeferSys<SYS_CO2AR, float, float> {
   static constexpr int NQ = 6;
@@ -128,7 +129,7 @@ template <> struct DeferSys<SYS_CO2AR, float, float> {
       d->rlo[i] = float(g->rlo[i]);
       d->fdip[i] = g->fdip[i];
     }
-    for (int j = threadIdx.x; j < 164; j += blockDim.x) {
+    for (int j = threadIdx.x; j < R_SLOTS; j += blockDim.x) {
       const double r = 0.25 * j;
       int i = 0;
       while (i < CO2AR_NINT - 1 && !(r < g->rbound[i])) ++i;
@@ -156,7 +157,7 @@ template <> struct DeferSys<SYS_CO2AR, float, float> {
   // sum_l P_l(x) z_l(R) and sum_l P_l'(x) x_l(R) of one sample
   __device__ __forceinline__ void sums(float R, float iR, const float2 (&P)[11], const float2 (&dP)[11], bool second,
                                        float &dz, float &ax) const {
-    const int i = t->ivl[min(int(R * 4.f), 163)];
+    const int i = t->ivl[r_slot(R)];
     const float2 tt = splat2(R - t->rlo[i]);
     const int fl = t->fdip[i];
     const float iR2 = iR * iR, iR4 = iR2 * iR2, iR5 = iR4 * iR, iR6 = iR5 * iR, iR7 = iR6 * iR;
@@ -216,7 +217,7 @@ struct DeferCo2arDipD {
   double2 row[CO2AR_NINT][CO2AR_NL][8];  // coefficient k of the (z, x) rows: a0..a3, b4..b7
   double rlo[CO2AR_NINT];
   int fdip[CO2AR_NINT];
-  unsigned char ivl[164];                // interval of R in [j / 4, (j + 1) / 4), j <= 160
+  unsigned char ivl[R_SLOTS];            // interval of the R of slot j (r_slot)
 };
 template <> struct DeferSys<SYS_CO2AR, double, double> {
   static constexpr int NQ = 6;
@@ -234,7 +235,7 @@ template <> struct DeferSys<SYS_CO2AR, double, double> {
       d->rlo[i] = g->rlo[i];
       d->fdip[i] = g->fdip[i];
     }
-    for (int j = threadIdx.x; j < 164; j += blockDim.x) {
+    for (int j = threadIdx.x; j < R_SLOTS; j += blockDim.x) {
       const double r = 0.25 * j;
       int i = 0;
       while (i < CO2AR_NINT - 1 && !(r < g->rbound[i])) ++i;
@@ -250,7 +251,7 @@ template <> struct DeferSys<SYS_CO2AR, double, double> {
     const double uh[3] = {q[3] * iu, q[4] * iu, q[5] * iu};
     const double x = rh[0] * uh[0] + rh[1] * uh[1] + rh[2] * uh[2];
     const double R = R2 * iR;
-    const int i = t->ivl[min(int(R * 4.0), 163)];
+    const int i = t->ivl[r_slot(R)];
     const double tt = R - t->rlo[i];
     const bool inv = t->fdip[i] & 1;
     const double iR2 = iR * iR, iR4 = iR2 * iR2, iR5 = iR4 * iR, iR6 = iR4 * iR2, iR7 = iR5 * iR2;
