@@ -47,7 +47,7 @@ EXPORTS = (
     "hh_cuda_prmu", "hh_cuda_debug_n2ar_dipole", "hh_cuda_m2", "hh_cuda_debug_tuning",
     "hh_cuda_debug_kernel_ms", "hh_cuda_debug_ch4co2_fold", "hh_cuda_moment_sums", "hh_cuda_debug_traj_tuning",
     "hh_cuda_debug_set_ch4_dipole", "hh_cuda_debug_set_defer", "hh_cuda_debug_set_defer_overlap", "hh_cuda_vegas",
-    "hh_cuda_set_requantization",
+    "hh_cuda_set_requantization", "hh_cuda_debug_candidates",
     "hh_write_correlation_function_ext", "hh_write_spectral_function_ext",
 )
 HH_REQ_NONE, HH_REQ_INTEGER, HH_REQ_HALFINTEGER = 0, 1, 2
@@ -104,6 +104,7 @@ class Stats(C.Structure):
 
 _dp = np.ctypeslib.ndpointer(dtype=np.float64, flags="C_CONTIGUOUS")
 _u32p = np.ctypeslib.ndpointer(dtype=np.uint32, flags="C_CONTIGUOUS")
+_u8p = np.ctypeslib.ndpointer(dtype=np.uint8, flags="C_CONTIGUOUS")
 _lib = None
 
 
@@ -144,6 +145,7 @@ def load(path: str | None = None):
     L.hh_cuda_strerror.restype = C.c_char_p
     L.hh_cuda_strerror.argtypes = [C.c_int]
     L.hh_cuda_mt_stream.argtypes = [C.c_uint32, C.c_uint64, _u32p]
+    L.hh_cuda_debug_candidates.argtypes = [C.POINTER(CalcParamsC), C.c_double, _u32p, C.c_uint64, C.c_int, _u8p]
     L.hh_cuda_debug_inject.argtypes = [C.c_int, C.c_int, C.c_int, C.c_int]
     L.hh_cuda_debug_item_trace.argtypes = [C.c_void_p, C.c_uint64]
     L.hh_cuda_fma_peak.argtypes = [C.c_int, C.POINTER(C.c_double)]
@@ -187,6 +189,17 @@ def ch4co2_fold_shape() -> tuple[int, int]:
     nb, ng = C.c_int(0), C.c_int(0)
     check(load().hh_cuda_debug_ch4co2_fold(C.byref(nb), C.byref(ng)))
     return nb.value, ng.value
+
+
+def candidate_accepted(params, T: float, words: np.ndarray, prefilter: bool) -> np.ndarray:
+    """Which of the candidates that the stream words [n_cand, words per candidate] make are
+    accepted at T (hh_cuda_debug_candidates), with or without the CH4-CO2 rejection ahead of
+    the momenta."""
+    w = np.ascontiguousarray(words, dtype=np.uint32)
+    out = np.empty(w.shape[0], dtype=np.uint8)
+    pc = params.to_c()
+    check(load().hh_cuda_debug_candidates(C.byref(pc), float(T), w.ravel(), w.shape[0], int(prefilter), out))
+    return out.astype(bool)
 
 
 def defer_samples(mode: int = -1) -> int:

@@ -2466,6 +2466,36 @@ int hh_cuda_mt_stream(uint32_t seed, uint64_t n, uint32_t *out) {
   return reseed(seed);
 }
 
+int hh_cuda_debug_candidates(const hh_calc_params *p, double T, const uint32_t *words, uint64_t n_cand, int prefilter,
+                             unsigned char *accept) {
+  if (!g.init) return HH_E_NOT_INITIALIZED;
+  int rc = check_params(p);
+  if (rc) return rc;
+  if (!words || !accept || n_cand == 0 || n_cand > (1ull << 23) || !(T > 0)) return HH_E_INVALID_ARGUMENT;
+  CK(cudaSetDevice(g.device));
+  const size_t nw = n_cand * (size_t)g.D;
+  DevBuf<uint32_t> dw;
+  auto run = [&]() -> int {
+    CK(dw.ensure(nw));
+    CK(g.accept.ensure(n_cand));
+    CK(g.consumed.ensure(n_cand));
+    CK(g.qp_cand.ensure(n_cand * (size_t)g.QP));
+    CK(g.energy.ensure(n_cand));
+    CK(g.cand_list.ensure(n_cand));
+    CK(g.scal.ensure(4));
+    CK(cudaMemcpyAsync(dw.p, words, nw * sizeof(uint32_t), cudaMemcpyHostToDevice, g.st));
+    CK(launch_candidates(g.sys, g.mu, g.II, T, p->sampler_Rmin, p->sampler_Rmax, p->pesmin, p->pair_state, g.d_tab,
+                         dw.p, (long long)nw, 0, g.D, (long long)n_cand, g.accept.p, g.consumed.p, g.qp_cand.p,
+                         g.energy.p, g.scal.p, g.sx, prefilter ? g.cand_list.p : nullptr, g.scal.p + 2, g.st));
+    CK(cudaMemcpyAsync(accept, g.accept.p, n_cand, cudaMemcpyDeviceToHost, g.st));
+    CK(cudaStreamSynchronize(g.st));
+    return HH_OK;
+  };
+  rc = run();
+  dw.release();
+  return rc;
+}
+
 namespace {
 // body-frame N2-Ar dipole at (R, T) as each precision path evaluates it
 __global__ void n2ar_dip_probe_kernel(const N2arDipFold *F, const float4 *tab, const double *R, const double *T,

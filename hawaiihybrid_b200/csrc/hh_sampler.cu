@@ -77,7 +77,9 @@ cudaError_t launch_candidates(int sys, double mu, double II, double T, double Rm
   size_t smem = (sys == SYS_CO2AR) ? sizeof(Co2arTables<double>) : 0;
   long long blocks = (n_cand + 255) / 256;
   const unsigned *cl = nullptr;
-  if (list && sys == SYS_CH4CO2 && D == 25) {
+  // (below 0.7 K exp(-pesmin / kT) overflows and the weight is 0, infinite or a NaN, which FP64
+  // accepts: every candidate goes there)
+  if (list && sys == SYS_CH4CO2 && D == 25 && -pesmin * HH_HKT / T < 700.0) {
     // the words of every candidate's regular window are there: n_words covers them
     cudaError_t e = cudaMemsetAsync(n_list, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return e;

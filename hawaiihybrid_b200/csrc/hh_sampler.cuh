@@ -215,11 +215,21 @@ __device__ __forceinline__ double bm_normal(const uint32_t *w, long long &pos, l
 // reject() compares exp(-V / kT) / M with the candidate's last uniform u; V depends on the
 // positions alone, which are the first eight words.  One thread per candidate evaluates V
 // in FP32 and rejects at once where the comparison is decided by more than a bound on its
-// error, in the exponent 0.01 + (1e-4 |V| + 1e-7 Hartree) / kT: the FP32 site sum is good to
-// 1e-6 of its terms.  The others, and candidates with a zero word at a Box-Muller
-// position (whose draw is retried), go on the list for candidate_kernel, which decides
-// them as it would have decided all.  14.8e6 candidates: 6.6 ms with all in FP64, so 1.1 ms
-// (bound by reading the words) and 0.8 ms for those left.
+// error, in the exponent 0.01 + (1e-4 |V| + 1e-6 |pesmin| + 1e-7 Hartree) / kT.  The others,
+// and candidates with a zero word at a Box-Muller position (whose draw is retried), go on the
+// list for candidate_kernel, which decides them as it would have decided all.
+//
+// The bound, e = 2^-24: with 1 + c = 2 u and 1 - c = 2 (1 - u) of a polar angle both from the
+// integer word (c - 1 formed in FP32 would lose the angle beside a pole), sines, cosines and
+// the quaternion are good to 15 e, the phases to 2 pi e and R to 5 e, so a site-site distance
+// d is off by at most (20 R + 70) e, 1.1e-5 bohr at R = 6, and V by (12 P + 6 Q) / d times
+// that (P, Q the sums of its repulsive and attractive terms).  Where the comparison is open
+// at all, V - pesmin < 22 kT: P = 0.017 and Q = 0.01 Hartree at 100 K, an error of 6e-7
+// against a bound of 4e-6; P = 0.003, Q = 0.0045 towards 0 K, 1.4e-7 against 2.5e-7; on the
+// wall, where P is V, 6e-5 V against 1e-4 V.  The closest decisions of a million candidates,
+// most of them beside a pole, agree with FP64 with an eighth of the bound too.
+// 14.8e6 candidates: 6.6 ms with all in FP64, so 1.1 ms (bound by reading the words) and
+// 0.8 ms for those left.
 __global__ void __launch_bounds__(256) ch4_prefilter_kernel(SamplerArgs a, const uint32_t *words, long long word_base,
                                                             long long n_cand, unsigned char *accept,
                                                             unsigned char *consumed, unsigned *list,
@@ -245,9 +255,11 @@ __global__ void __launch_bounds__(256) ch4_prefilter_kernel(SamplerArgs a, const
     sincospif(float(w[3]) * k, &s1, &c1);   // phi / 2
     sincospif(float(w[5]) * k, &s3, &c3);   // psi / 2
     sincospif(2.f * float(w[6]) * k, &s2, &c2);
-    const float cT = 2.f * (float(w[2]) * k) - 1.f, ct = 2.f * (float(w[4]) * k) - 1.f, cu = 2.f * (float(w[7]) * k) - 1.f;
-    const float sT = sqrtf(fmaxf(0.f, (1.f - cT) * (1.f + cT))), su = sqrtf(fmaxf(0.f, (1.f - cu) * (1.f + cu)));
-    const float cb = sqrtf(fmaxf(0.f, 0.5f * (1.f + ct))), sb = sqrtf(fmaxf(0.f, 0.5f * (1.f - ct)));
+    // u and 1 - u of the three polar angles: cos = u - (1 - u), sin = 2 sqrt(u (1 - u))
+    const float uT = float(w[2]) * k, vT = (float(~w[2]) + 1.f) * k, ut = float(w[4]) * k, vt = (float(~w[4]) + 1.f) * k,
+                uu = float(w[7]) * k, vu = (float(~w[7]) + 1.f) * k;
+    const float cT = uT - vT, sT = 2.f * sqrtf(uT * vT), cu = uu - vu, su = 2.f * sqrtf(uu * vu);
+    const float cb = sqrtf(ut), sb = sqrtf(vt);  // theta / 2
     const float r[3] = {-R * sT * cP, -R * sT * sP, R * cT}, u[3] = {-su * c2, -su * s2, cu};
     const float t0 = c1 * cb, t1 = c1 * sb, t2 = s1 * sb, t3 = s1 * cb;
     const float q[4] = {t0 * c3 - t3 * s3, t1 * c3 + t2 * s3, t2 * c3 - t1 * s3, t0 * s3 + t3 * c3};
@@ -257,7 +269,7 @@ __global__ void __launch_bounds__(256) ch4_prefilter_kernel(SamplerArgs a, const
     const float ikT = float(HH_HKT / a.T);
     // ln(exp(-V / kT) / M) against ln u, M = 1.5 exp(-pesmin / kT); a NaN keeps the candidate
     const float lw = (float(a.pesmin) - V) * ikT - 0.405465f;
-    const float err = 0.01f + (1e-4f * fabsf(V) + 1e-7f) * ikT;
+    const float err = 0.01f + (1e-4f * fabsf(V) + 1e-6f * fabsf(float(a.pesmin)) + 1e-7f) * ikT;
     keep = keep || !(lw + err < logf(float(w[24]) * k));
     if (!keep) {
       accept[c0 + threadIdx.x] = 0;

@@ -309,6 +309,12 @@ const char *hh_cuda_strerror(int code);
  * (1..5) at sample k, as if its integrator or dipole had failed there; traj < 0
  * switches injection off. */
 int hh_cuda_mt_stream(uint32_t seed, uint64_t n, uint32_t *out);
+/* Diagnostic (no counterpart in the reference): the acceptance of n_cand candidates of the
+ * bound system at T from the caller's own stream words (host memory, 10, 16 or 25 words a
+ * candidate: atom-atom, linear-atom, rotor-linear).  prefilter != 0: as sampling decides
+ * them, CH4-CO2 with the rejection ahead of the momenta; 0: every candidate in FP64. */
+int hh_cuda_debug_candidates(const hh_calc_params *p, double T, const uint32_t *words, uint64_t n_cand, int prefilter,
+                             unsigned char *accept);
 int hh_cuda_debug_inject(int traj, int dir, int k, int status);
 /* registers a host buffer of capacity_words uint32 that the next correlation
  * call fills with (steps, samples, start ns, end ns) per half-trajectory item
