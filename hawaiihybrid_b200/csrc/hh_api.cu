@@ -1225,7 +1225,7 @@ constexpr size_t DEFER_HEADROOM = 16384;
 // fit goes in several launches); a launch that wrote
 // more contexts than the buffer holds repeats the call with a larger estimate of
 // contexts per item (HH_DEFER_EST sets the first one), and a second overflow with
-// in-kernel samples.
+// in-kernel samples, as does a call whose contexts cannot be allocated.
 int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n, uint64_t per_iter,
               uint64_t n_iter, int *nfail_out) {
   const size_t N = (size_t)P.N;
@@ -1234,11 +1234,14 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
   const size_t vb = mixed ? sizeof(float) : sizeof(double);
   const size_t ctx_b = mixed ? sizeof(SampleCtx<float, 6>) : sizeof(SampleCtx<double, 6>);
   const size_t start_b = mixed ? item_start_bytes<float>(g.sys) : item_start_bytes<double>(g.sys);
-  double &est = g.defer_est[g.sys][mixed ? 1 : 0];
-  // contexts per item: about 21 (mixed), 70 (CO2-Ar FP64) and 100 (N2-Ar FP64)
-  if (est == 0.0) est = mixed ? 32.0 : 128.0;
+  // contexts per item: about 21 (mixed), 70 (CO2-Ar FP64) and 100 (N2-Ar FP64); kept for the
+  // next call once this one has measured them
+  double &last_est = g.defer_est[g.sys][mixed ? 1 : 0];
+  double est = last_est > 0.0 ? last_est : mixed ? 32.0 : 128.0;
+  if (const char *ee = getenv("HH_DEFER_EST")) est = std::max(0.01, atof(ee));
+  bool no_memory = false;
   for (int attempt = 0;; ++attempt) {
-    const bool defer = eligible && attempt < 2;
+    bool defer = eligible && attempt < 2 && !no_memory;
     if (attempt > 0) {
       CK(cudaMemsetAsync(g.crln.p, 0, N * n_iter * sizeof(double), g.st));
       CK(cudaMemsetAsync(g.counters.p, 0, 16 * sizeof(unsigned long long), g.st));
@@ -1251,8 +1254,6 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     unsigned long long cap = 0;
     uint64_t it_launch = n_iter, tr_launch = n, items_launch = 2 * n;
     if (defer) {
-      if (attempt == 0)
-        if (const char *ee = getenv("HH_DEFER_EST")) est = std::max(0.01, atof(ee));
       const char *eb = getenv("HH_DEFER_BUDGET_MB");
       const size_t want = (size_t)(est * double(2 * n)) + DEFER_HEADROOM;
       size_t free_b = 0, total_b = 0;
@@ -1279,13 +1280,30 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       // buffer would otherwise be reallocated (cudaFree and cudaMalloc of gigabytes)
       // inside a call
       const size_t alloc = (size_t)(1.1 * double(cap));
-      if (g.dctx.cap < cap * ctx_b) CK(g.dctx.ensure(alloc * ctx_b));
-      if (g.dvals.cap < cap * 2 * vb) CK(g.dvals.ensure(alloc * 2 * vb));
-      CK(g.dcount.ensure(DEFER_WORDS));
-      CK(g.item_status.ensure(2 * n));
-      CK(g.item_mu0.ensure(2 * n * 4 * vb));
-      CK(g.item_fail.ensure(2 * n));
-      CK(g.istart.ensure(2 * n * start_b));
+      cudaError_t e = cudaSuccess;
+      auto hold = [&](auto &buf, size_t need, size_t ask) {
+        if (e == cudaSuccess && buf.cap < need) e = buf.ensure(ask);
+      };
+      hold(g.dctx, cap * ctx_b, alloc * ctx_b);
+      hold(g.dvals, cap * 2 * vb, alloc * 2 * vb);
+      hold(g.dcount, DEFER_WORDS, DEFER_WORDS);
+      hold(g.item_status, 2 * n, 2 * n);
+      hold(g.item_mu0, 2 * n * 4 * vb, 2 * n * 4 * vb);
+      hold(g.item_fail, 2 * n, 2 * n);
+      hold(g.istart, 2 * n * start_b, 2 * n * start_b);
+      if (e == cudaErrorMemoryAllocation) {
+        // another user of the device has the memory: this call takes its samples in the kernel,
+        // which needs none of these
+        cudaGetLastError();
+        g.dctx.release();
+        g.dvals.release();
+        no_memory = true;
+        defer = false;
+      } else {
+        CK(e);
+      }
+    }
+    if (defer) {
       CK(cudaMemsetAsync(g.item_fail.p, 0xff, 2 * n * sizeof(unsigned), g.st));
       CK(cudaMemsetAsync(g.dcount.p, 0, 2 * sizeof(unsigned long long), g.st));
       io.ctx = g.dctx.p;
@@ -1342,9 +1360,11 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       const double per = double(peak) / double(std::max<uint64_t>(1, items_launch));
       if (peak > cap) {
         est = std::max(2.0 * est, 1.25 * per);
+        last_est = est;
         continue;
       }
       est = std::max(8.0, 1.25 * per);
+      last_est = est;
     }
     if (nfail > 0) {
       std::vector<int> fl(nfail), it(2 * (size_t)nfail);
@@ -1382,6 +1402,7 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
         CK(cudaStreamSynchronize(g.st));
         if (peak > io2.ctx_cap) {
           est *= 2.0;
+          last_est = est;
           continue;
         }
       }
