@@ -103,6 +103,12 @@ struct TrajTune {
   int handoff_mul;  // (more than the slots: the solo kernel's warps take the stored items in turn)
 };
 
+// sample contexts per item that calls of one kind (window, tolerance, pair state) have taken
+struct DeferEst {
+  int N, pair_state;
+  double dt, rtol, per_item;
+};
+
 struct Ctx {
   bool init = false;
   int device = -1;
@@ -179,8 +185,8 @@ struct Ctx {
   DevBuf<int> item_status;
   DevBuf<unsigned> item_fail;
   DevBuf<unsigned char> istart;  // precomputed item starts (ItemStart per item)
-  // contexts per item per [system][FP64, mixed], from the previous calls (0: none yet)
-  double defer_est[5][2] = {};
+  // contexts per item per [system][FP64, mixed] and kind of call, from the previous calls
+  std::vector<DeferEst> defer_est[5][2];
   // CORRELATION_ARRAY weights [n][n_sat]: with ratios (C(t)) and without (nstar)
   DevBuf<double> sat_w, sat_wraw;
   // CH4-CO2 record path: sample records, their dipoles, the piece sort
@@ -1217,28 +1223,57 @@ int traj_block_sync() {
 // contexts beyond the estimate: the solo warps' unused reservations
 constexpr size_t DEFER_HEADROOM = 16384;
 
+// Contexts per item before a call of this kind has been measured.  Free pairs leave the window
+// early: measured up to 37 (mixed), 82 (CO2-Ar FP64) and 109 (N2-Ar FP64) at 100 to 300 K.
+// Bound pairs fill it with steps: 1.7e-3 per atomic unit of time (FP64), 1.3e-3 to 3.7e-3
+// (mixed, long to short windows).  An eighth-order step shrinks with the eighth root of the
+// tolerance.  An item has no more contexts than samples, N - 1, and its warp's reservations.
+double defer_default_est(bool mixed, const TrajParams &P, int pair_state) {
+  double est = mixed ? 32.0 : 128.0;
+  if (pair_state == HH_PAIR_STATE_BOUND) est += 2.5e-3 * P.dt * P.N;
+  return est * std::max(1.0, pow((mixed ? 3e-8 : 1e-12) / P.rtol, 0.125));
+}
+
+// The kept estimate for calls of this kind (per_item 0: none yet), made when there is none:
+// 16 kinds, the oldest one makes room.
+DeferEst &defer_kept_est(bool mixed, const TrajParams &P, int pair_state) {
+  std::vector<DeferEst> &v = g.defer_est[g.sys][mixed ? 1 : 0];
+  for (DeferEst &k : v)
+    if (k.N == P.N && k.pair_state == pair_state && k.dt == P.dt && k.rtol == P.rtol) return k;
+  if (v.size() >= 16) v.erase(v.begin());
+  v.push_back({P.N, pair_state, P.dt, P.rtol, 0.0});
+  return v.back();
+}
+// items a launch needs to tell the contexts per item of others (a few long trajectories
+// among a hundred say little)
+constexpr uint64_t DEFER_LEARN_ITEMS = 4096;
+
 // The plain C(t) launches of run_trajectories, then the replay of failed trajectories
 // (the reference drops a trajectory whose correlation_eval returns 1 while still
 // counting it: both branches are replayed with the opposite weight).  With deferred
 // samples the iterations go in launches whose sample contexts fit the buffer (at most
 // 32 GiB and 40 % of the free memory, or HH_DEFER_BUDGET_MB; an iteration that does not
-// fit goes in several launches); a launch that wrote
-// more contexts than the buffer holds repeats the call with a larger estimate of
-// contexts per item (HH_DEFER_EST sets the first one), and a second overflow with
-// in-kernel samples, as does a call whose contexts cannot be allocated.
+// fit goes in several launches).  The buffer is sized by an estimate of contexts per item,
+// kept per kind of call, since short windows, long ones and bound pairs take 8 to 1,400 of
+// them, and by what it already holds; a launch that wrote more contexts than the buffer
+// holds repeats the call with a larger estimate (HH_DEFER_EST sets the first one, and holds
+// the buffer to it), and a second overflow with in-kernel samples, as does a call whose
+// contexts cannot be allocated.  (One estimate for all kinds, from the call before, repeated
+// every long call that followed a short one: CO2-Ar FP64, 4,000 x 8,192 after 4,000 x 64
+// 66 ms, so 33.)
 int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n, uint64_t per_iter,
-              uint64_t n_iter, int *nfail_out) {
+              uint64_t n_iter, int pair_state, int *nfail_out) {
   const size_t N = (size_t)P.N;
   const bool eligible = defer_eligible(precision, P, io0, n);
   const bool mixed = precision == HH_PRECISION_MIXED;
   const size_t vb = mixed ? sizeof(float) : sizeof(double);
   const size_t ctx_b = mixed ? sizeof(SampleCtx<float, 6>) : sizeof(SampleCtx<double, 6>);
   const size_t start_b = mixed ? item_start_bytes<float>(g.sys) : item_start_bytes<double>(g.sys);
-  // contexts per item: about 21 (mixed), 70 (CO2-Ar FP64) and 100 (N2-Ar FP64); kept for the
-  // next call once this one has measured them
-  double &last_est = g.defer_est[g.sys][mixed ? 1 : 0];
-  double est = last_est > 0.0 ? last_est : mixed ? 32.0 : 128.0;
-  if (const char *ee = getenv("HH_DEFER_EST")) est = std::max(0.01, atof(ee));
+  double unkept = 0.0;
+  double &kept = eligible ? defer_kept_est(mixed, P, pair_state).per_item : unkept;
+  double est = std::min(kept > 0.0 ? kept : defer_default_est(mixed, P, pair_state), double(P.N) + 6.0);
+  const char *forced = getenv("HH_DEFER_EST");
+  if (forced) est = std::max(0.01, atof(forced));
   bool no_memory = false;
   for (int attempt = 0;; ++attempt) {
     bool defer = eligible && attempt < 2 && !no_memory;
@@ -1308,6 +1343,7 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
       CK(cudaMemsetAsync(g.dcount.p, 0, 2 * sizeof(unsigned long long), g.st));
       io.ctx = g.dctx.p;
       io.ctx_count = g.dcount.p;
+      if (!forced) cap = std::min(g.dctx.cap / ctx_b, g.dvals.cap / (2 * vb));
       io.ctx_cap = cap;
       io.item_status = g.item_status.p;
       io.item_mu0 = g.item_mu0.p;
@@ -1357,14 +1393,11 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
     if (defer) CK(cudaMemcpyAsync(&peak, g.dcount.p + DEFER_PEAK, sizeof peak, cudaMemcpyDeviceToHost, g.st));
     CK(cudaStreamSynchronize(g.st));
     if (defer) {
-      const double per = double(peak) / double(std::max<uint64_t>(1, items_launch));
-      if (peak > cap) {
-        est = std::max(2.0 * est, 1.25 * per);
-        last_est = est;
-        continue;
-      }
-      est = std::max(8.0, 1.25 * per);
-      last_est = est;
+      const double per = 1.25 * double(peak) / double(std::max<uint64_t>(1, items_launch));
+      const bool over = peak > cap;
+      est = over ? std::max(2.0 * est, per) : std::max(8.0, per);
+      if (items_launch >= DEFER_LEARN_ITEMS) kept = std::max(kept, est);
+      if (over) continue;
     }
     if (nfail > 0) {
       std::vector<int> fl(nfail), it(2 * (size_t)nfail);
@@ -1402,7 +1435,6 @@ int run_plain(int precision, const TrajParams &P, const TrajIO &io0, uint64_t n,
         CK(cudaStreamSynchronize(g.st));
         if (peak > io2.ctx_cap) {
           est *= 2.0;
-          last_est = est;
           continue;
         }
       }
@@ -1508,7 +1540,7 @@ int run_trajectories(const hh_calc_params *p, const double *d_ic, uint64_t n, ui
     CK(cudaMemcpyAsync(&nfail, g.fail_count.p, sizeof nfail, cudaMemcpyDeviceToHost, g.st));
     CK(cudaStreamSynchronize(g.st));
   } else {
-    int rc = run_plain(precision, P, io, n, per_iter, n_iter, &nfail);
+    int rc = run_plain(precision, P, io, n, per_iter, n_iter, p->pair_state, &nfail);
     if (rc) return rc;
   }
   CK(cudaEventRecord(g.ev[3], g.st));
