@@ -375,8 +375,12 @@ int sample_into(const hh_calc_params *p, double T, uint64_t n, double *d_out, ui
     long long remaining = (long long)(n - got);
     double pe = std::max(g.p_accept, 0.01);
     // 4,096 candidates of headroom: a request for 64 trajectories makes 44 thousand words of
-    // the sequential stream (0.04 ms), not the 655 thousand of a minimum round of 65,536
+    // the sequential stream (0.04 ms), not the 655 thousand of a minimum round of 65,536.  A
+    // request that this first round leaves open goes on by 65,536 or more: where one candidate
+    // in ten thousand is accepted (bound pairs), rounds of some 5,900 for 16 phase points took
+    // twice as long (He-Ar, 300 K: 3.8 ms, with rounds of 65,536 from the first on 1.9, so 1.0).
     long long ncand = (long long)(remaining / pe * 1.15) + 4096;
+    if (ncand_total > 0) ncand = std::max(ncand, 65536LL);
     ncand = std::min(ncand, 1LL << 23);
     int rc = ensure_words(g.wpos + ncand * g.D + 4096);
     if (rc) return rc;
