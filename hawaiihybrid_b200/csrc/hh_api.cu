@@ -101,6 +101,7 @@ struct TrajTune {
   int warps;        // bulk kernel warps per block
   int handoff_div;  // hand-off when at most (solo warp slots) * handoff_mul / handoff_div items are open
   int handoff_mul;  // (more than the slots: the solo kernel's warps take the stored items in turn)
+  bool fixed;       // the threshold was set from outside: it holds for launches of every size
 };
 
 // sample contexts per item that calls of one kind (window, tolerance, pair state) have taken
@@ -637,8 +638,11 @@ int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
     if (rc) return rc;
   }
   const int w = tt.warps ? tt.warps : traj_warps<PHYS>();
-  const int d = tt.handoff_div ? tt.handoff_div : 1;
-  const int m = tt.handoff_mul ? tt.handoff_mul : default_handoff_mul(SYS);
+  // a pick timed on a large launch is for large ones: below, the default (He-Ar FP64, 1,000
+  // trajectories: 1.2 ms, and 1.8 with the threshold of cap that a 20,000 call had picked)
+  const bool pick = tt.fixed || io.n_items >= TRAJ_TUNE_MIN_ITEMS;
+  const int d = pick && tt.handoff_div ? tt.handoff_div : 1;
+  const int m = pick && tt.handoff_mul ? tt.handoff_mul : default_handoff_mul(SYS);
   return launch_traj_pick<SYS, PHYS, STG, COMP>(P, io, w, d, m, false);
 }
 
@@ -2628,7 +2632,7 @@ int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div,
   if (precision != HH_PRECISION_FP64 && precision != HH_PRECISION_MIXED) return HH_E_INVALID_ARGUMENT;
   TrajTune &tt = g.traj_tune[g.sys][precision == HH_PRECISION_MIXED ? 1 : 0];
   if (set_warps < 0 || set_handoff_div < 0) {
-    tt.warps = tt.handoff_div = tt.handoff_mul = 0;
+    tt = TrajTune{};
   } else if (set_warps > 0 || set_handoff_div > 0) {
     if (set_warps > 0 && set_warps != TRAJ_WARPS_CANDIDATES[0] && set_warps != TRAJ_WARPS_CANDIDATES[1])
       return HH_E_INVALID_ARGUMENT;
@@ -2637,7 +2641,10 @@ int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div,
     const int dw = precision == HH_PRECISION_MIXED ? traj_warps<float>() : traj_warps<double>();
     tt.warps = set_warps > 0 ? set_warps : (tt.warps ? tt.warps : dw);
     tt.handoff_div = set_handoff_div > 0 ? set_handoff_div : (tt.handoff_div ? tt.handoff_div : 1);
-    if (set_handoff_div > 0) tt.handoff_mul = 1;
+    if (set_handoff_div > 0) {
+      tt.handoff_mul = 1;
+      tt.fixed = true;
+    }
   }
   if (warps) *warps = tt.warps;
   if (handoff_div) *handoff_div = tt.handoff_div;
