@@ -47,7 +47,7 @@ EXPORTS = (
     "hh_cuda_prmu", "hh_cuda_debug_n2ar_dipole", "hh_cuda_m2", "hh_cuda_debug_tuning",
     "hh_cuda_debug_kernel_ms", "hh_cuda_debug_ch4co2_fold", "hh_cuda_moment_sums", "hh_cuda_debug_traj_tuning",
     "hh_cuda_debug_set_ch4_dipole", "hh_cuda_debug_set_defer", "hh_cuda_debug_set_defer_overlap", "hh_cuda_vegas",
-    "hh_cuda_set_requantization", "hh_cuda_debug_candidates",
+    "hh_cuda_set_requantization", "hh_cuda_debug_candidates", "hh_cuda_debug_traj_handoff",
     "hh_write_correlation_function_ext", "hh_write_spectral_function_ext",
 )
 HH_REQ_NONE, HH_REQ_INTEGER, HH_REQ_HALFINTEGER = 0, 1, 2
@@ -161,6 +161,7 @@ def load(path: str | None = None):
     L.hh_cuda_vegas.argtypes = [C.POINTER(CalcParamsC), C.c_int, C.c_double, C.c_uint64, C.c_uint64, C.c_uint64,
                                 C.POINTER(C.c_double), C.POINTER(C.c_double)]
     L.hh_cuda_debug_traj_tuning.argtypes = [C.c_int, C.c_int, C.c_int, C.POINTER(C.c_int), C.POINTER(C.c_int)]
+    L.hh_cuda_debug_traj_handoff.argtypes = [C.c_int, C.c_int, C.POINTER(C.c_int)]
     L.hh_cuda_shutdown.restype = None
     for name in EXPORTS:
         if name not in ("hh_cuda_strerror", "hh_cuda_shutdown") and not name.startswith("hh_write_"):
@@ -227,3 +228,11 @@ def traj_tuning(precision: int, set_warps: int = 0, set_handoff_div: int = 0) ->
     check(load().hh_cuda_debug_traj_tuning(int(precision), int(set_warps), int(set_handoff_div),
                                            C.byref(w), C.byref(d)))
     return w.value, d.value
+
+
+def traj_handoff_mul(precision: int, set_mul: int = 0) -> int:
+    """Multiple of the solo warp slots in the hand-off threshold (0 before the autotuner ran);
+    set_mul > 0 (1, 2, 4 or 8) fixes it for launches of every size."""
+    m = C.c_int(0)
+    check(load().hh_cuda_debug_traj_handoff(int(precision), int(set_mul), C.byref(m)))
+    return m.value

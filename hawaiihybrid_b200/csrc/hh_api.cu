@@ -543,17 +543,27 @@ int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int div, 
 //   He-Ar 1,000    1.77 1.32 1.32 1.32 1.33      PR_MU CO2-Ar 4,096  22.8 19.8 17.8 17.8 17.7
 // (mixed path: CO2-Ar 1,000 2.71 2.32 2.34, PR_MU 4,096 5.23 4.77 3.66).  CH4-CO2, whose
 // trajectories are all about as long, gains nothing.
-// HH_TRAJ_WARPS (4 or 8) and HH_TRAJ_HANDOFF_DIV (1, 2 or 4) fix a choice instead.
+// HH_TRAJ_WARPS (4 or 8) and HH_TRAJ_HANDOFF_DIV (1, 2 or 4) fix a choice instead, for launches
+// of every size.
 constexpr int TRAJ_TUNE_MIN_ITEMS = 16384;  // smaller launches use the defaults
 constexpr int TRAJ_TUNE_ITEMS = 32768;      // items the timing runs integrate
+constexpr int HANDOFF_MUL_MAX = 8;          // largest hand-off threshold, items per solo warp slot
+
+// the environment's choices (0: none)
+int env_traj_warps() {
+  const char *e = getenv("HH_TRAJ_WARPS");
+  const int w = e ? atoi(e) : 0;
+  return w == TRAJ_WARPS_CANDIDATES[0] || w == TRAJ_WARPS_CANDIDATES[1] ? w : 0;
+}
+int env_handoff_div() {
+  const char *e = getenv("HH_TRAJ_HANDOFF_DIV");
+  const int d = e ? atoi(e) : 0;
+  return d == 1 || d == 2 || d == 4 ? d : 0;
+}
 
 template <int SYS, typename PHYS, typename STG, bool COMP>
 int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
-  const char *ew = getenv("HH_TRAJ_WARPS");
-  const char *ed = getenv("HH_TRAJ_HANDOFF_DIV");
-  int fixed_w = ew ? atoi(ew) : 0, fixed_d = ed ? atoi(ed) : 0;
-  if (fixed_w != TRAJ_WARPS_CANDIDATES[0] && fixed_w != TRAJ_WARPS_CANDIDATES[1]) fixed_w = 0;
-  if (fixed_d != 1 && fixed_d != 2 && fixed_d != 4) fixed_d = 0;
+  const int fixed_w = env_traj_warps(), fixed_d = env_handoff_div();
   const int n_s = std::min(io.n_items, TRAJ_TUNE_ITEMS);
   const int nsl = std::max(1, io.n_sat);
   CK(g.tune_crln.ensure((size_t)P.N * nsl));
@@ -602,7 +612,7 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
     int rc = run(w_best, 1, 1, &bulk, &all);
     if (rc) return rc;
     float best = all;
-    for (int m : {2, 4, 8}) {
+    for (int m = 2; m <= HANDOFF_MUL_MAX; m *= 2) {
       rc = run(w_best, 1, m, &bulk, &all);
       if (rc) return rc;
       if (!(all < best)) break;
@@ -637,7 +647,9 @@ int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
     int rc = tune_traj<SYS, PHYS, STG, COMP>(P, io, &tt);
     if (rc) return rc;
   }
-  const int w = tt.warps ? tt.warps : traj_warps<PHYS>();
+  const int ew = tt.warps ? 0 : env_traj_warps(), ed = tt.fixed ? 0 : env_handoff_div();
+  const int w = tt.warps ? tt.warps : ew ? ew : traj_warps<PHYS>();
+  if (ed) return launch_traj_pick<SYS, PHYS, STG, COMP>(P, io, w, ed, 1, false);
   // a pick timed on a large launch is for large ones: below, the default (He-Ar FP64, 1,000
   // trajectories: 1.2 ms, and 1.8 with the threshold of cap that a 20,000 call had picked)
   const bool pick = tt.fixed || io.n_items >= TRAJ_TUNE_MIN_ITEMS;
@@ -2648,6 +2660,21 @@ int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div,
   }
   if (warps) *warps = tt.warps;
   if (handoff_div) *handoff_div = tt.handoff_div;
+  return HH_OK;
+}
+
+int hh_cuda_debug_traj_handoff(int precision, int set_mul, int *handoff_mul) {
+  if (!g.init) return HH_E_NOT_INITIALIZED;
+  if (precision != HH_PRECISION_FP64 && precision != HH_PRECISION_MIXED) return HH_E_INVALID_ARGUMENT;
+  if (set_mul < 0 || set_mul > HANDOFF_MUL_MAX || (set_mul & (set_mul - 1))) return HH_E_INVALID_ARGUMENT;
+  TrajTune &tt = g.traj_tune[g.sys][precision == HH_PRECISION_MIXED ? 1 : 0];
+  if (set_mul > 0) {
+    if (!tt.warps) tt.warps = precision == HH_PRECISION_MIXED ? traj_warps<float>() : traj_warps<double>();
+    tt.handoff_div = 1;
+    tt.handoff_mul = set_mul;
+    tt.fixed = true;
+  }
+  if (handoff_mul) *handoff_mul = tt.handoff_mul;
   return HH_OK;
 }
 

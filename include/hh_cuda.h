@@ -374,14 +374,22 @@ int hh_cuda_debug_kernel_ms(int enable, double *ms, uint64_t *launches, int n);
 /* Tuning knob (no counterpart in the reference): the trajectory launch's block
  * shape (bulk kernel warps per block, 4 or 8) and hand-off threshold (the launch
  * switches from 32 trajectories per warp to one when at most (solo warp slots) /
- * handoff_div items are open; 1, 2 or 4; with 1 the tuner may also pick two or four
- * times the slots) for the bound system and `precision`.  The
+ * handoff_div items are open; 1, 2 or 4; or at most a multiple of the slots, see
+ * hh_cuda_debug_traj_handoff) for the bound system and `precision`.  The
  * library times the candidates on the first plain-C(t) launch of at least 16,384
- * half-trajectories per system and precision (environment HH_TRAJ_WARPS,
- * HH_TRAJ_HANDOFF_DIV fix them instead).  set_* > 0 fixes a value, set_* < 0
- * forgets the pick (tuned again on the next large call), 0 leaves it; *warps and
- * *handoff_div receive the current pick (0: not tuned yet). */
+ * half-trajectories per system and precision and uses the threshold it picks for
+ * launches of that size; smaller ones take a fixed multiple of the slots (8 for N2-Ar, 1 for
+ * CH4-CO2, else 4).  The environment (HH_TRAJ_WARPS, HH_TRAJ_HANDOFF_DIV) fixes them
+ * instead, for launches of every size, as does set_* > 0 (a divisor also sets the multiple
+ * to 1).  set_* < 0 forgets the pick (tuned again on the next large call), 0 leaves it;
+ * *warps and *handoff_div receive the current pick (0: not tuned yet). */
 int hh_cuda_debug_traj_tuning(int precision, int set_warps, int set_handoff_div, int *warps, int *handoff_div);
+/* The multiple of the solo warp slots in the same threshold: the tuner picks 1, 2, 4 or 8
+ * (with 1 also a divisor).  set_mul > 0 fixes it for launches of every size, with divisor 1;
+ * 0 leaves it; *handoff_mul receives the current pick (0: not tuned yet).  A pick read as
+ * (warps, divisor, multiple) is reproduced by setting warps and the multiple where that is
+ * above 1, else warps and the divisor. */
+int hh_cuda_debug_traj_handoff(int precision, int set_mul, int *handoff_mul);
 /* Diagnostic (no counterpart in the reference): shape of the CH4-CO2 dipole's
  * coefficient stream (batches of 4 entries per radial piece, and the (Y1,
  * component, cos/sin) groups they form); HH_E_NOT_INITIALIZED before a CH4-CO2
