@@ -205,7 +205,7 @@ struct Ctx {
   DevBuf<double> m0_partials, m0_out;
   // VEGAS: grid edges, block sums, per-bin sums of F^2
   DevBuf<double> vg_edges, vg_sums, vg_hist;
-  // FFT, and the CUDA graph of its kernel sequence for the current (N, dt, buffers)
+  // CF -> SF: C(t), the spectrum, the transform's workspaces, the page-locked staging
   DevBuf<double> f_cf, f_sf;
   DevBuf<double2> f_a, f_b;
   PinBuf<double> f_pin;

@@ -16,9 +16,9 @@
 // uniforms ((w >> 8) + 0.5) * 2^-24, which are exact in FP32 and FP64, so the
 // FP32 and FP64 integrands see the same sample.
 //
-// Sums: per thread FP64 compensated sums of w and plain sums of w^2 per
-// temperature, a fixed-order block reduction, then one fixed-order pass over
-// the block partials.
+// Sums: per thread compensated sums of w and plain sums of w^2 per temperature
+// (FP64; on the mixed path FP32), a fixed-order block reduction in FP64, then one
+// fixed-order pass over the block partials.
 //
 // Second moment (calculate_M2, src/hawaii.c:1524-1617; VEGAS integrand_M2,
 // src/hep_hawaii.cpp:228-330): the integrand is |dmu/dt|^2 = qdot^T D D^T qdot with
