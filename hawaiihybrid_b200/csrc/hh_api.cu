@@ -20,6 +20,7 @@
 #include "hh_consts.h"
 #include "hh_defer.cuh"
 #include "hh_fft.cuh"
+#include "hh_handoff.h"
 #include "hh_internal.h"
 #include "hh_m0.cuh"
 #include "hh_prmu.cuh"
@@ -526,8 +527,8 @@ int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int div, 
 // trajectories per warp to one).  Timed on the launch's first items, into scratch
 // C(t) and counters, so the call's own results are untouched:
 //   1. each warps-per-block candidate with the full hand-off threshold: bulk kernel time;
-//   2. with the faster shape, the launch time at thresholds of 2 cap, 4 cap and 8 cap as long
-//      as each is faster; otherwise cap / 2 and, if faster, cap / 4.  More than cap:
+//   2. with the faster shape, the launch time at the default threshold, then at larger ones,
+//      else smaller ones, as long as each is clearly faster (pick_handoff).  More than cap:
 //      the solo kernel's warps take several stored items in turn, which pays where few of
 //      the bulk kernel's lanes are left busy long before the end (N2-Ar FP64, 20,011
 //      trajectories: 10 % of the lanes from a fifth of the launch on; the call 135 ms with a
@@ -547,7 +548,7 @@ int launch_traj_pick(const TrajParams &P, const TrajIO &io, int warps, int div, 
 // of every size.
 constexpr int TRAJ_TUNE_MIN_ITEMS = 16384;  // smaller launches use the defaults
 constexpr int TRAJ_TUNE_ITEMS = 32768;      // items the timing runs integrate
-constexpr int HANDOFF_MUL_MAX = 8;          // largest hand-off threshold, items per solo warp slot
+constexpr int default_handoff_mul(int sys) { return sys == SYS_CH4CO2 ? 1 : sys == SYS_N2AR ? 8 : 4; }
 
 // the environment's choices (0: none)
 int env_traj_warps() {
@@ -609,24 +610,9 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
   }
   int d_best = fixed_d ? fixed_d : 1, m_best = 1;
   if (!fixed_d) {
-    int rc = run(w_best, 1, 1, &bulk, &all);
+    int rc = pick_handoff(
+        default_handoff_mul(SYS), [&](int d, int m, float *ms) { return run(w_best, d, m, &bulk, ms); }, &d_best, &m_best);
     if (rc) return rc;
-    float best = all;
-    for (int m = 2; m <= HANDOFF_MUL_MAX; m *= 2) {
-      rc = run(w_best, 1, m, &bulk, &all);
-      if (rc) return rc;
-      if (!(all < best)) break;
-      best = all;
-      m_best = m;
-    }
-    for (int d : {2, 4}) {
-      if (m_best > 1) break;
-      rc = run(w_best, d, 1, &bulk, &all);
-      if (rc) return rc;
-      if (!(all < best)) break;
-      best = all;
-      d_best = d;
-    }
   }
   // the timing runs' sample contexts are scratch
   if (t.ctx_count) CK(cudaMemsetAsync(t.ctx_count, 0, sizeof(unsigned long long), g.st));
@@ -635,8 +621,6 @@ int tune_traj(const TrajParams &P, const TrajIO &io, TrajTune *out) {
   out->handoff_mul = m_best;
   return HH_OK;
 }
-
-constexpr int default_handoff_mul(int sys) { return sys == SYS_CH4CO2 ? 1 : sys == SYS_N2AR ? 8 : 4; }
 
 template <int SYS, typename PHYS, typename STG, bool COMP>
 int launch_traj(const TrajParams &P, const TrajIO &io, int *grid_out) {
