@@ -201,23 +201,46 @@ template <class F> void each(const Tensor &t, F f) {
       for (int q = -1; q <= 1; ++q) f(a, b, q);
 }
 double ladder(int l, int m, int s) { return std::sqrt(double(l * (l + 1) - m * (m + s))); }  // m -> m + s
-// J_s T, s = +1 or -1: the sum of the three ladder operators
-Tensor shift(const Tensor &t, int s) {
-  Tensor o(t.l1, t.l2);
-  each(t, [&](int a, int b, int q) {
-    cplx x = 0.0;
-    if (std::abs(a - s) <= t.l1) x += ladder(t.l1, a - s, s) * t.get(a - s, b, q);
-    if (std::abs(b - s) <= t.l2) x += ladder(t.l2, b - s, s) * t.get(a, b - s, q);
-    if (std::abs(q - s) <= 1) x += ladder(1, q - s, s) * t.get(a, b, q - s);
-    o.at(a, b, q) = x;
-  });
+// the elements of a tensor with a + b + q = K, one b for each (a, q)
+struct Slice {
+  int l1, l2, K;
+  std::vector<cplx> v;
+  Slice(int a, int b, int k) : l1(a), l2(b), K(k), v((size_t)(2 * a + 1) * 3, 0.0) {}
+  cplx &at(int a, int q) { return v[(size_t)(a + l1) * 3 + (q + 1)]; }
+  cplx get(int a, int b, int q) const {
+    if (a + b + q != K || std::abs(a) > l1 || std::abs(b) > l2 || std::abs(q) > 1) return 0.0;
+    return v[(size_t)(a + l1) * 3 + (q + 1)];
+  }
+};
+template <class F> void each(const Slice &t, F f) {
+  for (int a = -t.l1; a <= t.l1; ++a)
+    for (int q = -1; q <= 1; ++q)
+      if (std::abs(t.K - a - q) <= t.l2) f(a, t.K - a - q, q);
+}
+// element (a, b, q) of J_s T, s = +1 or -1: the sum of the three ladder operators
+template <class T> cplx shifted(const T &t, int s, int a, int b, int q) {
+  cplx x = 0.0;
+  if (std::abs(a - s) <= t.l1) x += ladder(t.l1, a - s, s) * t.get(a - s, b, q);
+  if (std::abs(b - s) <= t.l2) x += ladder(t.l2, b - s, s) * t.get(a, b - s, q);
+  if (std::abs(q - s) <= 1) x += ladder(1, q - s, s) * t.get(a, b, q - s);
+  return x;
+}
+// |J_s T|^2
+double shift_norm2(const Tensor &t, int s) {
+  double n = 0.0;
+  each(t, [&](int a, int b, int q) { n += std::norm(shifted(t, s, a, b, q)); });
+  return n;
+}
+// J_s T / c of a slice, which is the slice K + s.  (As whole tensors the ladder of slices took
+// 25 ms of every process that binds the system, so a tenth of it.)
+Slice shift(const Slice &t, int s, double c) {
+  Slice o(t.l1, t.l2, t.K + s);
+  each(o, [&](int a, int b, int q) { o.at(a, q) = shifted(t, s, a, b, q) / c; });
   return o;
 }
-Tensor slice(const Tensor &t, int K) {
-  Tensor o(t.l1, t.l2);
-  each(t, [&](int a, int b, int q) {
-    if (a + b + q == K) o.at(a, b, q) = t.get(a, b, q);
-  });
+Slice slice(const Tensor &t, int K) {
+  Slice o(t.l1, t.l2, K);
+  each(o, [&](int a, int b, int q) { o.at(a, q) = t.get(a, b, q); });
   return o;
 }
 double norm2(const Tensor &t) {
@@ -225,21 +248,18 @@ double norm2(const Tensor &t) {
   for (const cplx &x : t.v) n += std::norm(x);
   return n;
 }
-// P_l^m(cos theta) cos or sin (m phi) (Condon-Shortley) over the complex harmonics
-void real_harmonic(int l, int m, int cs, std::vector<cplx> &v) {
-  v.assign(2 * l + 1, 0.0);
+// P_l^m(cos theta) cos or sin (m phi) (Condon-Shortley) over the complex harmonics: the
+// coefficients of -m and m (m = 0: the first one)
+struct RealHarmonic {
+  cplx lo, hi;
+};
+RealHarmonic real_harmonic(int l, int m, int cs) {
   double r = 1.0;  // (l + m)! / (l - m)!
   for (int k = l - m + 1; k <= l + m; ++k) r *= k;
   const double n = std::sqrt((2 * l + 1) / (4.0 * M_PI) / r), sg = (m & 1) ? -1.0 : 1.0;
-  if (m == 0) {
-    v[l] = 1.0 / n;
-  } else if (cs == 0) {
-    v[l + m] = 0.5 / n;
-    v[l - m] = 0.5 * sg / n;
-  } else {
-    v[l + m] = cplx(0.0, -0.5) / n;
-    v[l - m] = cplx(0.0, 0.5) * sg / n;
-  }
+  if (m == 0) return {1.0 / n, 0.0};
+  if (cs == 0) return {0.5 * sg / n, 0.5 / n};
+  return {cplx(0.0, 0.5) * sg / n, cplx(0.0, -0.5) / n};
 }
 using Poly = std::vector<cplx>;  // coefficients K = -J..J
 Poly mul(const Poly &a, const Poly &b) {
@@ -295,26 +315,23 @@ int ch4co2_build_coupled(Ch4Co2CoupledHost *out) {
     lm_of(hh_ch4co2_tidx[kv.second[0]][3], &l2, &m2, &c2);
     if (l2 > CH4C_LMAX || (l2 & 1)) return -1;
     Tensor T(l1, l2);
-    std::vector<cplx> y1, y2;
     for (int t : kv.second) {
       const short *ix = hh_ch4co2_tidx[t];
       int a, am, ac, e, em, ec;
       lm_of(ix[2], &a, &am, &ac);
       lm_of(ix[3], &e, &em, &ec);
       if (a != l1 || e != l2) return -1;
-      real_harmonic(a, am, ac, y1);
-      real_harmonic(e, em, ec, y2);
-      for (int p = -l1; p <= l1; ++p)
-        if (y1[p + l1] != 0.0)
-          for (int r = -l2; r <= l2; ++r)
-            if (y2[r + l2] != 0.0)
-              for (int q = -1; q <= 1; ++q)
-                T.at(p, r, q) += hh_ch4co2_tcoef[t] * y1[p + l1] * y2[r + l2] * cart[ix[1]][q + 1];
+      const RealHarmonic y1 = real_harmonic(a, am, ac), y2 = real_harmonic(e, em, ec);
+      for (int p = -am; p <= am; p += std::max(1, 2 * am))
+        for (int r = -em; r <= em; r += std::max(1, 2 * em)) {
+          const cplx yy = hh_ch4co2_tcoef[t] * (p == -am ? y1.lo : y1.hi) * (r == -em ? y2.lo : y2.hi);
+          for (int q = -1; q <= 1; ++q) T.at(p, r, q) += yy * cart[ix[1]][q + 1];
+        }
     }
     const double n2 = norm2(T);
     if (!(n2 > 0.0)) continue;
     // J from <J^2> = |J_- T|^2 + <Jz^2 - Jz>
-    double jj = norm2(shift(T, -1)) / n2, kz = 0.0;
+    double jj = shift_norm2(T, -1) / n2, kz = 0.0;
     each(T, [&](int a, int e, int q) {
       const int K = a + e + q;
       kz += double(K) * (K - 1) * std::norm(T.get(a, e, q));
@@ -331,24 +348,18 @@ int ch4co2_build_coupled(Ch4Co2CoupledHost *out) {
     for (int K = 1; K <= J; ++K)
       if (std::abs(I[jx][K + J]) / sqrt_binom(J, K) > 1.0001 * std::abs(I[jx][K0 + J]) / sqrt_binom(J, K0)) K0 = K;
     const cplx alpha = sqrt_binom(J, K0) / I[jx][K0 + J];
-    std::map<int, Tensor> sl;
-    sl.emplace(K0, slice(T, K0));
-    for (int K = K0; K < J; ++K) {
-      Tensor n = shift(sl.at(K), 1);
-      for (cplx &x : n.v) x /= ladder(J, K, 1);
-      sl.emplace(K + 1, n);
-    }
-    for (int K = K0; K > -J; --K) {
-      Tensor n = shift(sl.at(K), -1);
-      for (cplx &x : n.v) x /= ladder(J, K, -1);
-      sl.emplace(K - 1, n);
-    }
+    std::vector<Slice> sl(2 * J + 1, Slice(l1, l2, 0));  // K = -J..J
+    sl[K0 + J] = slice(T, K0);
+    for (int K = K0; K < J; ++K) sl[K + 1 + J] = shift(sl[K + J], 1, ladder(J, K, 1));
+    for (int K = K0; K > -J; --K) sl[K - 1 + J] = shift(sl[K + J], -1, ladder(J, K, -1));
     // T = sum_K a_K |J K> with a_K = p_K / sqrt_binom(K) / alpha'
+    std::vector<cplx> aK(2 * J + 1);
+    for (int K = -J; K <= J; ++K) aK[K + J] = alpha * I[jx][K + J] / sqrt_binom(J, K);
     double off = 0.0;
     each(T, [&](int a, int e, int q) {
       const int K = a + e + q;
       cplx x = T.get(a, e, q);
-      if (std::abs(K) <= J) x -= alpha * I[jx][K + J] / sqrt_binom(J, K) * sl.at(K).get(a, e, q);
+      if (std::abs(K) <= J) x -= aK[K + J] * sl[K + J].get(a, e, q);
       off += std::norm(x);
     });
     if (!(off < 1e-18 * n2)) return -1;
@@ -357,7 +368,7 @@ int ch4co2_build_coupled(Ch4Co2CoupledHost *out) {
       for (int q = 0; q <= 1; ++q) {
         const int mm = K - q;
         if (std::abs(mm) > l2 || (q == 0 && mm < 0)) continue;
-        cplx gv = alpha * sl.at(K).get(0, mm, q) * yy / sqrt_binom(J, K);
+        cplx gv = alpha * sl[K + J].get(0, mm, q) * yy / sqrt_binom(J, K);
         if (mm < 0 && (mm & 1)) gv = -gv;       // P^{-m} = (-1)^m P^m in this normalisation
         if (std::abs(gv.imag()) > 1e-10 * std::abs(gv) + 1e-14) return -1;
         double gr = gv.real();
