@@ -336,7 +336,8 @@ def bench_ch4co2(args, hh, H, peaks):
     s64, s32 = C.c_int(0), C.c_int(0)
     _lib.check(_lib.load().hh_cuda_debug_tuning(C.byref(s64), C.byref(s32)))
     out["dipole_records_per_lane"] = {"fp64": s64.value, "mixed": s32.value,
-                                      "how": "timed per precision on the first call's records (the warm-up)"}
+                                      "how": "mixed: timed on the first call's records (the warm-up); FP64: the "
+                                             "coupled form (-2), without timing"}
     nb, ng = _lib.ch4co2_fold_shape()
     coupled = s64.value == -2
     stream_fl = flops.ch4_dipole_flops(4 * nb, ng)
