@@ -14,8 +14,11 @@ LIBDIR = os.path.join(PKG, "lib")
 LIB = os.path.join(LIBDIR, "libhh_cuda.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-# --split-compile=0: nvcc optimises the unit's kernels on every host core in parallel
-# (the register allocation of the trajectory kernels is the same as a serial build's)
+# --split-compile=0: nvcc optimises the unit's kernels on every host core in parallel.  The
+# code it makes of one source differs from build to build with the compiler's own (randomized)
+# addresses: two sets of register counts, and times a few percent apart (M0 mixed 5.35 or 5.55 ms,
+# the N2-Ar solo kernel 28 or 35, VEGAS 1.9 or 1.4).  A serial build is reproducible, but its bulk
+# kernels are slower (CH4-CO2 FP64 16 ms, not 6; CO2-Ar FP64 41, not 30).
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xptxas", "-O3", "--split-compile=0"]
 
 # translation units and their extra flags; the sampler keeps the reference's

@@ -387,7 +387,7 @@ __global__ void __launch_bounds__(256) m0_kernel(M0Args a, const Co2arTablesGlob
         if (a.pair_state == 1) keep = (H >= PHYS(0));
         else if (a.pair_state == 2) keep = (H <= PHYS(0));
         AT wv = keep ? AT(base * exp(-V * ikT[t])) : AT(0);
-        if constexpr (MOMENT == 2) wv *= AT(kappa / ikT[t]);  // (2K/nu) G with K = kappa kT
+        wv *= AT(kappa / ikT[t]);  // M2: (2K/nu) G with K = kappa kT
         // compensated accumulation of w, plain accumulation of w^2
         AT y = wv - c[t];
         AT tt = s[t] + y;
